@@ -851,7 +851,7 @@ k_center(int n, const Vec<D> *__restrict__ Yn, Vec<D> *__restrict__ Y, const dou
 // shared memory 256 at a time, FP32 per tile and FP64 across tiles.
 template <int D>
 __global__ void __launch_bounds__(256)
-k_exact_sv(int n, const Vec<D> *__restrict__ Y, float *__restrict__ s, Vec<D> *__restrict__ v)
+k_exact_sv(int n, const Vec<D> *__restrict__ Y, float4 *__restrict__ sv)
 {
     __shared__ Vec<D> sh[256];
     const int i = blockIdx.x * 256 + threadIdx.x;
@@ -878,32 +878,36 @@ k_exact_sv(int n, const Vec<D> *__restrict__ Y, float *__restrict__ s, Vec<D> *_
         for (int k = 0; k < D; k++) V[k] += tv[k];
     }
     if (i < n) {
-        s[i] = (float)S;
-        Vec<D> o = vzero<D>();
-        for (int k = 0; k < D; k++) vset(o, k, (float)V[k]);
-        v[i] = o;
+        sv[i] = make_float4((float)S, (float)V[0], (float)V[1], D == 3 ? (float)V[D - 1] : 0.f);
     }
+}
+
+// s and v of a point are packed as (s, v): the layout the H2 product leaves its sums in.
+template <int D>
+__device__ __forceinline__ float sv_v(const float4 &a, int k)
+{
+    return k == 0 ? a.y : (k == 1 ? a.z : a.w);
 }
 
 // Z identity (reference tsne_h2pack.c:558-590): Z = sum s + 2 sum |y|^2 s - 2 sum y.v,
 // three FP64 sums over fixed blocks.
 template <int D>
 __global__ void __launch_bounds__(RED_BLOCK)
-k_z_part(int n, const Vec<D> *__restrict__ Yp, const float *__restrict__ s, const Vec<D> *__restrict__ v,
-         double *__restrict__ partials)
+k_z_part(int n, const Vec<D> *__restrict__ Yp, const float4 *__restrict__ sv, double *__restrict__ partials)
 {
     double t[3] = {0.0, 0.0, 0.0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const Vec<D> y = Yp[i], vv = v[i];
+        const Vec<D> y = Yp[i];
+        const float4 a = sv[i];
         double yy = 0.0, yv = 0.0;
 #pragma unroll
         for (int k = 0; k < D; k++) {
             const double yk = vget(y, k);
             yy += yk * yk;
-            yv += yk * (double)vget(vv, k);
+            yv += yk * (double)sv_v<D>(a, k);
         }
-        t[0] += s[i];
-        t[1] += yy * s[i];
+        t[0] += a.x;
+        t[1] += yy * a.x;
         t[2] += yv;
     }
     __shared__ double sh[RED_BLOCK][3];
@@ -923,9 +927,8 @@ k_z_part(int n, const Vec<D> *__restrict__ Yp, const float *__restrict__ s, cons
 // non-finite Z skips the force, as the reference does.
 template <int D>
 __global__ void __launch_bounds__(RED_BLOCK)
-k_force(int n, const Vec<D> *__restrict__ Yp, const float *__restrict__ s, const Vec<D> *__restrict__ v,
-        const int *__restrict__ perm, Vec<D> *__restrict__ F, DevScalars *sc,
-        const double *__restrict__ partials, int nblk, int h2_path, int keep_rep)
+k_force(int n, const Vec<D> *__restrict__ Yp, const float4 *__restrict__ sv, const int *__restrict__ perm,
+        Vec<D> *__restrict__ F, DevScalars *sc, const double *__restrict__ partials, int nblk, int h2_path, int keep_rep)
 {
     __shared__ double tz[3];
     reduce_partials<3>(partials, nblk, tz);
@@ -940,11 +943,12 @@ k_force(int n, const Vec<D> *__restrict__ Yp, const float *__restrict__ s, const
     if (!ok) return;
     const double c = 4.0 / Z;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const Vec<D> y = Yp[i], vv = v[i];
-        const double si = s[i];
+        const Vec<D> y = Yp[i];
+        const float4 a = sv[i];
+        const double si = a.x;
         Vec<D> f = vzero<D>();
 #pragma unroll
-        for (int k = 0; k < D; k++) vset(f, k, (float)(c * ((double)vget(y, k) * si - (double)vget(vv, k))));
+        for (int k = 0; k < D; k++) vset(f, k, (float)(c * ((double)vget(y, k) * si - (double)sv_v<D>(a, k))));
         F[perm ? perm[i] : i] = f;
     }
 }
@@ -1331,20 +1335,19 @@ void launch_center(cudaStream_t st, int n, const void *Ynext, void *Ycur, const 
 }
 
 template <int D>
-void launch_exact_sv(cudaStream_t st, int n, const void *Y, float *s, void *v)
+void launch_exact_sv(cudaStream_t st, int n, const void *Y, float4 *sv)
 {
-    k_exact_sv<D><<<ceil_div(n, 256), 256, 0, st>>>(n, (const Vec<D> *)Y, s, (Vec<D> *)v);
+    k_exact_sv<D><<<ceil_div(n, 256), 256, 0, st>>>(n, (const Vec<D> *)Y, sv);
 }
 
 template <int D>
-void launch_z_force(cudaStream_t st, int n, const void *Ypts, const float *s, const void *v,
+void launch_z_force(cudaStream_t st, int n, const void *Ypts, const float4 *sv,
                     const int *perm, void *rep, DevScalars *sc, double *partials, int h2_path,
                     int keep_rep)
 {
     const int nblk = 148 * 2;
-    k_z_part<D><<<nblk, RED_BLOCK, 0, st>>>(n, (const Vec<D> *)Ypts, s, (const Vec<D> *)v, partials);
-    k_force<D><<<ew_grid(n), RED_BLOCK, 0, st>>>(n, (const Vec<D> *)Ypts, s, (const Vec<D> *)v, perm,
-                                                 (Vec<D> *)rep, sc, partials, nblk, h2_path, keep_rep);
+    k_z_part<D><<<nblk, RED_BLOCK, 0, st>>>(n, (const Vec<D> *)Ypts, sv, partials);
+    k_force<D><<<ew_grid(n), RED_BLOCK, 0, st>>>(n, (const Vec<D> *)Ypts, sv, perm, (Vec<D> *)rep, sc, partials, nblk, h2_path, keep_rep);
 }
 
 template <int D>
@@ -1424,9 +1427,9 @@ void launch_pcal(cudaStream_t st, int n, const int *indptr, const double *dist, 
                                    float, double *);                                                 \
     template void launch_center<D>(cudaStream_t, int, const void *, void *, const double *,         \
                                    DevScalars *, const void *, double *);                            \
-    template void launch_exact_sv<D>(cudaStream_t, int, const void *, float *, void *);             \
-    template void launch_z_force<D>(cudaStream_t, int, const void *, const float *, const void *,   \
-                                    const int *, void *, DevScalars *, double *, int, int);          \
+    template void launch_exact_sv<D>(cudaStream_t, int, const void *, float4 *);                    \
+    template void launch_z_force<D>(cudaStream_t, int, const void *, const float4 *, const int *,   \
+                                    void *, DevScalars *, double *, int, int);          \
     template void launch_kl<D>(cudaStream_t, int, const int *, const int *, const float *,          \
                                const void *, double, DevScalars *, double *);                       \
     template void launch_attr_only<D>(cudaStream_t, int, const int *, const int *, const float *,   \

@@ -131,8 +131,7 @@ struct tsne_workspace {
     DevBuf<float> val, val2;
     DevBuf<unsigned char> Y, Yn, uY, gains, rep, frc, tmpv, Yconv;
     DevBuf<unsigned char> attr;     // attractive sums of a rebuild iteration (computed during the build)
-    DevBuf<float> s;
-    DevBuf<unsigned char> v;
+    DevBuf<float4> sv;              // exact sums (s, v) per point
     DevBuf<DevScalars> sc;
     HostPinned<DevScalars> hsc;
     DevBuf<double> part, zpart, klpart, convpart;
@@ -419,11 +418,10 @@ void renumber(tsne_workspace *ws, const int *ord_dev)
 template <int D>
 void exact_force(tsne_workspace *ws)
 {
-    ws->s.exact(ws->n);
-    ws->v.exact(ws->vbytes * ws->n);
+    ws->sv.exact(ws->n);
     ws->frc.exact(ws->vbytes * ws->n);
-    launch_exact_sv<D>(ws->st, ws->n, ws->Y.p, ws->s.p, ws->v.p);
-    launch_z_force<D>(ws->st, ws->n, ws->Y.p, ws->s.p, ws->v.p, nullptr, ws->frc.p, ws->sc.p, ws->zpart.p, 0, 0);
+    launch_exact_sv<D>(ws->st, ws->n, ws->Y.p, ws->sv.p);
+    launch_z_force<D>(ws->st, ws->n, ws->Y.p, ws->sv.p, nullptr, ws->frc.p, ws->sc.p, ws->zpart.p, 0, 0);
     ws->n_launch += 3;
 }
 

@@ -52,8 +52,12 @@ struct TreeView {
     int *blkcnt, *blkoff;    // per block of TREE_BLOCK points, 2 x 32 counts / offsets
     int *bset, *nid;         // per level l: boundary starts B_l and their node ids (stride cap_node)
     int *btot;               // |B_l|
+    int *tickets;            // work-item counters of the dependency-ordered launches
     TreeInfo *info;
 };
+
+// each is zeroed by a kernel that runs before the launch that draws from it
+enum { TICKET_LISTS = 0, TICKET_BASES = 1, TICKET_DOWN = 2, N_TICKET = 3 };
 
 __device__ __forceinline__ void fma4(float4 &acc, float w, const float4 &v)
 {
@@ -66,7 +70,14 @@ __device__ __forceinline__ void add4(float4 &a, const float4 &b) { a.x += b.x; a
 // root box and keys
 // ---------------------------------------------------------------------------------
 template <int D>
-__global__ void __launch_bounds__(256) k_bbox(int n, const Vec<D> *__restrict__ Y, double *__restrict__ part)
+__device__ void root_from_parts(int n, int nblk, const double *part, const TreeView &tv);
+
+// Bounding box in one launch: a grid of partial boxes, and the block that finishes last reduces
+// them to the root box and writes the root node (`done` counts the finished blocks and is left
+// at zero for the next launch). A second launch for the root alone cost 5 us plus its gap.
+template <int D>
+__global__ void __launch_bounds__(256) k_bbox(int n, const Vec<D> *__restrict__ Y, double *__restrict__ part,
+                                              TreeView tv, int *__restrict__ done)
 {
     float lo[D], hi[D];
     int bad = 0;
@@ -101,22 +112,30 @@ __global__ void __launch_bounds__(256) k_bbox(int n, const Vec<D> *__restrict__ 
             part[(size_t)blockIdx.x * (2 * D + 1) + D + k] = sh[0][k];
         }
         part[(size_t)blockIdx.x * (2 * D + 1) + 2 * D] = sb[0];
+        __threadfence();
+        sb[1] = atomicAdd(done, 1) == (int)gridDim.x - 1;
     }
+    __syncthreads();
+    if (!sb[1]) return;
+    __threadfence();
+    root_from_parts<D>(n, gridDim.x, part, tv);
+    if (threadIdx.x == 0) *done = 0;
 }
 
-// Root box from the bounding box (min / max are exact in any order), then the root node.
+// Root box from the bounding box (min / max are exact in any order), then the root node; the
+// counters that the build's later kernels add to are cleared here.
 template <int D>
-__global__ void __launch_bounds__(256) k_root(int n, int L, int nblk, const double *__restrict__ part, TreeView tv)
+__device__ void root_from_parts(int n, int nblk, const double *part, const TreeView &tv)
 {
     __shared__ double slo[256][D], shi[256][D], sbad[256];
     double lo[D], hi[D], bad = 0.0;
     for (int k = 0; k < D; k++) { lo[k] = INFINITY; hi[k] = -INFINITY; }
     for (int b = threadIdx.x; b < nblk; b += blockDim.x) {
         for (int k = 0; k < D; k++) {
-            lo[k] = fmin(lo[k], part[(size_t)b * (2 * D + 1) + k]);
-            hi[k] = fmax(hi[k], part[(size_t)b * (2 * D + 1) + D + k]);
+            lo[k] = fmin(lo[k], __ldcg(part + (size_t)b * (2 * D + 1) + k));
+            hi[k] = fmax(hi[k], __ldcg(part + (size_t)b * (2 * D + 1) + D + k));
         }
-        bad += part[(size_t)b * (2 * D + 1) + 2 * D];
+        bad += __ldcg(part + (size_t)b * (2 * D + 1) + 2 * D);
     }
     for (int k = 0; k < D; k++) { slo[threadIdx.x][k] = lo[k]; shi[threadIdx.x][k] = hi[k]; }
     sbad[threadIdx.x] = bad;
@@ -149,6 +168,8 @@ __global__ void __launch_bounds__(256) k_root(int n, int L, int nblk, const doub
     info->max_leaf = 0;
     info->nset_overflow = 0;
     info->pad[0] = 0;   // node-capacity overflow
+    info->pad[2] = 0;   // list slot overflow
+    tv.tickets[TICKET_LISTS] = 0;
     for (int l = 0; l < 32; l++) info->n_level_nodes[l] = 0;
     for (int l = 0; l < 33; l++) info->level_begin[l] = 0;
     info->n_level_nodes[0] = 1;
@@ -298,7 +319,7 @@ __global__ void __launch_bounds__(TREE_BLOCK) k_tree_marks(TreeView tv)
 // Exclusive scans of the 64 per-block count columns (a CTA per column; each thread takes a
 // contiguous run of blocks, then a block-wide scan of the runs). Column totals: the node
 // counts per level (columns 0-31) into btot[32 + l], the boundary counts |B_l| (columns 32-63)
-// into btot[l]; k_tree_levels turns the level counts into the node table's level ranges.
+// into btot[l]; every block of k_tree_emit turns the level counts into the level ranges.
 constexpr int TREE_SCAN_THREADS = 1024;
 
 __global__ void __launch_bounds__(TREE_SCAN_THREADS) k_tree_scan(int nblk, TreeView tv)
@@ -339,40 +360,44 @@ __global__ void __launch_bounds__(TREE_SCAN_THREADS) k_tree_scan(int nblk, TreeV
     }
 }
 
-__global__ void k_tree_levels(TreeView tv)
-{
-    if (threadIdx.x != 0) return;
-    TreeInfo *info = tv.info;
-    int acc = 0, maxl = 0;
-    for (int l = 0; l < 32; l++) {
-        const int c = l <= tv.L ? tv.btot[32 + l] : 0;
-        info->level_begin[l] = acc;
-        info->n_level_nodes[l] = c;
-        if (c > 0) maxl = l;
-        acc += c;
-    }
-    info->level_begin[32] = acc;
-    info->n_node = acc;
-    info->max_level = maxl;
-    if (acc > tv.cap_node) {   // node table full: the host regrows it; nothing downstream runs
-        info->pad[0] = 1;
-        info->n_node = 0;
-        info->max_level = 0;
-        for (int l = 0; l < 32; l++) info->n_level_nodes[l] = 0;
-    }
-}
-
 // numbers the nodes and writes their start, level, leaf flag, box index and first child;
-// end, parent and child count are stored as positions in the boundary lists for k_tree_finish
+// end, parent and child count are stored as positions in the boundary lists for k_tree_finish.
+// Every block scans the 32 level counts itself (a warp; no launch of its own for that), block 0
+// writes the level table.
 template <int D>
 __global__ void __launch_bounds__(TREE_BLOCK) k_tree_emit(TreeView tv)
 {
     __shared__ int wo[2][32][TREE_BLOCK / 32];
-    const TreeInfo *info = tv.info;
-    if (info->pad[0]) return;
+    __shared__ int sboff[2][32], slb[32], s_over;
     const int n = tv.n, L = tv.L;
     const int s = blockIdx.x * TREE_BLOCK + threadIdx.x;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    if (w == 0) {   // level ranges
+        const int c = lane <= L ? tv.btot[32 + lane] : 0;
+        int x = c;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        const int total = __shfl_sync(0xffffffffu, x, 31);
+        const unsigned used = __ballot_sync(0xffffffffu, c > 0);
+        const int over = total > tv.cap_node;   // node table full: the host regrows it; nothing downstream runs
+        slb[lane] = x - c;
+        if (lane == 0) s_over = over;
+        if (blockIdx.x == 0) {
+            TreeInfo *info = tv.info;
+            info->level_begin[lane] = x - c;
+            info->n_level_nodes[lane] = over ? 0 : c;
+            if (lane == 0) {
+                info->level_begin[32] = total;
+                info->n_node = over ? 0 : total;
+                info->max_level = over ? 0 : 31 - __clz((int)used);
+                if (over) info->pad[0] = 1;
+            }
+        }
+    }
+    __syncthreads();
+    if (s_over) return;
     const unsigned lt = (1u << lane) - 1u;
     const int fm = s < n ? tv.fm[s] : -1;
     for (int l = 0; l <= L; l++) {
@@ -382,7 +407,6 @@ __global__ void __launch_bounds__(TREE_BLOCK) k_tree_emit(TreeView tv)
         if (lane == 0) { wo[0][l][w] = __popc(vn); wo[1][l][w] = __popc(vb); }
     }
     __syncthreads();
-    __shared__ int sboff[2][32], slb[32];
     if (threadIdx.x < 64) {   // exclusive scan over the warps, per array and level
         const int arr = threadIdx.x >> 5, l = threadIdx.x & 31;
         if (l <= L) {
@@ -391,7 +415,6 @@ __global__ void __launch_bounds__(TREE_BLOCK) k_tree_emit(TreeView tv)
         }
         // the block's level offsets, read once (not once per level by every warp)
         sboff[arr][l] = l <= L ? tv.blkoff[((size_t)blockIdx.x * 2 + arr) * 32 + l] : 0;
-        if (arr == 0) slb[l] = info->level_begin[l];
     }
     __syncthreads();
     const size_t cap = (size_t)tv.cap_node;
@@ -750,39 +773,144 @@ __global__ void __launch_bounds__(256) k_lists_compact(TreeView tv, ListOut lo)
     }
 }
 
-// rows of each node's interpolation matrix: a leaf's points, or (upper bound) the
-// children's skeletons; nodes above MIN_ADM_LEVEL are not compressed
-// iflag / lflag / bflag: 1 for the internal nodes / leaves of at most LEAF_SMALL (3D:
-// ID3_TINY_LEAF) points / larger leaves at level >= MIN_ADM_LEVEL (the items of the basis
-// launches)
+// Positions of every node's entries, from its counts: far_ptr, near_ptr (list segments), rowoff
+// (its rows of the interpolation matrices: a leaf's points, or the upper bound of the children's
+// skeletons; nodes above MIN_ADM_LEVEL have none) and the item lists of the basis launches
+// (ilist: the internal nodes at level >= MIN_ADM_LEVEL; llist / blist: the leaves there of at most
+// LEAF_SMALL (3D: ID3_TINY_LEAF) points / the larger ones), each list in increasing node id.
+// Two launches over the nodes there are (block sums, then every block adds the sums before its
+// own): six device-wide scans over the node capacity and their flag and memset launches took
+// 25 launches, 75 us of a rebuild at 20K points and 85 us at 1M.
 constexpr int LEAF_SMALL = 64;
 constexpr int ID3_TINY_LEAF = 32;   // 3D: the leaves of the smallest basis CTAs
-template <int D>
-__global__ void k_rowcap(TreeView tv, int *__restrict__ rowcap, int *__restrict__ iflag, int *__restrict__ lflag,
-                         int *__restrict__ bflag)
+constexpr int NODE_BLOCK = 1024;
+
+struct NodeSums {
+    long long rows;
+    int far, near, in, small, big, pad;
+};
+struct NodeScan {
+    const int *far_cnt, *near_cnt;
+    int *far_ptr, *near_ptr;
+    long long *rowoff;
+    int *ilist, *llist, *blist, *rank;
+    NodeSums *blk;
+};
+
+__device__ __forceinline__ NodeSums node_add(const NodeSums &a, const NodeSums &b)
 {
-    constexpr int NCH = 1 << D;
-    const int n_node = tv.info->n_node;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n_node; t += gridDim.x * blockDim.x) {
-        int r = 0;
-        const bool adm = tv.level[t] >= MIN_ADM_LEVEL;
-        if (adm) r = tv.leaf[t] ? tv.end[t] - tv.start[t] : NCH * Dim<D>::MAXR;
-        rowcap[t] = r;
-        iflag[t] = adm && !tv.leaf[t];
-        const int small = D == 2 ? LEAF_SMALL : ID3_TINY_LEAF;
-        lflag[t] = adm && tv.leaf[t] && r <= small;
-        bflag[t] = adm && tv.leaf[t] && r > small;
+    NodeSums c;
+    c.rows = a.rows + b.rows;
+    c.far = a.far + b.far; c.near = a.near + b.near;
+    c.in = a.in + b.in; c.small = a.small + b.small; c.big = a.big + b.big; c.pad = 0;
+    return c;
+}
+__device__ __forceinline__ NodeSums node_shfl_up(const NodeSums &a, int o)
+{
+    NodeSums c;
+    c.rows = __shfl_up_sync(0xffffffffu, a.rows, o);
+    c.far = __shfl_up_sync(0xffffffffu, a.far, o);
+    c.near = __shfl_up_sync(0xffffffffu, a.near, o);
+    c.in = __shfl_up_sync(0xffffffffu, a.in, o);
+    c.small = __shfl_up_sync(0xffffffffu, a.small, o);
+    c.big = __shfl_up_sync(0xffffffffu, a.big, o);
+    c.pad = 0;
+    return c;
+}
+__device__ __forceinline__ NodeSums node_zero()
+{
+    NodeSums c;
+    c.rows = 0; c.far = c.near = c.in = c.small = c.big = c.pad = 0;
+    return c;
+}
+template <int D>
+__device__ __forceinline__ NodeSums node_counts(const TreeView &tv, const NodeScan &q, int t)
+{
+    NodeSums c = node_zero();
+    c.far = q.far_cnt[t];
+    c.near = q.near_cnt[t];
+    if (tv.level[t] < MIN_ADM_LEVEL) return c;
+    if (!tv.leaf[t]) {
+        c.rows = (1 << D) * Dim<D>::MAXR;
+        c.in = 1;
+    } else {
+        const int r = tv.end[t] - tv.start[t];
+        c.rows = r;
+        if (r <= (D == 2 ? LEAF_SMALL : ID3_TINY_LEAF)) c.small = 1;
+        else c.big = 1;
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) { rowcap[n_node] = 0; iflag[n_node] = 0; lflag[n_node] = 0; bflag[n_node] = 0; }
+    return c;
+}
+// inclusive scan over the block; `total` receives the block's sum in every thread
+__device__ __forceinline__ NodeSums node_block_scan(NodeSums x, NodeSums *sh, NodeSums &total)
+{
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    for (int o = 1; o < 32; o <<= 1) {
+        const NodeSums y = node_shfl_up(x, o);
+        if (lane >= o) x = node_add(x, y);
+    }
+    if (lane == 31) sh[w] = x;
+    __syncthreads();
+    if (w == 0) {
+        NodeSums v = sh[lane];
+        for (int o = 1; o < 32; o <<= 1) {
+            const NodeSums y = node_shfl_up(v, o);
+            if (lane >= o) v = node_add(v, y);
+        }
+        sh[lane] = v;
+    }
+    __syncthreads();
+    total = sh[31];
+    if (w > 0) x = node_add(x, sh[w - 1]);
+    __syncthreads();
+    return x;
 }
 
-// ids of the flagged nodes in increasing order
-__global__ void k_flag_list(const int *__restrict__ n_node_p, const int *__restrict__ flag,
-                            const int *__restrict__ pos, int *__restrict__ list)
+template <int D>
+__global__ void __launch_bounds__(NODE_BLOCK) k_node_sums(TreeView tv, NodeScan q)
 {
-    const int n_node = *n_node_p;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n_node; t += gridDim.x * blockDim.x)
-        if (flag[t]) list[pos[t]] = t;
+    __shared__ NodeSums sh[32];
+    const int n_node = tv.info->n_node, t = blockIdx.x * NODE_BLOCK + threadIdx.x;
+    if (blockIdx.x * NODE_BLOCK >= n_node) return;
+    NodeSums total;
+    node_block_scan(t < n_node ? node_counts<D>(tv, q, t) : node_zero(), sh, total);
+    if (threadIdx.x == 0) q.blk[blockIdx.x] = total;
+}
+
+template <int D>
+__global__ void __launch_bounds__(NODE_BLOCK) k_node_scan(TreeView tv, NodeScan q)
+{
+    __shared__ NodeSums sh[32];
+    TreeInfo *info = tv.info;
+    const int n_node = info->n_node, t = blockIdx.x * NODE_BLOCK + threadIdx.x;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        q.far_ptr[0] = 0; q.near_ptr[0] = 0; q.rowoff[0] = 0;
+        tv.tickets[TICKET_BASES] = 0;
+        if (n_node == 0) { info->n_far = info->n_near = info->n_int = info->n_small = info->n_big = 0; info->n_rows = 0; }
+    }
+    if (blockIdx.x * NODE_BLOCK >= n_node) return;
+    // the blocks before this one
+    NodeSums before = node_zero(), total;
+    for (int b = threadIdx.x; b < (int)blockIdx.x; b += NODE_BLOCK) before = node_add(before, q.blk[b]);
+    node_block_scan(before, sh, before);
+    const NodeSums own = t < n_node ? node_counts<D>(tv, q, t) : node_zero();
+    const NodeSums inc = node_add(node_block_scan(own, sh, total), before);
+    if (t >= n_node) return;
+    q.far_ptr[t + 1] = inc.far;
+    q.near_ptr[t + 1] = inc.near;
+    q.rowoff[t + 1] = inc.rows;
+    if (own.in) q.ilist[inc.in - 1] = t;
+    if (own.small) q.llist[inc.small - 1] = t;
+    if (own.big) q.blist[inc.big - 1] = t;
+    if (tv.level[t] < MIN_ADM_LEVEL) q.rank[t] = 0;   // no basis; the others' ranks come with theirs
+    if (t == n_node - 1) {
+        info->n_far = inc.far;
+        info->n_near = inc.near;
+        info->n_rows = inc.rows;
+        info->n_int = inc.in;
+        info->n_small = inc.small;
+        info->n_big = inc.big;
+    }
 }
 
 // ---------------------------------------------------------------------------------
@@ -1942,6 +2070,7 @@ __global__ void __launch_bounds__(256) k_far_c(int first, int n_node, ProdArgs g
     const Vec<D> *xt = (const Vec<D> *)g.xt;
     const Vec<D> *skel = (const Vec<D> *)g.skel;
     const int lane = threadIdx.x & 31;
+    if (blockIdx.x == 0 && threadIdx.x == 0) tv.tickets[TICKET_DOWN] = 0;   // for the downward pass
     for (int t = first + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); t < n_node;
          t += (gridDim.x * blockDim.x) >> 5) {
         const int r = g.rank[t], lt = tv.level[t];
@@ -2288,19 +2417,6 @@ __global__ void __launch_bounds__(256) k_down_leaves(ProdArgs g)
     }
 }
 
-template <int D>
-__global__ void k_split_out(int n, const float4 *__restrict__ yp, float *__restrict__ s, Vec<D> *__restrict__ v)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 a = yp[i];
-        s[i] = a.x;
-        Vec<D> o;
-        if constexpr (D == 2) o = make_float2(a.y, a.z);
-        else o = make_float4(a.y, a.z, a.w, 0.f);
-        v[i] = o;
-    }
-}
-
 inline int grid_for(long long work, int block, int cap = 148 * 16)
 {
     long long g = (work + block - 1) / block;
@@ -2334,24 +2450,25 @@ public:
         TSNE_CUDA_CHECK(cudaEventCreateWithFlags(&near_ev_, cudaEventDisableTiming));
         TSNE_CUDA_CHECK(cudaEventCreateWithFlags(&lists_ev_, cudaEventDisableTiming));
         keys_in_.exact(n); keys_.exact(n); idx_in_.exact(n); perm_.exact(n); xt_.exact(n);
-        yp_.exact(n); s_.exact(n); v_.exact(n);
+        yp_.exact(n);
         bbox_part_.exact((size_t)BBOX_BLOCKS * (2 * D + 1));
         delta_.exact((size_t)n + 1);
         fm_.exact(n);
         blkcnt_.exact((size_t)ceil_div(n, TREE_BLOCK) * 64);
         blkoff_.exact((size_t)ceil_div(n, TREE_BLOCK) * 64);
         btot_.exact(64);
-        ticket_.exact(1);
+        tickets_.exact(N_TICKET);
+        done_.exact(1);
+        TSNE_CUDA_CHECK(cudaMemsetAsync(tickets_.p, 0, sizeof(int) * N_TICKET, st_));
+        TSNE_CUDA_CHECK(cudaMemsetAsync(done_.p, 0, sizeof(int), st_));
         info_.exact(1);
         TSNE_CUDA_CHECK(cudaMemsetAsync(info_.p, 0, sizeof(TreeInfo), st_));
         TSNE_CUDA_CHECK(cudaEventCreateWithFlags(&counts_ev_, cudaEventDisableTiming));
-        size_t b1 = 0, b2 = 0;
+        size_t b1 = 0;
         TSNE_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(nullptr, b1, keys_in_.p, keys_.p, idx_in_.p,
                                                         perm_.p, n, 0, D * Dim<D>::L, st_));
-        TSNE_CUDA_CHECK(cub::DeviceScan::InclusiveSum(nullptr, b2, (int *)nullptr, (int *)nullptr,
-                                                      n + 1, st_));
         sort_bytes_ = b1;
-        cub_tmp_.exact(std::max(b1, b2) + 256);
+        cub_tmp_.exact(b1 + 256);
         cap_node_ = std::max(1024, 4 * (n / 16) + 1024);
         nset_cap_ = Dim<D>::NSET;
         alloc_nodes();
@@ -2382,15 +2499,14 @@ public:
         sec_begin();
         // One batch: root box, keys, sort, the whole tree (four kernels over the points, no level
         // loop) and the counting pass of the interaction lists (kernels read the level and node
-        // counts on the device; scans run over the node capacity, whose unused tail counts are
-        // zero), then a single synchronisation reads the tree, the list totals and the basis
-        // rows. A full node table or a full inadmissible-source set are caught there and redone.
+        // counts on the device), then one copy to pinned memory and one wait bring the tree, the
+        // list totals and the basis rows (TreeInfo): copies to pageable members held the host,
+        // and with it the work queued to overlap the wait, for about 50 us per rebuild. A full node table or a full inadmissible-source set are caught there and redone.
         bool tree_ok = false;
         for (int attempt = 0; attempt < 12; attempt++) {
             if (!tree_ok) {
                 const int nblk = ceil_div(n_, TREE_BLOCK);
-                k_bbox<D><<<BBOX_BLOCKS, 256, 0, st_>>>(n_, (const Vec<D> *)Y, bbox_part_.p);
-                k_root<D><<<1, 256, 0, st_>>>(n_, L, BBOX_BLOCKS, bbox_part_.p, view());
+                k_bbox<D><<<BBOX_BLOCKS, 256, 0, st_>>>(n_, (const Vec<D> *)Y, bbox_part_.p, view(), done_.p);
                 k_keys<D><<<grid_for(n_, 256), 256, 0, st_>>>(n_, L, (const Vec<D> *)Y, info_.p, keys_in_.p, idx_in_.p);
                 size_t bytes = sort_bytes_;
                 TSNE_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(cub_tmp_.p, bytes, keys_in_.p, keys_.p, idx_in_.p,
@@ -2399,20 +2515,13 @@ public:
                                                                      (Vec<D> *)xt_.p, keys_.p, delta_.p);
                 k_tree_marks<D><<<nblk, TREE_BLOCK, 0, st_>>>(view());
                 k_tree_scan<<<64, TREE_SCAN_THREADS, 0, st_>>>(nblk, view());
-                k_tree_levels<<<1, 32, 0, st_>>>(view());
                 k_tree_emit<D><<<nblk, TREE_BLOCK, 0, st_>>>(view());
                 k_tree_finish<D><<<grid_for(cap_node_, 256, 148 * 8), 256, 0, st_>>>(view());
-                launches_ += 10 + 4;
+                launches_ += 8 + 4;
                 tree_ok = true;
             }
             launch_list_counts();
             TSNE_CUDA_CHECK(cudaMemcpyAsync(hinfo_.p, info_.p, sizeof(TreeInfo), cudaMemcpyDeviceToHost, st_));
-            TSNE_CUDA_CHECK(cudaMemcpyAsync(&htot_[0], far_ptr_.p + cap_node_, sizeof(int), cudaMemcpyDeviceToHost, st_));
-            TSNE_CUDA_CHECK(cudaMemcpyAsync(&htot_[1], near_ptr_.p + cap_node_, sizeof(int), cudaMemcpyDeviceToHost, st_));
-            TSNE_CUDA_CHECK(cudaMemcpyAsync(&hrows_, rowoff_.p + cap_node_, sizeof(long long), cudaMemcpyDeviceToHost, st_));
-            TSNE_CUDA_CHECK(cudaMemcpyAsync(&hint_, ipos_.p + cap_node_, sizeof(int), cudaMemcpyDeviceToHost, st_));
-            TSNE_CUDA_CHECK(cudaMemcpyAsync(&hleaf_, lpos_.p + cap_node_, sizeof(int), cudaMemcpyDeviceToHost, st_));
-            TSNE_CUDA_CHECK(cudaMemcpyAsync(&hbig_, bpos_.p + cap_node_, sizeof(int), cudaMemcpyDeviceToHost, st_));
             TSNE_CUDA_CHECK(cudaEventRecord(counts_ev_, st_));
             if (overlap != nullptr && *overlap) {
                 (*overlap)();
@@ -2434,7 +2543,12 @@ public:
             if (I.nset_overflow) {   // inadmissible-source set full: grow, recount
                 nset_cap_ *= 2;
                 alloc_lists();
-                if (attempt < 11) continue;
+                if (attempt < 11) {   // the counters that the root kernel cleared for the first count
+                    TSNE_CUDA_CHECK(cudaMemsetAsync(&info_.p->nset_overflow, 0, sizeof(int), st_));
+                    TSNE_CUDA_CHECK(cudaMemsetAsync(&info_.p->pad[2], 0, sizeof(int), st_));
+                    TSNE_CUDA_CHECK(cudaMemsetAsync(&tickets_.p[TICKET_LISTS], 0, sizeof(int), st_));
+                    continue;
+                }
             }
             break;
         }
@@ -2447,6 +2561,10 @@ public:
         stats_.n_node = n_node_;
         stats_.max_level = max_level_;
         stats_.max_leaf = I.max_leaf;
+        hrows_ = I.n_rows;
+        hint_ = I.n_int;
+        hleaf_ = I.n_small;
+        hbig_ = I.n_big;
         if (max_level_ <= 2) { built_ = false; return 1; }
 
         // The list write (and in 3D the segmented sort of each target's entries) needs only the
@@ -2454,8 +2572,8 @@ public:
         // bases; the near blocks follow it there. Its buffers are allocated first, in the
         // workspace stream's order (the stream-ordered pool), and the side stream starts from
         // that point. Readers on the workspace stream join it first (join_lists).
-        stats_.n_far = htot_[0];
-        stats_.n_near = htot_[1];
+        stats_.n_far = htot_[0] = I.n_far;
+        stats_.n_near = htot_[1] = I.n_near;
         far_idx_.ensure(std::max(1, htot_[0]));
         near_idx_.ensure(std::max(1, htot_[1]));
         if (D == 3) {
@@ -2485,8 +2603,6 @@ public:
         // bases, bottom-up
         cudaEvent_t t_bases = mark_begin();
         constexpr int MAXR = Dim<D>::MAXR, P = Dim<D>::NPROXY;
-        rank_.exact(n_node_);
-        TSNE_CUDA_CHECK(cudaMemsetAsync(rank_.p, 0, sizeof(int) * n_node_, st_));
         skel_.ensure((size_t)n_node_ * MAXR);
         y0_.ensure((size_t)n_node_ * MAXR);
         y1_.ensure((size_t)n_node_ * MAXR);
@@ -2509,7 +2625,7 @@ public:
         if (D == 2 && stats_.max_leaf <= ID2_THREADS) {
             // leaves in one launch, then the internal nodes of every level in one
             // dependency-ordered launch
-            DepArgs dp{flag_.p, ticket_.p, &info_.p->pad[1], ++epoch_};
+            DepArgs dp{flag_.p, tickets_.p + TICKET_BASES, &info_.p->pad[1], ++epoch_};
             if (hleaf_ > 0)
                 k_id2d<true, ID2_SMALL><<<hleaf_, ID2_SMALL, id2_smem(ID2_SMALL), st_>>>(hleaf_, llist_.p, il, dp);
             if (hbig_ > 0)
@@ -2527,7 +2643,6 @@ public:
                     launches_++;
                 }
             } else if (hint_ > 0) {
-                TSNE_CUDA_CHECK(cudaMemsetAsync(ticket_.p, 0, sizeof(int), st_));
                 DepArgs d2 = dp;
                 d2.flag2 = flag2_.p;
                 k_id2d<false, ID2_THREADS><<<hint_, ID2_THREADS, id2_smem(ID2_THREADS), st_>>>(hint_, ilist_.p, il, d2);
@@ -2542,7 +2657,7 @@ public:
             rank_stats_valid_ = false;
             return 0;
         }
-        DepArgs dp{flag_.p, ticket_.p, &info_.p->pad[1], ++epoch_};
+        DepArgs dp{flag_.p, tickets_.p + TICKET_BASES, &info_.p->pad[1], ++epoch_};
         if (D == 3 && id3_) {
             // recomputed-row decompositions: leaves by size (llist: at most ID3_TINY points;
             // blist: the others, up to ID3_ROWS; larger leaves, only at the depth limit, take
@@ -2562,7 +2677,6 @@ public:
             t_bases = mark_begin();
             near_fork_point();
             if (hint_ > 0) {
-                TSNE_CUDA_CHECK(cudaMemsetAsync(ticket_.p, 0, sizeof(int), st_));
                 DepArgs d2 = dp;
                 d2.flag2 = flag2_.p;
                 id3_launch<false, 512, ID3_ROWS>(hint_, ilist_.p, 0, il, d2);
@@ -2585,7 +2699,6 @@ public:
         IdArgs ia = il;
         ia.mcap = mcap;
         if (hint_ > 0) {
-            TSNE_CUDA_CHECK(cudaMemsetAsync(ticket_.p, 0, sizeof(int), st_));
             k_id<D, false><<<hint_, IDG_THREADS, id_smem_bytes<D>(mcap), st_>>>(0, ia, hint_, ilist_.p, dp);
             launches_++;
         }
@@ -2598,35 +2711,20 @@ public:
         return 0;
     }
 
-    // counting pass of the lists (internal targets, then every leaf target), the pointer
-    // scans and the basis row offsets, all over the node capacity
+    // counting pass of the lists (internal targets, then every leaf target), the list pointers,
+    // the basis row offsets and the basis launches' item lists
     void launch_list_counts()
     {
-        TSNE_CUDA_CHECK(cudaMemsetAsync(far_cnt_.p, 0, sizeof(int) * (cap_node_ + 1), st_));
-        TSNE_CUDA_CHECK(cudaMemsetAsync(near_cnt_.p, 0, sizeof(int) * (cap_node_ + 1), st_));
-        TSNE_CUDA_CHECK(cudaMemsetAsync(rowcap_.p, 0, sizeof(int) * (cap_node_ + 1), st_));
-        TSNE_CUDA_CHECK(cudaMemsetAsync(&info_.p->nset_overflow, 0, sizeof(int), st_));
-        TSNE_CUDA_CHECK(cudaMemsetAsync(&info_.p->pad[2], 0, sizeof(int), st_));
         ListOut lo = list_out(0);
-        TSNE_CUDA_CHECK(cudaMemsetAsync(ticket_.p, 0, sizeof(int), st_));
-        DepArgs dp{flag_.p, ticket_.p, &info_.p->pad[1], ++epoch_};
+        DepArgs dp{flag_.p, tickets_.p + TICKET_LISTS, &info_.p->pad[1], ++epoch_};
         k_lists_internal<D><<<148 * 4, 256, 0, st_>>>(view(), lo, dp);
         k_lists_leaves<D><<<148 * 8, 128, 0, st_>>>(view(), lo);
-        launches_ += 2;
-        TSNE_CUDA_CHECK(cudaMemsetAsync(iflag_.p, 0, sizeof(int) * (cap_node_ + 1), st_));
-        TSNE_CUDA_CHECK(cudaMemsetAsync(lflag_.p, 0, sizeof(int) * (cap_node_ + 1), st_));
-        TSNE_CUDA_CHECK(cudaMemsetAsync(bflag_.p, 0, sizeof(int) * (cap_node_ + 1), st_));
-        k_rowcap<D><<<148 * 4, 256, 0, st_>>>(view(), rowcap_.p, iflag_.p, lflag_.p, bflag_.p);
-        scan_exclusive(far_cnt_.p, far_ptr_.p, cap_node_);
-        scan_exclusive(near_cnt_.p, near_ptr_.p, cap_node_);
-        scan_exclusive_ll(rowcap_.p, rowoff_.p, cap_node_);
-        scan_exclusive(iflag_.p, ipos_.p, cap_node_);
-        scan_exclusive(lflag_.p, lpos_.p, cap_node_);
-        scan_exclusive(bflag_.p, bpos_.p, cap_node_);
-        k_flag_list<<<148 * 4, 256, 0, st_>>>(&info_.p->n_node, iflag_.p, ipos_.p, ilist_.p);
-        k_flag_list<<<148 * 4, 256, 0, st_>>>(&info_.p->n_node, lflag_.p, lpos_.p, llist_.p);
-        k_flag_list<<<148 * 4, 256, 0, st_>>>(&info_.p->n_node, bflag_.p, bpos_.p, blist_.p);
-        launches_ += 12;
+        const NodeScan q{far_cnt_.p, near_cnt_.p, far_ptr_.p, near_ptr_.p, rowoff_.p, ilist_.p, llist_.p, blist_.p,
+                         rank_.p, node_blk_.p};
+        const int nb = ceil_div(cap_node_, NODE_BLOCK);
+        k_node_sums<D><<<nb, NODE_BLOCK, 0, st_>>>(view(), q);
+        k_node_scan<D><<<nb, NODE_BLOCK, 0, st_>>>(view(), q);
+        launches_ += 4;
     }
 
     void alloc_lists()
@@ -2636,11 +2734,10 @@ public:
         nset_cnt_.exact(c + 1);
         far_cnt_.exact(c + 1); near_cnt_.exact(c + 1);
         far_ptr_.exact(c + 2); near_ptr_.exact(c + 2);
-        rowcap_.exact(c + 1);
-        iflag_.exact(c + 1); ipos_.exact(c + 2); ilist_.exact(c + 1);
-        lflag_.exact(c + 1); lpos_.exact(c + 2); llist_.exact(c + 1);
-        bflag_.exact(c + 1); bpos_.exact(c + 2); blist_.exact(c + 1);
+        ilist_.exact(c + 1); llist_.exact(c + 1); blist_.exact(c + 1);
         rowoff_.exact(c + 2);
+        rank_.exact(c);
+        node_blk_.exact(ceil_div(c, NODE_BLOCK));
         if (D == 2) {
             far_slot_.exact(c * LIST_SLOT);
             near_slot_.exact(c * LIST_SLOT);
@@ -2651,30 +2748,26 @@ public:
     {
         run_product();
         cudaEvent_t t_force = mark_begin();
-        k_split_out<D><<<grid_for(n_, 256), 256, 0, st_>>>(n_, yp_.p, s_.p, (Vec<D> *)v_.p);
-        launch_z_force<D>(st_, n_, xt_.p, s_.p, v_.p, perm_.p, F, sc, partials, 1, keep_rep);
-        launches_ += 3;
+        launch_z_force<D>(st_, n_, xt_.p, yp_.p, perm_.p, F, sc, partials, 1, keep_rep);
+        launches_ += 2;
         mark_end(t_force, 6);
     }
 
     void product_host(std::vector<float> &s, std::vector<float> &v) override
     {
         run_product();
-        k_split_out<D><<<grid_for(n_, 256), 256, 0, st_>>>(n_, yp_.p, s_.p, (Vec<D> *)v_.p);
-        std::vector<float> st(n_);
-        std::vector<Vec<D>> vt(n_);
+        std::vector<float4> yt(n_);
         std::vector<int> perm(n_);
-        TSNE_CUDA_CHECK(cudaMemcpyAsync(st.data(), s_.p, sizeof(float) * n_, cudaMemcpyDeviceToHost, st_));
-        TSNE_CUDA_CHECK(cudaMemcpyAsync(vt.data(), v_.p, sizeof(Vec<D>) * n_, cudaMemcpyDeviceToHost, st_));
+        TSNE_CUDA_CHECK(cudaMemcpyAsync(yt.data(), yp_.p, sizeof(float4) * n_, cudaMemcpyDeviceToHost, st_));
         TSNE_CUDA_CHECK(cudaMemcpyAsync(perm.data(), perm_.p, sizeof(int) * n_, cudaMemcpyDeviceToHost, st_));
         TSNE_CUDA_CHECK(cudaStreamSynchronize(st_));
         s.assign(n_, 0.f);
         v.assign((size_t)n_ * D, 0.f);
         for (int k = 0; k < n_; k++) {
             const int i = perm[k];
-            s[i] = st[k];
-            const float *vv = reinterpret_cast<const float *>(&vt[k]);
-            for (int c = 0; c < D; c++) v[(size_t)c * n_ + i] = vv[c];
+            const float *a = reinterpret_cast<const float *>(&yt[k]);   // s, v
+            s[i] = a[0];
+            for (int c = 0; c < D; c++) v[(size_t)c * n_ + i] = a[1 + c];
         }
     }
 
@@ -2771,7 +2864,7 @@ public:
     {
         if (n_node_ <= 0) return -1;
         // an epoch that no launch has published: the wait runs out after `polls` polls
-        DepArgs dp{flag_.p, ticket_.p, &info_.p->pad[1], epoch_ + (1 << 24), polls};
+        DepArgs dp{flag_.p, tickets_.p, &info_.p->pad[1], epoch_ + (1 << 24), polls};
         k_dep_probe<<<1, 32, 0, st_>>>(dp, 0);
         launches_++;
         return wait_failed();
@@ -2888,7 +2981,8 @@ private:
         v.keys = keys_.p; v.start = start_.p; v.end = end_.p; v.level = level_.p; v.parent = parent_.p;
         v.fchild = fchild_.p; v.nchild = nchild_.p; v.leaf = leaf_.p; v.ix = ix_.p;
         v.delta = delta_.p; v.fm = fm_.p; v.blkcnt = blkcnt_.p; v.blkoff = blkoff_.p;
-        v.bset = bset_.p; v.nid = nid_.p; v.btot = btot_.p; v.info = info_.p;
+        v.bset = bset_.p; v.nid = nid_.p; v.btot = btot_.p; v.tickets = tickets_.p;
+        v.info = info_.p;
         return v;
     }
 
@@ -2906,16 +3000,6 @@ private:
         return lo;
     }
 
-    // out[0] = 0, out[i + 1] = in[0] + ... + in[i]
-    void scan_exclusive(const int *in, int *out, int count)
-    {
-        TSNE_CUDA_CHECK(cudaMemsetAsync(out, 0, sizeof(int), st_));
-        size_t need = 0;
-        TSNE_CUDA_CHECK(cub::DeviceScan::InclusiveSum(nullptr, need, in, out + 1, count, st_));
-        if (need > cub_tmp_.cap) cub_tmp_.exact(need + 256);
-        size_t bytes = cub_tmp_.cap;
-        TSNE_CUDA_CHECK(cub::DeviceScan::InclusiveSum(cub_tmp_.p, bytes, in, out + 1, count, st_));
-    }
     void sort_reserve(DevBuf<int> &idx, DevBuf<int> &alt, int count, const int *ptr)
     {
         if (count <= 1) return;
@@ -2936,16 +3020,6 @@ private:
         if (keys.Current() != idx.p) idx.swap(alt);
         launches_ += 2;
     }
-    void scan_exclusive_ll(const int *in, long long *out, int count)
-    {
-        TSNE_CUDA_CHECK(cudaMemsetAsync(out, 0, sizeof(long long), st_));
-        size_t need = 0;
-        TSNE_CUDA_CHECK(cub::DeviceScan::InclusiveSum(nullptr, need, in, out + 1, count, st_));
-        if (need > cub_tmp_.cap) cub_tmp_.exact(need + 256);
-        size_t bytes = cub_tmp_.cap;
-        TSNE_CUDA_CHECK(cub::DeviceScan::InclusiveSum(cub_tmp_.p, bytes, in, out + 1, count, st_));
-    }
-
     ProdArgs prod_args(const float4 *xin)
     {
         ProdArgs g;
@@ -3015,8 +3089,7 @@ private:
         mark_end(t_near, 4);
         cudaEvent_t t_down = mark_begin();
         if (hint_ > 0) {
-            TSNE_CUDA_CHECK(cudaMemsetAsync(ticket_.p, 0, sizeof(int), st_));
-            DepArgs dp{flag_.p, ticket_.p, &info_.p->pad[1], ++epoch_};
+            DepArgs dp{flag_.p, tickets_.p + TICKET_DOWN, &info_.p->pad[1], ++epoch_};
             k_down_internal<D><<<grid_for((long long)hint_ * 32, 256, 148 * 8), 256, 0, st_>>>(hint_, ilist_.p, g, dp);
             launches_++;
         }
@@ -3053,7 +3126,8 @@ private:
     DevBuf<int> start_, end_, level_, parent_, fchild_, nchild_, leaf_, ix_;
     DevBuf<signed char> delta_;
     DevBuf<int> fm_, blkcnt_, blkoff_, bset_, nid_, btot_;
-    DevBuf<int> flag_, ticket_;   // dependency-ordered launches
+    DevBuf<int> flag_, tickets_;  // dependency-ordered launches
+    DevBuf<int> done_;            // finished blocks of the bounding-box launch
     DevBuf<int> flag2_;           // second flags (bases: upward coefficients final)
     cudaStream_t st2_ = nullptr;  // side stream: the list write and the near field beside the bases
     cudaEvent_t fork_ev_ = nullptr, near_ev_ = nullptr, lists_ev_ = nullptr;
@@ -3062,18 +3136,17 @@ private:
     int epoch_ = 0;
     DevBuf<int> nset_, nset_cnt_, far_cnt_, near_cnt_, far_ptr_, near_ptr_, far_idx_, near_idx_;
     DevBuf<int> far_alt_, near_alt_;   // segmented-sort partners of the 3D lists
-    DevBuf<int> rowcap_;
-    DevBuf<int> iflag_, ipos_, ilist_;   // internal nodes at level >= 2, in increasing id
-    DevBuf<int> lflag_, lpos_, llist_;   // leaves at level >= 2 of at most LEAF_SMALL points
-    DevBuf<int> bflag_, bpos_, blist_;   // the larger leaves at level >= 2
+    DevBuf<NodeSums> node_blk_;          // block sums of the node scan
+    DevBuf<int> ilist_;                  // internal nodes at level >= 2, in increasing id
+    DevBuf<int> llist_;                  // leaves at level >= 2 of at most LEAF_SMALL points
+    DevBuf<int> blist_;                  // the larger leaves at level >= 2
     int hint_ = 0, hleaf_ = 0, hbig_ = 0;
     cudaEvent_t counts_ev_ = nullptr;   // end of a build's count batch (host waits on it)
     DevBuf<long long> rowoff_;
     DevBuf<int> rank_;
     DevBuf<Vec<D>> skel_;
     DevBuf<float4> y0_, y1_, yp_, xin_;
-    DevBuf<float> U_, s_;
-    DevBuf<Vec<D>> v_;
+    DevBuf<float> U_;
     DevBuf<float> gA_, gnrm_;
     DevBuf<int> gsel_;
     DevBuf<Vec<D>> gcand_;

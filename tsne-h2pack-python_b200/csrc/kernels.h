@@ -32,6 +32,9 @@ struct TreeInfo {
     int pad[3];
     double corner[3];
     double radius;
+    // totals of the list counts and of the basis launches' items
+    long long n_rows;
+    int n_far, n_near, n_int, n_small, n_big;
 };
 
 // ---- dense per-point kernels (dense.cu) ----
@@ -51,9 +54,9 @@ template <int D>
 void launch_center(cudaStream_t st, int n, const void *Ynext, void *Ycur, const double *partials,
                    DevScalars *sc, const void *Yprev_conv, double *conv_partials);
 template <int D>
-void launch_exact_sv(cudaStream_t st, int n, const void *Y, float *s, void *v);
+void launch_exact_sv(cudaStream_t st, int n, const void *Y, float4 *sv);
 template <int D>
-void launch_z_force(cudaStream_t st, int n, const void *Ypts, const float *s, const void *v,
+void launch_z_force(cudaStream_t st, int n, const void *Ypts, const float4 *sv,
                     const int *perm, void *rep, DevScalars *sc, double *partials, int h2_path,
                     int keep_rep);
 template <int D>
