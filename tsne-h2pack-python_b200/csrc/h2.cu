@@ -47,6 +47,7 @@ struct TreeView {
     int n, L, leaf_size, cap_node, nset_cap;
     const unsigned long long *keys;
     int *start, *end, *level, *parent, *fchild, *nchild, *leaf, *ix;
+    int4 *rec;               // per node, packed for the list pass: see node_rec
     signed char *delta;      // shared leading digits with the previous key (n + 1)
     int *fm;                 // per point: first | last level << 8 of the nodes it starts, or -1
     int *blkcnt, *blkoff;    // per block of TREE_BLOCK points, 2 x 32 counts / offsets
@@ -450,7 +451,27 @@ __global__ void __launch_bounds__(TREE_BLOCK) k_tree_emit(TreeView tv)
     }
 }
 
-// end, parent and child count of every node from the boundary lists; the largest leaf
+// The node record of the list pass, two 16-byte loads for what lies in seven arrays:
+// [2t] = (first child, children | leaf << 8 | level << 16, parent, 0), [2t + 1] = box index.
+struct NodeRec {
+    int fchild, nchild, level, parent;
+    bool leaf;
+    int ix[3];
+};
+__device__ __forceinline__ NodeRec node_rec(const TreeView &tv, int t)
+{
+    const int4 a = __ldg(tv.rec + 2 * (size_t)t), b = __ldg(tv.rec + 2 * (size_t)t + 1);
+    NodeRec r;
+    r.fchild = a.x;
+    r.nchild = a.y & 0xff;
+    r.leaf = (a.y >> 8) & 1;
+    r.level = a.y >> 16;
+    r.parent = a.z;
+    r.ix[0] = b.x; r.ix[1] = b.y; r.ix[2] = b.z;
+    return r;
+}
+
+// end, parent and child count of every node from the boundary lists; its record; the largest leaf
 template <int D>
 __global__ void k_tree_finish(TreeView tv)
 {
@@ -462,15 +483,18 @@ __global__ void k_tree_finish(TreeView tv)
         const int l = tv.level[t], s = tv.start[t], pos = tv.end[t];
         const int e = pos + 1 < tv.btot[l] ? tv.bset[(size_t)l * cap + pos + 1] : tv.n;
         tv.end[t] = e;
-        if (l > 0) tv.parent[t] = tv.nid[(size_t)(l - 1) * cap + tv.parent[t]];
-        if (tv.leaf[t]) {
+        int par = -1, c = 0;
+        if (l > 0) tv.parent[t] = par = tv.nid[(size_t)(l - 1) * cap + tv.parent[t]];
+        const int lf = tv.leaf[t];
+        if (lf) {
             atomicMax(&info->max_leaf, e - s);
         } else {
             const int c0 = tv.nchild[t], lim = tv.btot[l + 1];
-            int c = 0;
             while (c0 + c < lim && tv.bset[(size_t)(l + 1) * cap + c0 + c] < e) c++;
             tv.nchild[t] = c;
         }
+        tv.rec[2 * (size_t)t] = make_int4(tv.fchild[t], c | lf << 8 | l << 16, par, 0);
+        tv.rec[2 * (size_t)t + 1] = make_int4(tv.ix[3 * (size_t)t], tv.ix[3 * (size_t)t + 1], tv.ix[3 * (size_t)t + 2], 0);
     }
 }
 
@@ -510,7 +534,7 @@ __device__ __forceinline__ void dep_wait(const DepArgs &dp, int node)
     const int *f = dp.flag + node;
     for (int it = 0; it < dp.limit; it++) {
         if (ld_acquire_gpu(f) == dp.epoch) return;
-        __nanosleep(100);
+        __nanosleep(it < 64 ? 32 : 128);
     }
     atomicExch(dp.err, 1);
 }
@@ -545,231 +569,247 @@ __global__ void k_dep_probe(DepArgs dp, int node)
 // interaction lists
 // ---------------------------------------------------------------------------------
 template <int D>
-__device__ __forceinline__ bool admissible(const TreeView &tv, int t, int s)
+__device__ __forceinline__ bool admissible(int L, const NodeRec &t, const NodeRec &s)
 {
-    const long long wt = 1LL << (tv.L - tv.level[t]);
-    const long long ws = 1LL << (tv.L - tv.level[s]);
+    const long long wt = 1LL << (L - t.level);
+    const long long ws = 1LL << (L - s.level);
     long long dist = 0;
+#pragma unroll
     for (int k = 0; k < D; k++) {
-        const long long ct = 2LL * tv.ix[(size_t)t * 3 + k] * wt + wt;
-        const long long cs = 2LL * tv.ix[(size_t)s * 3 + k] * ws + ws;
+        const long long ct = 2LL * t.ix[k] * wt + wt;
+        const long long cs = 2LL * s.ix[k] * ws + ws;
         const long long df = ct > cs ? ct - cs : cs - ct;
         dist = df > dist ? df : dist;
     }
     return dist >= wt + ws + (long long)ADM_EXTRA * (wt < ws ? wt : ws);
 }
 
-// 2D: the count pass also parks each target's entries in fixed slots of LIST_SLOT entries, so
-// that the list write is a compaction; a target with more entries sets slot_over and the build
-// falls back to the traversing write pass
-constexpr int LIST_SLOT = 128;
+// The count pass also parks each target's entries in fixed slots, so that the list write is a
+// compaction; a target with more entries sets slot_over and the build falls back to the
+// traversing write pass. (2D targets hold about 22 far and 9 near entries, 3D ones 57 and 20.)
+constexpr int far_slots(int d) { return d == 2 ? 128 : 256; }
+constexpr int NEAR_SLOTS = 128;
 
 struct ListOut {
     int *far_cnt, *near_cnt;             // count pass
     const int *far_ptr, *near_ptr;       // write pass
     int *far_idx, *near_idx;
-    int *nset, *nset_cnt;
-    int *far_slot, *near_slot;           // count pass (2D): LIST_SLOT entries per target, or null
+    int *nset, *nset_cnt;                // inadmissible sources, packed: see nset_pack
+    int *far_slot, *near_slot;           // count pass: far_slots(D) / NEAR_SLOTS entries per target
     int *slot_over;
-    int write;
 };
 
-__device__ __forceinline__ void emit(int *idx, const int *ptr, int t, int &c, int v, int write,
-                                     int *slot = nullptr, int *over = nullptr)
+// A source s that is inadmissible for a target, as the target's children will meet it: the range
+// of its children, or s itself when it is a leaf (first node << 4 | nodes)
+__device__ __forceinline__ int nset_pack(int s, const NodeRec &r)
 {
-    if (write) idx[ptr[t] + c] = v;
-    else if (slot != nullptr) {
-        if (c < LIST_SLOT) slot[(size_t)t * LIST_SLOT + c] = v;
-        else *over = 1;
-    }
-    c++;
+    return r.leaf ? (s << 4 | 1) : (r.fchild << 4 | r.nchild);
 }
 
-// leaf target t against the subtree of c (c neither admissible nor a leaf)
+// ---- the traversing write pass: a thread per target (only when a target overflowed its slots)
 template <int D>
-__device__ void descend(const TreeView &tv, ListOut &lo, int t, int c, int &fc, int &nc)
+__device__ void descend(const TreeView &tv, ListOut &lo, int t, const NodeRec &rt, const NodeRec &rc, int &fc, int &nc)
 {
     int stk[STACK_CAP];
     int sp = 0;
-    for (int k = tv.nchild[c] - 1; k >= 0; k--) stk[sp++] = tv.fchild[c] + k;
+    for (int k = rc.nchild - 1; k >= 0; k--) stk[sp++] = rc.fchild + k;
     while (sp > 0) {
         const int s = stk[--sp];
-        if (admissible<D>(tv, t, s)) { emit(lo.far_idx, lo.far_ptr, t, fc, s, lo.write, lo.far_slot, lo.slot_over); continue; }
-        if (tv.leaf[s]) { emit(lo.near_idx, lo.near_ptr, t, nc, s, lo.write, lo.near_slot, lo.slot_over); continue; }
-        if (sp + tv.nchild[s] > STACK_CAP) { atomicExch(&tv.info->nset_overflow, 1); return; }
-        for (int k = tv.nchild[s] - 1; k >= 0; k--) stk[sp++] = tv.fchild[s] + k;
+        const NodeRec rs = node_rec(tv, s);
+        if (admissible<D>(tv.L, rt, rs)) { lo.far_idx[lo.far_ptr[t] + fc++] = s; continue; }
+        if (rs.leaf) { lo.near_idx[lo.near_ptr[t] + nc++] = s; continue; }
+        if (sp + rs.nchild > STACK_CAP) { atomicExch(&tv.info->nset_overflow, 1); return; }
+        for (int k = rs.nchild - 1; k >= 0; k--) stk[sp++] = rs.fchild + k;
     }
-}
-
-template <int D>
-__device__ void process_target(const TreeView &tv, ListOut &lo, int t)
-{
-    int fc = 0, nc = 0, ns = 0;
-    if (t == 0) {
-        if (tv.leaf[0]) emit(lo.near_idx, lo.near_ptr, 0, nc, 0, lo.write, lo.near_slot, lo.slot_over);
-        else if (!lo.write) { lo.nset[0] = 0; ns = 1; }
-    } else {
-        const int p = tv.parent[t];
-        const int pn = lo.nset_cnt[p];
-        for (int a = 0; a < pn; a++) {
-            const int s = lo.nset[(size_t)p * tv.nset_cap + a];
-            const int c0 = tv.leaf[s] ? s : tv.fchild[s];
-            const int c1 = tv.leaf[s] ? s + 1 : tv.fchild[s] + tv.nchild[s];
-            for (int c = c0; c < c1; c++) {
-                if (c == t) {
-                    if (tv.leaf[t]) emit(lo.near_idx, lo.near_ptr, t, nc, t, lo.write, lo.near_slot, lo.slot_over);
-                    else if (!lo.write) {
-                        if (ns < tv.nset_cap) lo.nset[(size_t)t * tv.nset_cap + ns] = c;
-                        ns++;
-                    }
-                } else if (admissible<D>(tv, t, c)) {
-                    emit(lo.far_idx, lo.far_ptr, t, fc, c, lo.write, lo.far_slot, lo.slot_over);
-                } else if (tv.leaf[t]) {
-                    if (tv.leaf[c]) emit(lo.near_idx, lo.near_ptr, t, nc, c, lo.write, lo.near_slot, lo.slot_over);
-                    else descend<D>(tv, lo, t, c, fc, nc);
-                } else if (!lo.write) {
-                    if (ns < tv.nset_cap) lo.nset[(size_t)t * tv.nset_cap + ns] = c;
-                    ns++;
-                }
-            }
-        }
-    }
-    if (!lo.write) {
-        lo.far_cnt[t] = fc;
-        lo.near_cnt[t] = nc;
-        if (ns > tv.nset_cap) { atomicExch(&tv.info->nset_overflow, 1); ns = tv.nset_cap; }
-        lo.nset_cnt[t] = ns;
-    } else if (D == 2) {
-        // ascending partners (insertion sort of this target's short segments; 3D lists are
-        // longer and are sorted afterwards by a segmented sort)
-        int *f = lo.far_idx + lo.far_ptr[t];
-        for (int a = 1; a < fc; a++) { const int v = f[a]; int z = a - 1; while (z >= 0 && f[z] > v) { f[z + 1] = f[z]; z--; } f[z + 1] = v; }
-        int *g = lo.near_idx + lo.near_ptr[t];
-        for (int a = 1; a < nc; a++) { const int v = g[a]; int z = a - 1; while (z >= 0 && g[z] > v) { g[z + 1] = g[z]; z--; } g[z + 1] = v; }
-    }
-}
-
-// count pass of the internal targets of every level in one dependency-ordered launch
-// (persistent warps; a warp per target, in increasing node id, so a target's parent comes
-// first). For target t the lanes take the entries a of the parent's inadmissible set, each
-// with its candidate children c (the entry itself when it is a leaf): c goes to the far list
-// when c != t and (t, c) is admissible, else to t's inadmissible set, which is written in
-// (a, c) order, as process_target does.
-template <int D>
-__global__ void __launch_bounds__(256) k_lists_internal(TreeView tv, ListOut lo, DepArgs dp)
-{
-    constexpr int NCH = 1 << D;
-    const int lane = threadIdx.x & 31;
-    const int n_node = tv.info->n_node;
-    const int cap = tv.nset_cap;
-    for (;;) {
-        int item = 0;
-        if (lane == 0) item = atomicAdd(dp.ticket, 1);
-        const int t = __shfl_sync(0xffffffffu, item, 0);
-        if (t >= n_node) break;
-        if (tv.leaf[t]) continue;
-        int nf = 0, ns = 0, nf_run = 0;
-        if (t == 0) {
-            if (lane == 0) lo.nset[0] = 0;
-            ns = 1;
-        } else {
-            const int p = tv.parent[t];
-            if (lane == 0) dep_wait(dp, p);
-            __syncwarp();
-            const int pn = __ldcg(lo.nset_cnt + p);
-            for (int a0 = 0; a0 < pn; a0 += 32) {
-                const int a = a0 + lane;
-                int c0 = 0, c1 = 0, nn = 0;
-                if (a < pn) {
-                    const int src = __ldcg(lo.nset + (size_t)p * cap + a);
-                    const bool sl = tv.leaf[src] != 0;
-                    c0 = sl ? src : tv.fchild[src];
-                    c1 = sl ? src + 1 : tv.fchild[src] + tv.nchild[src];
-                }
-                int nfl = 0;
-#pragma unroll
-                for (int k = 0; k < NCH; k++) {
-                    const int c = c0 + k;
-                    if (c < c1) {
-                        if (c != t && admissible<D>(tv, t, c)) nfl++;
-                        else nn++;
-                    }
-                }
-                int inc = nn, incf = nfl;
-                for (int o = 1; o < 32; o <<= 1) {
-                    const int y = __shfl_up_sync(0xffffffffu, inc, o);
-                    const int yf = __shfl_up_sync(0xffffffffu, incf, o);
-                    if (lane >= o) { inc += y; incf += yf; }
-                }
-                int w = ns + inc - nn, wf = nf_run + incf - nfl;
-#pragma unroll
-                for (int k = 0; k < NCH; k++) {
-                    const int c = c0 + k;
-                    if (c < c1) {
-                        if (!(c != t && admissible<D>(tv, t, c))) {
-                            if (w < cap) lo.nset[(size_t)t * cap + w] = c;
-                            w++;
-                        } else if (lo.far_slot != nullptr) {
-                            if (wf < LIST_SLOT) lo.far_slot[(size_t)t * LIST_SLOT + wf] = c;
-                            else *lo.slot_over = 1;
-                            wf++;
-                        }
-                    }
-                }
-                ns += __shfl_sync(0xffffffffu, inc, 31);
-                nf_run += __shfl_sync(0xffffffffu, incf, 31);
-                nf += nfl;
-            }
-        }
-        nf = warp_sum(nf);
-        if (lane == 0) {
-            lo.far_cnt[t] = nf;
-            lo.near_cnt[t] = 0;
-            if (ns > cap) { atomicExch(&tv.info->nset_overflow, 1); ns = cap; }
-            lo.nset_cnt[t] = ns;
-        }
-        __syncwarp();
-        if (lane == 0) dep_publish(dp, t);
-    }
-}
-
-// count pass, every leaf target (leaves need only their parent's NSET)
-template <int D>
-__global__ void __launch_bounds__(128) k_lists_leaves(TreeView tv, ListOut lo)
-{
-    const int n_node = tv.info->n_node;
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n_node; t += gridDim.x * blockDim.x)
-        if (tv.leaf[t]) process_target<D>(tv, lo, t);
 }
 
 template <int D>
 __global__ void __launch_bounds__(128) k_lists_write(int n_node, TreeView tv, ListOut lo)
 {
-    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n_node; t += gridDim.x * blockDim.x)
-        process_target<D>(tv, lo, t);
-}
-
-// the list write from the count pass's slots: a warp per target copies its entries to its
-// list segment and sorts them ascending (the traversing write pass emits the same set and
-// sorts it the same way)
-__device__ __forceinline__ void warp_copy_sorted(const int *slot, int cnt, int *dst, int lane)
-{
-    // rank of each entry among the segment's (distinct) entries
-    for (int a = lane; a < cnt; a += 32) {
-        const int v = slot[a];
-        int r = 0;
-        for (int b = 0; b < cnt; b++) r += slot[b] < v;
-        dst[r] = v;
+    for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n_node; t += gridDim.x * blockDim.x) {
+        const NodeRec rt = node_rec(tv, t);
+        int fc = 0, nc = 0;
+        if (t == 0) {
+            if (rt.leaf) lo.near_idx[lo.near_ptr[0] + nc++] = 0;
+        } else {
+            const int pn = lo.nset_cnt[rt.parent];
+            for (int a = 0; a < pn; a++) {
+                const int e = lo.nset[(size_t)rt.parent * tv.nset_cap + a];
+                for (int c = e >> 4; c < (e >> 4) + (e & 15); c++) {
+                    if (c == t) {
+                        if (rt.leaf) lo.near_idx[lo.near_ptr[t] + nc++] = t;
+                        continue;
+                    }
+                    const NodeRec rc = node_rec(tv, c);
+                    if (admissible<D>(tv.L, rt, rc)) lo.far_idx[lo.far_ptr[t] + fc++] = c;
+                    else if (rt.leaf) {
+                        if (rc.leaf) lo.near_idx[lo.near_ptr[t] + nc++] = c;
+                        else descend<D>(tv, lo, t, rt, rc, fc, nc);
+                    }
+                }
+            }
+        }
+        if (D == 2) {
+            // ascending partners (insertion sort of this target's short segments; 3D lists are
+            // longer and are sorted afterwards by a segmented sort)
+            int *f = lo.far_idx + lo.far_ptr[t];
+            for (int a = 1; a < fc; a++) { const int v = f[a]; int z = a - 1; while (z >= 0 && f[z] > v) { f[z + 1] = f[z]; z--; } f[z + 1] = v; }
+            int *g = lo.near_idx + lo.near_ptr[t];
+            for (int a = 1; a < nc; a++) { const int v = g[a]; int z = a - 1; while (z >= 0 && g[z] > v) { g[z + 1] = g[z]; z--; } g[z + 1] = v; }
+        }
     }
 }
 
+// Count pass of every target in one dependency-ordered launch: persistent warps, a warp per
+// target, in increasing node id, so a target's parent comes first. The lanes take the entries of
+// the parent's inadmissible set, each with its nodes c. An internal target t sends c to its far
+// list when c != t and (t, c) is admissible, else to its own inadmissible set. A leaf target
+// sends an admissible c to its far list, a leaf c to its near list, and puts any other c on the
+// warp's stack, whose nodes are then expanded 32 children at a time, deepest first: a round pops
+// G = 32 / 2^D nodes, so a level of the tree holds at most G - 1 + 32 stack entries, under 1024
+// over the depth, plus one chunk's 32 * 2^D.
+// What bounds it is the chain from the root (a level each: the parent's flag, its set, the nodes'
+// records, the publication), so the next ticket is drawn while a target is worked on, the set
+// holds ready child ranges and a node is one record. Leaves had a thread each in a launch of
+// their own, every step of whose traversal was a dependent load: with the internal pass 98 us
+// at 20K points 2D and 200 us at 1M, 403 us at 100K in 3D (and the traversal again to write).
+constexpr int LIST_WARPS = 4;
+constexpr int LIST_CTAS = 8;   // per SM
+template <int D> constexpr int list_stack() { return 1024 + 32 * (1 << D); }
+
+template <int D>
+__global__ void __launch_bounds__(32 * LIST_WARPS) k_lists(TreeView tv, ListOut lo, DepArgs dp)
+{
+    constexpr int NCH = 1 << D, G = 32 / NCH, FS = far_slots(D);
+    __shared__ int stack_[LIST_WARPS][list_stack<D>()];
+    int *stack = stack_[threadIdx.x >> 5];
+    const int lane = threadIdx.x & 31;
+    const unsigned lt = (1u << lane) - 1u;
+    const int n_node = tv.info->n_node, cap = tv.nset_cap, L = tv.L;
+    int next = 0;
+    if (lane == 0) next = atomicAdd(dp.ticket, 1);
+    for (;;) {
+        const int t = __shfl_sync(0xffffffffu, next, 0);
+        if (t >= n_node) break;
+        if (lane == 0) next = atomicAdd(dp.ticket, 1);
+        const NodeRec rt = node_rec(tv, t);
+        int *fslot = lo.far_slot + (size_t)t * FS, *nslot = lo.near_slot + (size_t)t * NEAR_SLOTS;
+        int nf = 0, nn = 0, ns = 0;   // far, near and inadmissible entries so far
+        // every lane's c (its flags say whether it has one): appended in lane order
+        auto put_far = [&](bool on, int c) {
+            const unsigned m = __ballot_sync(0xffffffffu, on);
+            if (on) {
+                const int w = nf + __popc(m & lt);
+                if (w < FS) fslot[w] = c;
+            }
+            nf += __popc(m);
+        };
+        auto put_near = [&](bool on, int c) {
+            const unsigned m = __ballot_sync(0xffffffffu, on);
+            if (on) {
+                const int w = nn + __popc(m & lt);
+                if (w < NEAR_SLOTS) nslot[w] = c;
+            }
+            nn += __popc(m);
+        };
+        if (t == 0) {
+            if (rt.leaf) put_near(lane == 0, 0);
+            else {
+                if (lane == 0) lo.nset[0] = nset_pack(0, rt);
+                ns = 1;
+            }
+        } else {
+            const int p = rt.parent;
+            if (lane == 0) dep_wait(dp, p);
+            __syncwarp();
+            const int pn = __ldcg(lo.nset_cnt + p);
+            for (int a0 = 0; a0 < pn; a0 += 32) {
+                const int e = a0 + lane < pn ? __ldcg(lo.nset + (size_t)p * cap + a0 + lane) : 0;
+                const int c0 = e >> 4, cn = e & 15;
+                int sp = 0;
+#pragma unroll
+                for (int k = 0; k < NCH; k++) {
+                    const bool on = k < cn;
+                    const int c = c0 + k;
+                    const NodeRec rc = node_rec(tv, on ? c : 0);
+                    const bool self = on && c == t;
+                    const bool far = on && !self && admissible<D>(L, rt, rc);
+                    put_far(far, c);
+                    if (!rt.leaf) {
+                        const bool in = on && !far;
+                        const unsigned m = __ballot_sync(0xffffffffu, in);
+                        if (in) {
+                            const int w = ns + __popc(m & lt);
+                            if (w < cap) lo.nset[(size_t)t * cap + w] = nset_pack(c, rc);
+                        }
+                        ns += __popc(m);
+                    } else {
+                        put_near(on && !far && rc.leaf, c);   // the target itself is a leaf too
+                        const bool in = on && !far && !rc.leaf;
+                        const unsigned m = __ballot_sync(0xffffffffu, in);
+                        if (in) stack[sp + __popc(m & lt)] = rc.fchild << 4 | rc.nchild;
+                        sp += __popc(m);
+                    }
+                }
+                while (sp > 0) {   // leaf targets only
+                    __syncwarp();
+                    const int take = min(G, sp), g = lane / NCH, k = lane % NCH;
+                    const int q = g < take ? stack[sp - take + g] : 0;
+                    sp -= take;
+                    __syncwarp();
+                    const bool on = k < (q & 15);
+                    const int c = (q >> 4) + k;
+                    const NodeRec rc = node_rec(tv, on ? c : 0);
+                    const bool far = on && admissible<D>(L, rt, rc);
+                    put_far(far, c);
+                    put_near(on && !far && rc.leaf, c);
+                    const bool in = on && !far && !rc.leaf;
+                    const unsigned m = __ballot_sync(0xffffffffu, in);
+                    if (in) stack[sp + __popc(m & lt)] = rc.fchild << 4 | rc.nchild;
+                    sp += __popc(m);
+                }
+                __syncwarp();
+            }
+        }
+        if (lane == 0) {
+            lo.far_cnt[t] = nf;
+            lo.near_cnt[t] = nn;
+            if (nf > FS || nn > NEAR_SLOTS) *lo.slot_over = 1;
+            if (ns > cap) { atomicExch(&tv.info->nset_overflow, 1); ns = cap; }
+            lo.nset_cnt[t] = ns;
+        }
+        __syncwarp();
+        if (!rt.leaf && lane == 0) dep_publish(dp, t);
+    }
+}
+
+// The list write from the count pass's slots: a warp per target copies its entries to its list
+// segment, ascending (each entry's place is its rank among the segment's distinct entries,
+// counted from the warp's staged copy; the traversing write pass emits and sorts the same set)
+__device__ __forceinline__ void warp_copy_sorted(const int *slot, int cnt, int *dst, int *stage, int lane)
+{
+    for (int a = lane; a < cnt; a += 32) stage[a] = slot[a];
+    __syncwarp();
+    for (int a = lane; a < cnt; a += 32) {
+        const int v = stage[a];
+        int r = 0;
+        for (int b = 0; b < cnt; b++) r += stage[b] < v;
+        dst[r] = v;
+    }
+    __syncwarp();
+}
+
+template <int D>
 __global__ void __launch_bounds__(256) k_lists_compact(TreeView tv, ListOut lo)
 {
+    constexpr int FS = far_slots(D);
+    __shared__ int stage_[8][FS > NEAR_SLOTS ? FS : NEAR_SLOTS];
     const int n_node = tv.info->n_node;
     const int lane = threadIdx.x & 31;
+    int *stage = stage_[threadIdx.x >> 5];
     for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < n_node; t += (gridDim.x * blockDim.x) >> 5) {
-        warp_copy_sorted(lo.far_slot + (size_t)t * LIST_SLOT, lo.far_cnt[t], lo.far_idx + lo.far_ptr[t], lane);
-        warp_copy_sorted(lo.near_slot + (size_t)t * LIST_SLOT, lo.near_cnt[t], lo.near_idx + lo.near_ptr[t], lane);
+        warp_copy_sorted(lo.far_slot + (size_t)t * FS, lo.far_cnt[t], lo.far_idx + lo.far_ptr[t], stage, lane);
+        warp_copy_sorted(lo.near_slot + (size_t)t * NEAR_SLOTS, lo.near_cnt[t], lo.near_idx + lo.near_ptr[t], stage, lane);
     }
 }
 
@@ -2567,8 +2607,7 @@ public:
         hbig_ = I.n_big;
         if (max_level_ <= 2) { built_ = false; return 1; }
 
-        // The list write (and in 3D the segmented sort of each target's entries) needs only the
-        // count pass, and the bases read no list, so it runs on the side stream beside the leaf
+        // The list write needs only the count pass, and the bases read no list, so it runs on the side stream beside the leaf
         // bases; the near blocks follow it there. Its buffers are allocated first, in the
         // workspace stream's order (the stream-ordered pool), and the side stream starts from
         // that point. Readers on the workspace stream join it first (join_lists).
@@ -2576,7 +2615,8 @@ public:
         stats_.n_near = htot_[1] = I.n_near;
         far_idx_.ensure(std::max(1, htot_[0]));
         near_idx_.ensure(std::max(1, htot_[1]));
-        if (D == 3) {
+        const bool slot_over = I.pad[2] != 0;   // a target with more entries than slots
+        if (D == 3 && slot_over) {
             sort_reserve(far_idx_, far_alt_, htot_[0], far_ptr_.p);
             sort_reserve(near_idx_, near_alt_, htot_[1], near_ptr_.p);
         }
@@ -2584,17 +2624,16 @@ public:
             TSNE_CUDA_CHECK(cudaEventRecord(fork_ev_, st_));
             TSNE_CUDA_CHECK(cudaStreamWaitEvent(st2_, fork_ev_, 0));
             cudaEvent_t t_lists = mark_begin(st2_);
-            ListOut lo = list_out(1);
-            if (D == 2 && !I.pad[2]) {
-                k_lists_compact<<<grid_for((long long)n_node_ * 32, 256, 148 * 8), 256, 0, st2_>>>(view(), lo);
+            if (!slot_over) {
+                k_lists_compact<D><<<grid_for((long long)n_node_ * 32, 256, 148 * 8), 256, 0, st2_>>>(view(), list_out());
             } else {
-                k_lists_write<D><<<grid_for(n_node_, 128, 148 * 8), 128, 0, st2_>>>(n_node_, view(), lo);
+                k_lists_write<D><<<grid_for(n_node_, 128, 148 * 8), 128, 0, st2_>>>(n_node_, view(), list_out());
+                if (D == 3) {
+                    sort_segments(far_idx_, far_alt_, htot_[0], far_ptr_.p, st2_);
+                    sort_segments(near_idx_, near_alt_, htot_[1], near_ptr_.p, st2_);
+                }
             }
             launches_++;
-            if (D == 3) {
-                sort_segments(far_idx_, far_alt_, htot_[0], far_ptr_.p, st2_);
-                sort_segments(near_idx_, near_alt_, htot_[1], near_ptr_.p, st2_);
-            }
             mark_end(t_lists, 1, st2_);
             TSNE_CUDA_CHECK(cudaEventRecord(lists_ev_, st2_));
             lists_pending_ = true;
@@ -2711,20 +2750,19 @@ public:
         return 0;
     }
 
-    // counting pass of the lists (internal targets, then every leaf target), the list pointers,
-    // the basis row offsets and the basis launches' item lists
+    // counting pass of the lists, the list pointers, the basis row offsets and the basis
+    // launches' item lists
     void launch_list_counts()
     {
-        ListOut lo = list_out(0);
         DepArgs dp{flag_.p, tickets_.p + TICKET_LISTS, &info_.p->pad[1], ++epoch_};
-        k_lists_internal<D><<<148 * 4, 256, 0, st_>>>(view(), lo, dp);
-        k_lists_leaves<D><<<148 * 8, 128, 0, st_>>>(view(), lo);
+        k_lists<D><<<std::min(148 * LIST_CTAS, ceil_div(cap_node_, LIST_WARPS)), 32 * LIST_WARPS, 0, st_>>>(
+            view(), list_out(), dp);
         const NodeScan q{far_cnt_.p, near_cnt_.p, far_ptr_.p, near_ptr_.p, rowoff_.p, ilist_.p, llist_.p, blist_.p,
                          rank_.p, node_blk_.p};
         const int nb = ceil_div(cap_node_, NODE_BLOCK);
         k_node_sums<D><<<nb, NODE_BLOCK, 0, st_>>>(view(), q);
         k_node_scan<D><<<nb, NODE_BLOCK, 0, st_>>>(view(), q);
-        launches_ += 4;
+        launches_ += 3;
     }
 
     void alloc_lists()
@@ -2738,10 +2776,8 @@ public:
         rowoff_.exact(c + 2);
         rank_.exact(c);
         node_blk_.exact(ceil_div(c, NODE_BLOCK));
-        if (D == 2) {
-            far_slot_.exact(c * LIST_SLOT);
-            near_slot_.exact(c * LIST_SLOT);
-        }
+        far_slot_.exact(c * far_slots(D));
+        near_slot_.exact(c * NEAR_SLOTS);
     }
 
     void product_force(void *F, DevScalars *sc, double *partials, int keep_rep) override
@@ -2965,6 +3001,7 @@ private:
         const size_t c = cap_node_;
         start_.exact(c); end_.exact(c); level_.exact(c); parent_.exact(c); fchild_.exact(c);
         nchild_.exact(c); leaf_.exact(c); ix_.exact(3 * c);
+        rec_.exact(2 * c);
         bset_.exact(c * (Dim<D>::L + 1));
         flag_.exact(c);
         TSNE_CUDA_CHECK(cudaMemsetAsync(flag_.p, 0, sizeof(int) * c, st_));
@@ -2979,24 +3016,23 @@ private:
         TreeView v;
         v.n = n_; v.L = Dim<D>::L; v.leaf_size = leaf_size_; v.cap_node = cap_node_; v.nset_cap = nset_cap_;
         v.keys = keys_.p; v.start = start_.p; v.end = end_.p; v.level = level_.p; v.parent = parent_.p;
-        v.fchild = fchild_.p; v.nchild = nchild_.p; v.leaf = leaf_.p; v.ix = ix_.p;
+        v.fchild = fchild_.p; v.nchild = nchild_.p; v.leaf = leaf_.p; v.ix = ix_.p; v.rec = rec_.p;
         v.delta = delta_.p; v.fm = fm_.p; v.blkcnt = blkcnt_.p; v.blkoff = blkoff_.p;
         v.bset = bset_.p; v.nid = nid_.p; v.btot = btot_.p; v.tickets = tickets_.p;
         v.info = info_.p;
         return v;
     }
 
-    ListOut list_out(int write)
+    ListOut list_out()
     {
         ListOut lo;
         lo.far_cnt = far_cnt_.p; lo.near_cnt = near_cnt_.p;
         lo.far_ptr = far_ptr_.p; lo.near_ptr = near_ptr_.p;
         lo.far_idx = far_idx_.p; lo.near_idx = near_idx_.p;
         lo.nset = nset_.p; lo.nset_cnt = nset_cnt_.p;
-        lo.far_slot = D == 2 ? far_slot_.p : nullptr;
-        lo.near_slot = D == 2 ? near_slot_.p : nullptr;
+        lo.far_slot = far_slot_.p;
+        lo.near_slot = near_slot_.p;
         lo.slot_over = &info_.p->pad[2];
-        lo.write = write;
         return lo;
     }
 
@@ -3132,7 +3168,8 @@ private:
     cudaStream_t st2_ = nullptr;  // side stream: the list write and the near field beside the bases
     cudaEvent_t fork_ev_ = nullptr, near_ev_ = nullptr, lists_ev_ = nullptr;
     bool near_pending_ = false, lists_pending_ = false;
-    DevBuf<int> far_slot_, near_slot_;   // 2D: list entries parked by the count pass
+    DevBuf<int4> rec_;                   // node records of the list pass
+    DevBuf<int> far_slot_, near_slot_;   // list entries parked by the count pass
     int epoch_ = 0;
     DevBuf<int> nset_, nset_cnt_, far_cnt_, near_cnt_, far_ptr_, near_ptr_, far_idx_, near_idx_;
     DevBuf<int> far_alt_, near_alt_;   // segmented-sort partners of the 3D lists
