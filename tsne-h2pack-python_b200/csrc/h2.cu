@@ -48,6 +48,7 @@ struct TreeView {
     const unsigned long long *keys;
     int *start, *end, *level, *parent, *fchild, *nchild, *leaf, *ix;
     int4 *rec;               // per node, packed for the list pass: see node_rec
+    float4 *proxies;         // per level: see proxy_table
     signed char *delta;      // shared leading digits with the previous key (n + 1)
     int *fm;                 // per point: first | last level << 8 of the nodes it starts, or -1
     int *blkcnt, *blkoff;    // per block of TREE_BLOCK points, 2 x 32 counts / offsets
@@ -471,12 +472,82 @@ __device__ __forceinline__ NodeRec node_rec(const TreeView &tv, int t)
     return r;
 }
 
-// end, parent and child count of every node from the boundary lists; its record; the largest leaf
+// ---------------------------------------------------------------------------------
+// proxy points (shells |y - c|_inf = rho h around a box of half-width h)
+// ---------------------------------------------------------------------------------
+template <int D>
+__device__ __forceinline__ void proxy_point(int p, double h, float *out)
+{
+    if constexpr (D == 2) {
+        const int sh = p / SHELL_PTS_2D, k = p % SHELL_PTS_2D;
+        const double rad = shell_rho(sh) * h;
+        const double off = (sh & 1) ? 0.0 : 0.5;
+        const double u = ((double)k + off) * (8.0 / SHELL_PTS_2D);
+        const int side = (int)(u * 0.5);
+        const double a = u - 2.0 * side - 1.0;
+        double x, y;
+        switch (side) {
+            case 0: x = a; y = -1.0; break;
+            case 1: x = 1.0; y = a; break;
+            case 2: x = -a; y = 1.0; break;
+            default: x = -1.0; y = -a; break;
+        }
+        out[0] = (float)(x * rad);
+        out[1] = (float)(y * rad);
+    } else {
+        constexpr int g = SHELL_GRID_3D, per = 6 * g * g;
+        const int sh = p / per, r = p % per, f = r / (g * g), ij = r % (g * g), i = ij / g, j = ij % g;
+        const double rad = shell_rho(sh) * h;
+        const int ax = f >> 1;
+        const double sgn = (f & 1) ? 1.0 : -1.0;
+        const double a = ((double)i + 0.5) * (2.0 / g) - 1.0;
+        const double b = ((double)j + 0.5) * (2.0 / g) - 1.0;
+        double c[3];
+        c[ax] = sgn;
+        c[(ax + 1) % 3] = a;
+        c[(ax + 2) % 3] = b;
+        for (int k = 0; k < 3; k++) out[k] = (float)(c[k] * rad);
+    }
+}
+
+// The proxies of every level, relative to a node's centre, once per build (they are FP64 work that
+// every node of a level repeated: 26,000 of a 3D node's 550,000 cycles, 1,500 of a 2D node's 70,000).
+// 2D: (x, y) per proxy; 3D: the pairs (2j, 2j + 1) as (-2x, -2x', -2y, -2y'), then, ID3_PB further,
+// (-2z, -2z', |p|^2, |p'|^2).
+constexpr int PROXY_F4 = 216;   // float4 per level
+template <int D>
+__device__ __forceinline__ void proxy_table(int l, double radius, float4 *table)
+{
+    constexpr int P = Dim<D>::NPROXY;
+    static_assert(D == 2 ? P * sizeof(float2) <= PROXY_F4 * sizeof(float4) : P == PROXY_F4, "table row");
+    const double h = radius / (double)(1LL << l);
+    float4 *row = table + (size_t)l * PROXY_F4;
+    if constexpr (D == 2) {
+        for (int p = threadIdx.x; p < P; p += blockDim.x) {
+            float y[2];
+            proxy_point<2>(p, h, y);
+            reinterpret_cast<float2 *>(row)[p] = make_float2(y[0], y[1]);
+        }
+    } else {
+        for (int j = threadIdx.x; j < P / 2; j += blockDim.x) {
+            float p0[3], p1[3];
+            proxy_point<3>(2 * j, h, p0);
+            proxy_point<3>(2 * j + 1, h, p1);
+            row[j] = make_float4(-2.f * p0[0], -2.f * p1[0], -2.f * p0[1], -2.f * p1[1]);
+            row[P / 2 + j] = make_float4(-2.f * p0[2], -2.f * p1[2], fmaf(p0[0], p0[0], fmaf(p0[1], p0[1], p0[2] * p0[2])),
+                                         fmaf(p1[0], p1[0], fmaf(p1[1], p1[1], p1[2] * p1[2])));
+        }
+    }
+}
+
+// end, parent and child count of every node from the boundary lists; its record; the largest
+// leaf; the proxy table
 template <int D>
 __global__ void k_tree_finish(TreeView tv)
 {
     TreeInfo *info = tv.info;
     if (info->pad[0]) return;
+    for (int l = blockIdx.x; l <= tv.L; l += gridDim.x) proxy_table<D>(l, info->radius, tv.proxies);
     const int n_node = info->n_node;
     const size_t cap = (size_t)tv.cap_node;
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n_node; t += gridDim.x * blockDim.x) {
@@ -822,24 +893,26 @@ __global__ void __launch_bounds__(256) k_lists_compact(TreeView tv, ListOut lo)
 // (its rows of the interpolation matrices: a leaf's points, or the upper bound of the children's
 // skeletons; nodes above MIN_ADM_LEVEL have none), the item lists of the basis launches
 // (ilist: the internal nodes at level >= MIN_ADM_LEVEL; llist / blist: the leaves there of at most
-// LEAF_SMALL (3D: ID3_TINY_LEAF) points / the larger ones) and flist, the leaves with far entries
+// LEAF_SMALL points / the larger ones; 3D: at most ID3_TINY_LEAF / ID3_SMALL_LEAF points, and clist
+// the larger ones) and flist, the leaves with far entries
 // finer than themselves; each list in increasing node id.
 // Two launches over the nodes there are (block sums, then every block adds the sums before its
 // own): six device-wide scans over the node capacity and their flag and memset launches took
 // 25 launches, 75 us of a rebuild at 20K points and 85 us at 1M.
 constexpr int LEAF_SMALL = 64;
-constexpr int ID3_TINY_LEAF = 32;   // 3D: the leaves of the smallest basis CTAs
+constexpr int ID3_TINY_LEAF = 32;    // 3D: the leaves of the smallest basis CTAs,
+constexpr int ID3_SMALL_LEAF = 64;   // and of the next
 constexpr int NODE_BLOCK = 1024;
 
 struct NodeSums {
     long long rows;
-    int far, near, in, small, big, fine;
+    int far, near, in, small, big, large, fine, pad;
 };
 struct NodeScan {
     const int *far_cnt, *near_cnt, *fine_cnt;
     int *far_ptr, *near_ptr;
     long long *rowoff;
-    int *ilist, *llist, *blist, *flist, *rank;
+    int *ilist, *llist, *blist, *clist, *flist, *rank;
     NodeSums *blk;
 };
 
@@ -848,7 +921,8 @@ __device__ __forceinline__ NodeSums node_add(const NodeSums &a, const NodeSums &
     NodeSums c;
     c.rows = a.rows + b.rows;
     c.far = a.far + b.far; c.near = a.near + b.near;
-    c.in = a.in + b.in; c.small = a.small + b.small; c.big = a.big + b.big; c.fine = a.fine + b.fine;
+    c.in = a.in + b.in; c.small = a.small + b.small; c.big = a.big + b.big;
+    c.large = a.large + b.large; c.fine = a.fine + b.fine; c.pad = 0;
     return c;
 }
 __device__ __forceinline__ NodeSums node_shfl_up(const NodeSums &a, int o)
@@ -860,13 +934,15 @@ __device__ __forceinline__ NodeSums node_shfl_up(const NodeSums &a, int o)
     c.in = __shfl_up_sync(0xffffffffu, a.in, o);
     c.small = __shfl_up_sync(0xffffffffu, a.small, o);
     c.big = __shfl_up_sync(0xffffffffu, a.big, o);
+    c.large = __shfl_up_sync(0xffffffffu, a.large, o);
     c.fine = __shfl_up_sync(0xffffffffu, a.fine, o);
+    c.pad = 0;
     return c;
 }
 __device__ __forceinline__ NodeSums node_zero()
 {
     NodeSums c;
-    c.rows = 0; c.far = c.near = c.in = c.small = c.big = c.fine = 0;
+    c.rows = 0; c.far = c.near = c.in = c.small = c.big = c.large = c.fine = c.pad = 0;
     return c;
 }
 template <int D>
@@ -884,7 +960,8 @@ __device__ __forceinline__ NodeSums node_counts(const TreeView &tv, const NodeSc
         const int r = tv.end[t] - tv.start[t];
         c.rows = r;
         if (r <= (D == 2 ? LEAF_SMALL : ID3_TINY_LEAF)) c.small = 1;
-        else c.big = 1;
+        else if (D == 2 || r <= ID3_SMALL_LEAF) c.big = 1;
+        else c.large = 1;
     }
     return c;
 }
@@ -933,7 +1010,7 @@ __global__ void __launch_bounds__(NODE_BLOCK) k_node_scan(TreeView tv, NodeScan 
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         q.far_ptr[0] = 0; q.near_ptr[0] = 0; q.rowoff[0] = 0;
         tv.tickets[TICKET_BASES] = 0;
-        if (n_node == 0) { info->n_far = info->n_near = info->n_int = info->n_small = info->n_big = info->n_fine = 0; info->n_rows = 0; }
+        if (n_node == 0) { info->n_far = info->n_near = info->n_int = info->n_small = info->n_big = info->n_large = info->n_fine = 0; info->n_rows = 0; }
     }
     if (blockIdx.x * NODE_BLOCK >= n_node) return;
     // the blocks before this one
@@ -949,6 +1026,7 @@ __global__ void __launch_bounds__(NODE_BLOCK) k_node_scan(TreeView tv, NodeScan 
     if (own.in) q.ilist[inc.in - 1] = t;
     if (own.small) q.llist[inc.small - 1] = t;
     if (own.big) q.blist[inc.big - 1] = t;
+    if (own.large) q.clist[inc.large - 1] = t;
     if (own.fine) q.flist[inc.fine - 1] = t;
     if (tv.level[t] < MIN_ADM_LEVEL) q.rank[t] = 0;   // no basis; the others' ranks come with theirs
     if (t == n_node - 1) {
@@ -958,45 +1036,8 @@ __global__ void __launch_bounds__(NODE_BLOCK) k_node_scan(TreeView tv, NodeScan 
         info->n_int = inc.in;
         info->n_small = inc.small;
         info->n_big = inc.big;
+        info->n_large = inc.large;
         info->n_fine = inc.fine;
-    }
-}
-
-// ---------------------------------------------------------------------------------
-// proxy points (shells |y - c|_inf = rho h around a box of half-width h)
-// ---------------------------------------------------------------------------------
-template <int D>
-__device__ __forceinline__ void proxy_point(int p, double h, float *out)
-{
-    if constexpr (D == 2) {
-        const int sh = p / SHELL_PTS_2D, k = p % SHELL_PTS_2D;
-        const double rad = shell_rho(sh) * h;
-        const double off = (sh & 1) ? 0.0 : 0.5;
-        const double u = ((double)k + off) * (8.0 / SHELL_PTS_2D);
-        const int side = (int)(u * 0.5);
-        const double a = u - 2.0 * side - 1.0;
-        double x, y;
-        switch (side) {
-            case 0: x = a; y = -1.0; break;
-            case 1: x = 1.0; y = a; break;
-            case 2: x = -a; y = 1.0; break;
-            default: x = -1.0; y = -a; break;
-        }
-        out[0] = (float)(x * rad);
-        out[1] = (float)(y * rad);
-    } else {
-        constexpr int g = SHELL_GRID_3D, per = 6 * g * g;
-        const int sh = p / per, r = p % per, f = r / (g * g), ij = r % (g * g), i = ij / g, j = ij % g;
-        const double rad = shell_rho(sh) * h;
-        const int ax = f >> 1;
-        const double sgn = (f & 1) ? 1.0 : -1.0;
-        const double a = ((double)i + 0.5) * (2.0 / g) - 1.0;
-        const double b = ((double)j + 0.5) * (2.0 / g) - 1.0;
-        double c[3];
-        c[ax] = sgn;
-        c[(ax + 1) % 3] = a;
-        c[(ax + 2) % 3] = b;
-        for (int k = 0; k < 3; k++) out[k] = (float)(c[k] * rad);
     }
 }
 
@@ -1601,40 +1642,54 @@ k_id2d(int n_item, const int *__restrict__ items, IdArgs g, DepArgs dp)
 }
 
 // ---------------------------------------------------------------------------------
-// 3D interpolative decompositions with recomputed rows
+// 3D interpolative decompositions
 // ---------------------------------------------------------------------------------
 // The 3D proxy matrix has 216 columns and up to 512 candidate rows (eight children of rank
-// <= 64): 442 KB in FP32, more than one SM holds. Its entries are cheap to recompute, one
-// reciprocal each in the expanded form (1 + |x|^2 + |p|^2 - 2 x.p)^-2 (x: candidate relative
-// to the node's centre, p: proxy), so no row is stored: the column-pivoted Gram-Schmidt runs
-// left-looking. Step r takes the row b of the largest residual norm and orthonormalises it
-// against the earlier directions q_0..q_{r-1} by classical Gram-Schmidt applied twice (the
-// first pass from b's stored projections, the second recomputed, so the directions stay
-// orthonormal to rounding); every other row a then recomputes its entries once for its dot
-// product c = a . q_r (= its residual's, as q_r is orthogonal to the earlier directions),
-// kept in shared memory as R12, with its squared residual norm downdated in FP64 by c^2.
-// R11's column r is b's projections on q_0..q_{r-1} and its residual norm. The stop rule, tie
-// rule, back substitution U = [I ; R11^-1 R12]^T and the upward coefficients are those of k_id.
+// <= 64). The column-pivoted Gram-Schmidt runs left-looking, so the matrix is never changed:
+// step r takes the row b of the largest residual norm and orthonormalises it against the earlier
+// directions q_0..q_{r-1} by classical Gram-Schmidt applied twice (the first pass from b's stored
+// projections, the second recomputed, so the directions stay orthonormal to rounding); every
+// other row a then takes its dot product c = a . q_r (= its residual's, as q_r is orthogonal to
+// the earlier directions), kept in shared memory as R12, with its squared residual norm
+// downdated in FP64 by c^2. R11's column r is b's projections on q_0..q_{r-1} and its residual
+// norm. The stop rule, tie rule, back substitution U = [I ; R11^-1 R12]^T and the upward
+// coefficients are those of k_id.
 //
-// One CTA per node, in three sizes (THREADS, ROWS = the most candidate rows it takes): 512
-// threads and 512 rows (internal nodes, leaves above 128 points; one CTA per SM), 256 and 128
-// (leaves of 33..128 points; two per SM), 128 and 32 (leaves of at most 32 points, four per
-// SM). The proxies are held in pairs (2j, 2j + 1) for the paired FP32 instructions; a row is
-// split over S adjacent lanes (the largest S <= 16 with THREADS / S >= rows, else 2), lane
-// `sub` taking the pairs j = sub mod S, and lane group g = tid / S covers the rows
-// g + (THREADS / S) k; the S partial sums of a row meet by butterfly shuffles, which give
-// every lane of the group the same value.
+// The rows' entries (1 + |x|^2 + |p|^2 - 2 x.p)^-2 (x: candidate relative to the node's centre, p:
+// proxy; one reciprocal each) are evaluated once and held: the first THREADS / 4 rows in
+// registers (at most 28 pairs of proxies per lane, four lanes or more per row), of a node with more
+// candidates the next ones in the shared memory that is left, and only rows beyond that are
+// evaluated again in every step. Evaluating every row in every step kept the reciprocal pipe at a
+// quarter of its rate and the rows' pass at 18 instructions per pair of entries; held, a pair is
+// one load and one paired FMA. At 100K points (h2_tol 3e-2, late in a run; nodes of 178 candidates
+// and rank 42 on average) the internal launch went from 2,034 to 1,580 us, the leaves' from 928 to
+// 731 us a rebuild. It is bound by the chain of the largest nodes (420 candidates, of which about
+// 245 are evaluated in every step) and by the latencies of a step: the pivot's two
+// orthonormalisations take about half of it.
+//
+// The proxies go in pairs (2j, 2j + 1) for the paired FP32 instructions. A row's dot product is S
+// chains over the pairs j = c mod S in increasing j (S = 16, 8, 4, 2 by the number of rows against
+// the threads), joined by butterfly shuffles. A row held by as many lanes as chains has a chain
+// per lane; with S = 2, four lanes hold a row, and the chain's first 28 pairs and its last 26 are
+// two lanes', the second going on from the first's sum. S and the order of a chain are part of
+// the result's rounding, so they do not depend on where a row is held.
+//
+// One CTA per node: 128 threads (leaves of at most 32 points), 256 (33..64), 512 (the others).
 //
 // Internal nodes run in one dependency-ordered launch: a node waits for its internal
 // children's skeletons and ranks (flag), published right after their pivot loop, and, before
 // its upward coefficients, for their coefficients (second flag, published last).
 constexpr int ID3_P = Dim<3>::NPROXY;
+constexpr int ID3_NP = ID3_P / 2;            // proxy pairs
 constexpr int ID3_ROWS = 8 * Dim<3>::MAXR;   // candidate rows of an internal node
 constexpr int ID3_QS = 220;                  // row stride of the directions (16-byte rows,
                                              // conflict-free for 4 lanes x 8 directions)
 constexpr int ID3_TINY = 32;                 // leaves of the 128-thread CTAs
-constexpr int ID3_SMALL = 128;               // leaves of the 256-thread CTAs
-static_assert(ID3_TINY == ID3_TINY_LEAF, "the small-leaf list is the 128-thread launch's");
+constexpr int ID3_SMALL = 64;                // leaves of the 256-thread CTAs
+constexpr int ID3_MID = 128;                 // leaves whose rows a 512-thread CTA holds in registers
+constexpr int ID3_HELD = 28;                 // most pairs per lane
+constexpr int ID3_VP = 400;                  // the residual in the lanes' order (id3_place)
+static_assert(ID3_TINY == ID3_TINY_LEAF && ID3_SMALL == ID3_SMALL_LEAF, "the leaf lists are the launches'");
 static_assert(ID3_P % 8 == 0 && ID3_QS >= ID3_P && ID3_QS % 4 == 0, "proxy pairs, 16-byte rows");
 
 template <int THREADS, int ROWS>
@@ -1642,27 +1697,33 @@ struct Id3 {
     static constexpr int QR = ROWS < Dim<3>::MAXR ? ROWS : Dim<3>::MAXR;   // rank bound
     static constexpr int CS = QR + 1;                                      // row stride of R12 / U
     static constexpr int NW = THREADS / 32;
-    static constexpr int NKMAX = 2 * ROWS > THREADS ? 2 * ROWS / THREADS : 1;   // rows per lane group
-    static constexpr int SMIN = THREADS >= 2 * ROWS ? THREADS / ROWS : 2;       // smallest lane split
-    static_assert(NKMAX <= 2 && THREADS >= 4 * QR, "row groups, four lanes per direction");
+    static constexpr int REG_ROWS = THREADS / 4;                           // rows held in registers
+    static constexpr int NK = ROWS > REG_ROWS ? (ROWS - REG_ROWS + THREADS / 2 - 1) / (THREADS / 2) : 0;
+    static_assert(THREADS >= 4 * QR || ROWS < QR * 2, "four lanes per direction");
     struct Smem {
         float Q[QR * ID3_QS];                  // directions q_0..q_{r-1}; at the end: y0 partials
-        float C[ROWS * CS];                    // R12 (the rows' dots), then U
-        float4 pa[ID3_P / 2];                  // proxy pairs: (-2x, -2x', -2y, -2y')
-        float4 pb[ID3_P / 2];                  //              (-2z, -2z', |p|^2, |p'|^2)
-        float4 cand[ROWS];                     // candidates: (x, y, z) - centre, 1 + |.|^2
+        float4 pa[ID3_NP];                     // proxy pairs: (-2x, -2x', -2y, -2y')
+        float4 pb[ID3_NP];                     //              (-2z, -2z', |p|^2, |p'|^2)
         float R11[QR * (QR + 1) / 2];          // column j at j (j + 1) / 2
+        float4 vp[ID3_VP / 4];                 // the residual's pairs in the order of the rows' lanes
+        float4 red[(NW + 3) / 4];
         float res[ID3_P];                      // the pivot's residual
         float dc[QR];                          // its second-pass projections
         int piv[QR];
-        int selpos[ROWS];                      // pivot position of each row, or -1
         float bv[2][NW];
         int bi[2][NW];
-        float red[NW];
         int coff[9];
         int item;
     };
     static_assert(QR * ID3_QS * sizeof(float) >= THREADS * sizeof(float4), "y0 partials in the directions");
+    // the parts sized by the node's rows m follow: candidates ((x, y, z) - centre, 1 + |.|^2),
+    // pivot position of each row or -1, R12 (the rows' dots, then U), held entries
+    static constexpr size_t fixed() { return (sizeof(Smem) + 15) / 16 * 16; }
+    static constexpr size_t sized(int m) { return (size_t)m * (sizeof(float4) + sizeof(int) + sizeof(float) * CS); }
+    static constexpr size_t row_bytes() { return sizeof(float2) * ID3_NP; }
+    static constexpr size_t most() { return 227 * 1024; }
+    static constexpr size_t smem() { return ROWS > REG_ROWS ? most() : fixed() + sized(ROWS) + 16; }
+    static_assert(fixed() + sized(ROWS) + 16 <= most(), "a node of ROWS candidates fits");
 };
 
 // entry of proxy p (scalar form of the paired arithmetic below: the same operations in the
@@ -1677,78 +1738,106 @@ __device__ __forceinline__ float id3_entry(const SM &s, const float4 &c, int p)
     const float w = fast_rcp(d);
     return w * w;
 }
-
-// Over the lane's share of the proxies (pairs sub, sub + S, ...), for its NK rows
-// g + RPG k: NORM: sum of squared entries (FP64); otherwise the dot product with v (FP32,
-// two partial sums per row).
-template <int S, int NK, bool NORM, typename SM>
-__device__ __forceinline__ void id3_rows(const SM &s, const float *v, int g, int rpg, int sub, double (&out)[2])
+// entries of the pair j of candidate c
+template <typename SM>
+__device__ __forceinline__ F2 id3_pair(const SM &s, const float4 &c, int j)
 {
-    F2 cx[NK], cy[NK], cz[NK], cw[NK], acc[NK];
-    double dn[NK];
-#pragma unroll
-    for (int k = 0; k < NK; k++) {
-        const float4 c = s.cand[g + rpg * k];
-        cx[k] = f2_pack(c.x, c.x); cy[k] = f2_pack(c.y, c.y); cz[k] = f2_pack(c.z, c.z); cw[k] = f2_pack(c.w, c.w);
-        acc[k] = f2_pack(0.f, 0.f);
-        dn[k] = 0.0;
-    }
-#pragma unroll 2
-    for (int j = sub; j < ID3_P / 2; j += S) {
-        const float4 A = s.pa[j], B = s.pb[j];
-        const F2 mx = f2_pack(A.x, A.y), my = f2_pack(A.z, A.w), mz = f2_pack(B.x, B.y), e = f2_pack(B.z, B.w);
-        F2 vv;
-        if (!NORM) {
-            const float2 v2 = *reinterpret_cast<const float2 *>(v + 2 * j);
-            vv = f2_pack(v2.x, v2.y);
-        }
-#pragma unroll
-        for (int k = 0; k < NK; k++) {
-            const F2 d = f2_fma(cz[k], mz, f2_fma(cy[k], my, f2_fma(cx[k], mx, f2_add(cw[k], e))));
-            float d0, d1;
-            f2_unpack(d, d0, d1);
-            const F2 w = f2_pack(fast_rcp(d0), fast_rcp(d1));
-            const F2 w2 = f2_mul(w, w);
-            if (NORM) {
-                float a0, a1;
-                f2_unpack(w2, a0, a1);
-                dn[k] = fma((double)a0, (double)a0, dn[k]);
-                dn[k] = fma((double)a1, (double)a1, dn[k]);
-            } else {
-                acc[k] = f2_fma(w2, vv, acc[k]);
-            }
-        }
-    }
-#pragma unroll
-    for (int k = 0; k < NK; k++) {
-        if (NORM) out[k] = dn[k];
-        else {
-            float a0, a1;
-            f2_unpack(acc[k], a0, a1);
-            out[k] = (double)(a0 + a1);
-        }
-    }
+    const float4 A = s.pa[j], B = s.pb[j];
+    const F2 mx = f2_pack(A.x, A.y), my = f2_pack(A.z, A.w), mz = f2_pack(B.x, B.y), e = f2_pack(B.z, B.w);
+    const F2 d = f2_fma(f2_pack(c.z, c.z), mz,
+                        f2_fma(f2_pack(c.y, c.y), my, f2_fma(f2_pack(c.x, c.x), mx, f2_add(f2_pack(c.w, c.w), e))));
+    float d0, d1;
+    f2_unpack(d, d0, d1);
+    const F2 w = f2_pack(fast_rcp(d0), fast_rcp(d1));
+    return f2_mul(w, w);
+}
+__device__ __forceinline__ void id3_norm2(F2 w, double &dn)
+{
+    float a0, a1;
+    f2_unpack(w, a0, a1);
+    dn = fma((double)a0, (double)a0, dn);
+    dn = fma((double)a1, (double)a1, dn);
+}
+__device__ __forceinline__ F2 id3_v(const float *v, int j)
+{
+    const float2 x = *reinterpret_cast<const float2 *>(v + 2 * j);
+    return f2_pack(x.x, x.y);
+}
+__device__ __forceinline__ float f2_sum(F2 a)
+{
+    float a0, a1;
+    f2_unpack(a, a0, a1);
+    return a0 + a1;
 }
 
-// the lane group's row sums (every lane of the group gets the same values)
-template <bool NORM, int SMIN, int NKMAX, typename SM>
-__device__ __forceinline__ void id3_rows_any(const SM &s, const float *v, int S, int g, int rpg, int sub, int nk,
-                                             double (&out)[2])
+// The lane's part of a row in registers. S >= 4: a lane per chain, lane q holds the pairs q + S i.
+// S == 2: four lanes, lane q (chain q & 1, half q >> 1) holds the pairs (q & 1) + 2 (28 (q >> 1) + i).
+__device__ __forceinline__ int id3_log2(int S) { return S == 2 ? 1 : S == 4 ? 2 : S == 8 ? 3 : 4; }
+__device__ __forceinline__ int id3_count(int S, int q)
 {
-    out[0] = out[1] = 0.0;
-    if (nk > 0) {
-        if (S == 16) id3_rows<16, 1, NORM>(s, v, g, rpg, sub, out);
-        else if (S == 8) id3_rows<8, 1, NORM>(s, v, g, rpg, sub, out);
-        else if (SMIN <= 4 && S == 4) id3_rows<4, 1, NORM>(s, v, g, rpg, sub, out);
-        else if constexpr (SMIN <= 2) {
-            if (NKMAX >= 2 && nk == 2) id3_rows<2, (NKMAX >= 2 ? 2 : 1), NORM>(s, v, g, rpg, sub, out);
-            else id3_rows<2, 1, NORM>(s, v, g, rpg, sub, out);
+    return S == 2 ? (q >> 1 ? 26 : 28) : (ID3_NP - q + S - 1) >> id3_log2(S);
+}
+__device__ __forceinline__ int id3_held_pair(int S, int q, int i) { return S == 2 ? (q & 1) + 2 * (28 * (q >> 1) + i) : q + S * i; }
+// The place of pair j of the residual, so that a lane's pairs lie together and two are one 16-byte
+// load (the lanes' starts fall on different banks).
+__device__ __forceinline__ int id3_stride(int S) { return S <= 4 ? 28 : S == 8 ? 16 : 12; }
+__device__ __forceinline__ int id3_place(int S, int j)
+{
+    return S == 2 ? (j & 1) * 56 + (j >> 1) : (j & (S - 1)) * id3_stride(S) + (j >> id3_log2(S));
+}
+__device__ __forceinline__ int id3_start(int S, int q) { return S == 2 ? (q & 1) * 56 + (q >> 1) * 28 : q * id3_stride(S); }
+
+// w: the lane's entries, zeros after its last; dn: the row's squared norm
+template <typename SM>
+__device__ __forceinline__ void id3_hold(const SM &s, const float4 &c, int S, int q, F2 (&w)[ID3_HELD], double &dn)
+{
+    const int n = id3_count(S, q);
+    dn = 0.0;
+#pragma unroll
+    for (int i = 0; i < ID3_HELD; i++) {
+        w[i] = f2_pack(0.f, 0.f);
+        if (i < n) w[i] = id3_pair(s, c, id3_held_pair(S, q, i));
+        id3_norm2(w[i], dn);   // (a zero leaves it as it is)
+    }
+    if (S == 2) {
+        const double head = __shfl_xor_sync(0xffffffffu, dn, 2);
+        dn = head;   // in the second half: the chain's sum so far
+#pragma unroll
+        for (int i = 0; i < 26; i++) {
+            asm volatile("" : "+l"(w[i].v));   // converted again here, not held as 56 doubles
+            id3_norm2(w[i], dn);
         }
     }
-    for (int o = 1; o < S; o <<= 1) {
-        out[0] += __shfl_xor_sync(0xffffffffu, out[0], o);
-        out[1] += __shfl_xor_sync(0xffffffffu, out[1], o);
+    for (int o = 1; o < S; o <<= 1) dn += __shfl_xor_sync(0xffffffffu, dn, o);
+}
+// acc = fma(w[i], v[i], acc) over the lane's pairs, four at a time. Past its last pair the lane
+// holds zeros, and the residual's places there hold finite values: the sum is unchanged.
+__device__ __forceinline__ F2 id3_chain(const F2 (&w)[ID3_HELD], const float4 *v, int n, F2 acc)
+{
+#pragma unroll
+    for (int i = 0; i < ID3_HELD; i += 4) {
+        if (i >= n) break;   // uniform: n is the longest lane's
+        const float4 x = v[i / 2], y = v[i / 2 + 1];
+        acc = f2_fma(w[i], f2_pack(x.x, x.y), acc);
+        acc = f2_fma(w[i + 1], f2_pack(x.z, x.w), acc);
+        acc = f2_fma(w[i + 2], f2_pack(y.x, y.y), acc);
+        acc = f2_fma(w[i + 3], f2_pack(y.z, y.w), acc);
     }
+    return acc;
+}
+// The row's dot product with the residual (complete in every lane; S == 2: in the lanes of the
+// second half). n: the longest lane's pairs.
+__device__ __forceinline__ float id3_dot_held(const float4 *v, int n, int S, const F2 (&w)[ID3_HELD])
+{
+    F2 acc = id3_chain(w, v, n, f2_pack(0.f, 0.f));
+    if (S == 2) {
+        acc.v = __shfl_xor_sync(0xffffffffu, acc.v, 2);   // in the second half: the chain's sum so far
+        const float y = f2_sum(id3_chain(w, v, n, acc));
+        return __fadd_rn(y, __shfl_xor_sync(0xffffffffu, y, 1));   // = the FP64 sum of two, rounded
+    }
+    double out = (double)f2_sum(acc);
+    for (int o = 1; o < S; o <<= 1) out += __shfl_xor_sync(0xffffffffu, out, o);
+    return (float)out;
 }
 
 // d[j] = q_j . res for the directions j < r (four lanes per direction, 54 proxies each)
@@ -1777,6 +1866,7 @@ __device__ __forceinline__ float id3_sub(const float *Q, int r, int p, const flo
 {
     float a0 = v, a1 = 0.f, a2 = 0.f, a3 = 0.f;
     int j = 0;
+#pragma unroll 2
     for (; j + 3 < r; j += 4) {
         a0 = fmaf(-d[j], Q[j * ID3_QS + p], a0);
         a1 = fmaf(-d[j + 1], Q[(j + 1) * ID3_QS + p], a1);
@@ -1790,14 +1880,15 @@ __device__ __forceinline__ float id3_sub(const float *Q, int r, int p, const flo
 template <int THREADS>
 constexpr int id3_min_blocks() { return THREADS >= 512 ? 1 : (THREADS >= 256 ? 2 : 4); }
 
-// LEAVES: the leaves of `items` with mlo < points <= ROWS (others are another launch's).
+// LEAVES: the leaves of `items` with mlo < points <= ROWS (others are another launch's); `chains`
+// is the thread count by which S is chosen.
 template <bool LEAVES, int THREADS, int ROWS>
 __global__ void __launch_bounds__(THREADS, id3_min_blocks<THREADS>())
-k_id3(int n_item, const int *__restrict__ items, int mlo, IdArgs g, DepArgs dp)
+k_id3(int n_item, const int *__restrict__ items, int mlo, int chains, IdArgs g, DepArgs dp)
 {
     using K = Id3<THREADS, ROWS>;
     using SM = typename K::Smem;
-    constexpr int P = ID3_P, MAXR = Dim<3>::MAXR, QR = K::QR, CS = K::CS, NW = K::NW;
+    constexpr int P = ID3_P, MAXR = Dim<3>::MAXR, QR = K::QR, CS = K::CS, NW = K::NW, NK = K::NK;
     constexpr int PPT = (P + THREADS - 1) / THREADS;   // proxies per thread in the pivot's steps
     extern __shared__ __align__(16) unsigned char smraw[];
     SM &s = *reinterpret_cast<SM *>(smraw);
@@ -1813,36 +1904,37 @@ k_id3(int n_item, const int *__restrict__ items, int mlo, IdArgs g, DepArgs dp)
         if (mm <= mlo || mm > ROWS) return;   // uniform over the CTA
     }
     const int cfirst = tv.fchild[t], nch = LEAVES ? 0 : tv.nchild[t];
-    if (!LEAVES && tid < nch && !tv.leaf[cfirst + tid]) dep_wait(dp, cfirst + tid);
-    __syncthreads();
-    if (tid == 0) {
-        int acc = 0;
-        for (int c = 0; c < nch; c++) {
-            s.coff[c] = acc;
-            acc += __ldcg(g.rank + cfirst + c);
-        }
-        s.coff[nch] = acc;
-    }
-    __syncthreads();
-    const int m = LEAVES ? tv.end[t] - tv.start[t] : s.coff[nch];
     const int s0 = tv.start[t];
     const int lvl = tv.level[t];
     const long long roff = g.rowoff[t];
     float *U = g.U + roff * MAXR;
     const float4 *xt = (const float4 *)g.xt;
     float4 *skel = (float4 *)g.skel;
+    for (int j = tid; j < ID3_NP; j += THREADS) {
+        const float4 *row = tv.proxies + (size_t)lvl * PROXY_F4;
+        s.pa[j] = row[j];
+        s.pb[j] = row[ID3_NP + j];
+    }
+    for (int j = tid; j < ID3_VP / 4; j += THREADS) s.vp[j] = make_float4(0.f, 0.f, 0.f, 0.f);
     const double h = tv.info->radius / (double)(1LL << lvl);
     float ctr[3];
     for (int k = 0; k < 3; k++)
         ctr[k] = (float)(tv.info->corner[k] + (double)(2 * tv.ix[(size_t)t * 3 + k] + 1) * h);
-    for (int j = tid; j < P / 2; j += THREADS) {
-        float p0[3], p1[3];
-        proxy_point<3>(2 * j, h, p0);
-        proxy_point<3>(2 * j + 1, h, p1);
-        s.pa[j] = make_float4(-2.f * p0[0], -2.f * p1[0], -2.f * p0[1], -2.f * p1[1]);
-        s.pb[j] = make_float4(-2.f * p0[2], -2.f * p1[2], fmaf(p0[0], p0[0], fmaf(p0[1], p0[1], p0[2] * p0[2])),
-                              fmaf(p1[0], p1[0], fmaf(p1[1], p1[1], p1[2] * p1[2])));
+    if (!LEAVES && tid < nch && !tv.leaf[cfirst + tid]) dep_wait(dp, cfirst + tid);
+    __syncthreads();
+    if (!LEAVES) {
+        if (tid < nch) s.coff[tid + 1] = __ldcg(g.rank + cfirst + tid);
+        __syncthreads();
+        if (tid == 0) {
+            s.coff[0] = 0;
+            for (int c = 0; c < nch; c++) s.coff[c + 1] += s.coff[c];
+        }
+        __syncthreads();
     }
+    const int m = LEAVES ? tv.end[t] - tv.start[t] : s.coff[nch];
+    float4 *cand = reinterpret_cast<float4 *>(smraw + K::fixed());
+    int *selpos = reinterpret_cast<int *>(cand + m);
+    float *C = reinterpret_cast<float *>(selpos + m);
     for (int a = tid; a < m; a += THREADS) {
         float4 x;
         if (LEAVES) x = xt[s0 + a];
@@ -1852,55 +1944,93 @@ k_id3(int n_item, const int *__restrict__ items, int mlo, IdArgs g, DepArgs dp)
             x = __ldcg(skel + (size_t)(cfirst + c) * MAXR + (a - s.coff[c]));
         }
         const float rx = x.x - ctr[0], ry = x.y - ctr[1], rz = x.z - ctr[2];
-        s.cand[a] = make_float4(rx, ry, rz, 1.f + fmaf(rx, rx, fmaf(ry, ry, rz * rz)));
-        s.selpos[a] = -1;
+        cand[a] = make_float4(rx, ry, rz, 1.f + fmaf(rx, rx, fmaf(ry, ry, rz * rz)));
+        selpos[a] = -1;
     }
     __syncthreads();
 
-    int S = 2;   // uniform over the CTA
-    while (S < 16 && THREADS / (2 * S) >= m) S <<= 1;
-    const int rpg = THREADS / S, sub = tid & (S - 1), rb = tid / S;
-    const int nk = max(0, min(K::NKMAX, (m - rb + rpg - 1) / rpg));   // rows rb + rpg k < m
-    double nrm[2];
-    int pos[2];   // -1: open row, -2: no row, >= 0: pivot position
-    id3_rows_any<true, K::SMIN, K::NKMAX>(s, nullptr, S, rb, rpg, sub, nk, nrm);
+    int S = 2;   // chains per row; uniform over the CTA
+    while (S < 16 && chains / (2 * S) >= m) S <<= 1;
+    const int lanes = S > 4 ? S : 4, q = tid & (lanes - 1), ra = tid >> (S > 4 ? id3_log2(S) : 2);
+    // the lane that keeps a register row's state (its sums are complete there)
+    const bool keeper = q == (S == 2 ? 2 : 0);
+    const int held_n = id3_count(S, 0);
+    const float4 *vrow = s.vp + id3_start(S, q) / 2;
+    F2 w[ID3_HELD];
+    double nrm = -1.0, nrx[NK > 0 ? NK : 1];
+    int pos = -2, pox[NK > 0 ? NK : 1];   // -1: open row, -2: no row, >= 0: pivot position
+    {
+        const float4 c = cand[ra < m ? ra : 0];
+        id3_hold(s, c, S, q, w, nrm);
+        if (ra < m && keeper) pos = -1;
+        else nrm = -1.0;
+    }
+    // further rows (S = 2): two lanes each, in shared memory while it lasts
+    const int mx = NK > 0 ? max(0, m - K::REG_ROWS) : 0;
+    float4 *held = reinterpret_cast<float4 *>(((uintptr_t)(C + (size_t)m * CS) + 15) & ~(uintptr_t)15);
+    const int nheld = NK > 0 ? min(mx, (int)((smraw + K::most() - reinterpret_cast<unsigned char *>(held)) / (int)K::row_bytes())) : 0;
+    const int ch = tid & 1;
 #pragma unroll
-    for (int k = 0; k < 2; k++) {
-        pos[k] = k < nk ? -1 : -2;
-        if (pos[k] == -2) nrm[k] = -1.0;
+    for (int k = 0; k < NK; k++) {
+        const int x = tid / 2 + k * (THREADS / 2);
+        double dn = 0.0;
+        pox[k] = -2;
+        if (x < mx) {
+            const float4 c = cand[K::REG_ROWS + x];
+            for (int i = 0; i < ID3_NP / 4; i++) {   // the chain's pairs 2i and 2i + 1
+                const F2 e0 = id3_pair(s, c, ch + 4 * i), e1 = id3_pair(s, c, ch + 4 * i + 2);
+                if (x < nheld) {
+                    float4 e;
+                    f2_unpack(e0, e.x, e.y);
+                    f2_unpack(e1, e.z, e.w);
+                    held[i * 2 * nheld + 2 * x + ch] = e;
+                }
+                id3_norm2(e0, dn);
+                id3_norm2(e1, dn);
+            }
+        }
+        dn += __shfl_xor_sync(0xffffffffu, dn, 1);
+        nrx[k] = -1.0;
+        if (x < mx && ch == 0) { pox[k] = -1; nrx[k] = dn; }
     }
     float bv = -1.f, lmax = 0.f;
     int bi = INT_MAX;
-#pragma unroll
-    for (int k = 0; k < 2; k++) {
-        const float v = (float)nrm[k];
-        if (pos[k] == -1 && sub == 0 && v > bv) { bv = v; bi = rb + rpg * k; }
+    if (pos == -1) {
+        const float v = (float)nrm;
         lmax = fmaxf(lmax, v);
+        if (v > bv) { bv = v; bi = ra; }
     }
+#pragma unroll
+    for (int k = 0; k < NK; k++)
+        if (pox[k] == -1) {
+            const float v = (float)nrx[k];
+            lmax = fmaxf(lmax, v);
+            if (v > bv) { bv = v; bi = K::REG_ROWS + tid / 2 + k * (THREADS / 2); }
+        }
     lmax = __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(lmax)));
     warp_argmax(bv, bi);
-    if (lane == 0) { s.red[wid] = lmax; s.bv[0][wid] = bv; s.bi[0][wid] = bi; }
+    if (lane == 0) { reinterpret_cast<float *>(s.red)[wid] = lmax; s.bv[0][wid] = bv; s.bi[0][wid] = bi; }
     __syncthreads();
-    float n0 = 0.f;
-    for (int w = 0; w < NW; w++) n0 = fmaxf(n0, s.red[w]);
+    float *red = reinterpret_cast<float *>(s.red);
+    const float n0 = __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(lane < NW ? red[lane] : 0.f)));
+    __syncthreads();   // red is used again
     const float stop2 = g.tol2 * n0;
     const int rmax = min(min(m, P), QR);
     int r = 0, buf = 0;
     while (r < rmax) {
-        float v = s.bv[buf][0];
-        int best = s.bi[buf][0];
-        for (int w = 1; w < NW; w++)
-            if (s.bv[buf][w] > v || (s.bv[buf][w] == v && s.bi[buf][w] < best)) { v = s.bv[buf][w]; best = s.bi[buf][w]; }
+        float v = lane < NW ? s.bv[buf][lane] : -1.f;
+        int best = lane < NW ? s.bi[buf][lane] : INT_MAX;
+        warp_argmax(v, best);
         if (best == INT_MAX || !(v > stop2) || !(v > 0.f)) break;
         // the pivot's residual: thread tid takes the proxies tid + THREADS i
-        const float *cb = s.C + best * CS;   // the pivot's projections on q_0..q_{r-1}
+        const float *cb = C + best * CS;   // the pivot's projections on q_0..q_{r-1}
         float rv[PPT];
 #pragma unroll
         for (int i = 0; i < PPT; i++) {
             const int p = tid + THREADS * i;
             rv[i] = 0.f;
             if (p < P) {
-                rv[i] = id3_sub(s.Q, r, p, cb, id3_entry(s, s.cand[best], p));
+                rv[i] = id3_sub(s.Q, r, p, cb, id3_entry(s, cand[best], p));
                 s.res[p] = rv[i];
             }
         }
@@ -1913,43 +2043,73 @@ k_id3(int n_item, const int *__restrict__ items, int mlo, IdArgs g, DepArgs dp)
             const int p = tid + THREADS * i;
             if (p < P) {
                 rv[i] = id3_sub(s.Q, r, p, s.dc, rv[i]);
-                s.res[p] = rv[i];
+                reinterpret_cast<float *>(s.vp)[2 * id3_place(S, p >> 1) + (p & 1)] = rv[i];
                 sq = fmaf(rv[i], rv[i], sq);
             }
         }
         for (int o = 16; o > 0; o >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, o);
-        if (lane == 0) s.red[wid] = sq;
+        if (lane == 0) red[wid] = sq;
         __syncthreads();
-        float rr2 = 0.f;
-        for (int w = 0; w < NW; w++) rr2 += s.red[w];
-        const float rr = sqrtf(rr2);
+        float rr2 = 0.f;   // the warps that have proxies, in order
+        constexpr int PW = NW < (P + 31) / 32 ? NW : (P + 31) / 32;
+#pragma unroll
+        for (int x = 0; x < PW; x += 4) {
+            const float4 y = s.red[x / 4];
+            rr2 += y.x;
+            if (x + 1 < PW) rr2 += y.y;
+            if (x + 2 < PW) rr2 += y.z;
+            if (x + 3 < PW) rr2 += y.w;
+        }
+        const float rr = __fsqrt_rn(rr2);
         if (!(rr > 0.f) || !(rr < INFINITY)) break;   // uniform: every thread sums the same values
-        const float inv = 1.0f / rr;
+        const float inv = __frcp_rn(rr);
 #pragma unroll
         for (int i = 0; i < PPT; i++)
             if (tid + THREADS * i < P) s.Q[r * ID3_QS + tid + THREADS * i] = rv[i] * inv;
         if (tid < r) s.R11[r * (r + 1) / 2 + tid] = cb[tid] + s.dc[tid];
         if (tid == r) s.R11[r * (r + 1) / 2 + r] = rr;
-        if (tid == 0) { s.piv[r] = best; s.selpos[best] = r; }
-#pragma unroll
-        for (int k = 0; k < 2; k++)
-            if (pos[k] == -1 && rb + rpg * k == best) { pos[k] = r; nrm[k] = -1.0; }
+        if (tid == 0) { s.piv[r] = best; selpos[best] = r; }
+        if (pos == -1 && ra == best) pos = r;
         // every open row: c = a . q_r (from the unscaled residual), its R12 entry; squared
         // residual norm -= c^2
-        double part[2];
-        id3_rows_any<false, K::SMIN, K::NKMAX>(s, s.res, S, rb, rpg, sub, nk, part);
         bv = -1.f;
         bi = INT_MAX;
+        const float part = id3_dot_held(vrow, held_n, S, w);
+        if (pos == -1) {
+            const float c = part * inv;
+            nrm = fmax(nrm - (double)c * (double)c, 0.0);
+            C[ra * CS + r] = c;
+            const float nv = (float)nrm;
+            if (nv > bv) { bv = nv; bi = ra; }
+        }
 #pragma unroll
-        for (int k = 0; k < 2; k++) {
-            const float c = (float)part[k] * inv;
-            if (pos[k] == -1) {
-                nrm[k] = fmax(nrm[k] - (double)c * (double)c, 0.0);
-                if (sub == 0) {
-                    s.C[(rb + rpg * k) * CS + r] = c;
-                    const float nv = (float)nrm[k];
-                    if (nv > bv) { bv = nv; bi = rb + rpg * k; }
+        for (int k = 0; k < NK; k++) {
+            if (k * (THREADS / 2) >= mx) break;   // uniform
+            const int x = tid / 2 + k * (THREADS / 2), a = K::REG_ROWS + x;
+            F2 acc = f2_pack(0.f, 0.f);
+            if (x < nheld) {
+                const float4 *e = held + 2 * x + ch, *v4 = s.vp + ch * 28;
+#pragma unroll 9
+                for (int i = 0; i < ID3_NP / 4; i++) {
+                    const float4 y = e[i * 2 * nheld], v = v4[i];
+                    acc = f2_fma(f2_pack(y.x, y.y), f2_pack(v.x, v.y), acc);
+                    acc = f2_fma(f2_pack(y.z, y.w), f2_pack(v.z, v.w), acc);
                 }
+            } else if (x < mx) {
+                const float4 c = cand[a];
+                const float *v2 = reinterpret_cast<const float *>(s.vp);
+#pragma unroll 2
+                for (int i = 0; i < ID3_NP / 2; i++)
+                    acc = f2_fma(id3_pair(s, c, ch + 2 * i), id3_v(v2, ch * 56 + i), acc);
+            }
+            const float y = f2_sum(acc), px = __fadd_rn(y, __shfl_xor_sync(0xffffffffu, y, 1));
+            if (pox[k] == -1 && a == best) pox[k] = r;
+            if (pox[k] == -1) {
+                const float c = px * inv;
+                nrx[k] = fmax(nrx[k] - (double)c * (double)c, 0.0);
+                C[a * CS + r] = c;
+                const float nv = (float)nrx[k];
+                if (nv > bv) { bv = nv; bi = a; }
             }
         }
         warp_argmax(bv, bi);
@@ -1976,19 +2136,36 @@ k_id3(int n_item, const int *__restrict__ items, int mlo, IdArgs g, DepArgs dp)
         __syncthreads();
         if (tid == 0) dep_publish(dp, t);
     }
-    // U = R12 times R11^-1 for the open rows (back substitution, one thread per row), the
-    // pivot rows rows of the identity
+    // U = R12 times R11^-1 for the open rows (back substitution, one thread per row, four columns
+    // at a time in registers: column i takes the later columns k in decreasing order, then its
+    // division), the pivot rows rows of the identity
     for (int a = tid; a < m; a += THREADS) {
-        float *u = s.C + a * CS;
-        const int sp = s.selpos[a];
+        float *u = C + a * CS;
+        const int sp = selpos[a];
         if (sp >= 0) {
             for (int i = 0; i < r; i++) u[i] = i == sp ? 1.f : 0.f;
-        } else {
-            for (int k = r - 1; k >= 0; k--) {
-                const float *col = s.R11 + k * (k + 1) / 2;
-                const float uk = u[k] / col[k];
-                u[k] = uk;
-                for (int i = 0; i < k; i++) u[i] = fmaf(-col[i], uk, u[i]);
+            continue;
+        }
+        for (int top = r - 1; top >= 0; top -= 4) {
+            float acc[4];
+#pragma unroll
+            for (int z = 0; z < 4; z++) acc[z] = top - z >= 0 ? u[top - z] : 0.f;
+            for (int k = r - 1; k > top; k--) {
+                const float uk = u[k];
+                const float *col = s.R11 + k * (k + 1) / 2 + top;
+#pragma unroll
+                for (int z = 0; z < 4; z++)
+                    if (top - z >= 0) acc[z] = fmaf(-col[-z], uk, acc[z]);
+            }
+#pragma unroll
+            for (int z = 0; z < 4; z++) {
+                if (top - z < 0) break;
+                const float *col = s.R11 + (top - z) * (top - z + 1) / 2;
+                const float uk = acc[z] / col[top - z];
+                u[top - z] = uk;
+#pragma unroll
+                for (int y = z + 1; y < 4; y++)
+                    if (top - y >= 0) acc[y] = fmaf(-col[top - y], uk, acc[y]);
             }
         }
     }
@@ -1996,18 +2173,19 @@ k_id3(int n_item, const int *__restrict__ items, int mlo, IdArgs g, DepArgs dp)
     __syncthreads();
     for (int idx = tid; idx < m * r; idx += THREADS) {
         const int a = idx / r, k = idx - a * r;
-        U[(size_t)a * MAXR + k] = s.C[a * CS + k];
+        U[(size_t)a * MAXR + k] = C[a * CS + k];
     }
     // upward coefficients y0 = U^T (the leaf's [1 | x] | the children's y0): groups of RG
-    // threads over k and THREADS / RG groups over the rows, summed in a fixed order
+    // threads over k and YT / RG groups over the rows, summed in a fixed order
     {
+        const int YT = min(THREADS, chains);
         float4 *part = reinterpret_cast<float4 *>(s.Q);
         const int RG = r <= 16 ? 16 : (r <= 32 ? 32 : 64);
-        const int C = THREADS / RG, kk = tid % RG, cg = tid / RG;
+        const int G = YT / RG, kk = tid % RG, cg = tid / RG;
         float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (kk < r) {
-            for (int a = cg; a < m; a += C) {
-                const float w = s.C[a * CS + kk];
+        if (kk < r && cg < G) {
+            for (int a = cg; a < m; a += G) {
+                const float w = C[a * CS + kk];
                 if (LEAVES) {
                     const float4 x = xt[s0 + a];
                     acc.x += w;
@@ -2025,7 +2203,7 @@ k_id3(int n_item, const int *__restrict__ items, int mlo, IdArgs g, DepArgs dp)
         __syncthreads();
         if (tid < r) {
             float4 y = part[tid];
-            for (int c = 1; c < C; c++) add4(y, part[c * RG + tid]);
+            for (int c = 1; c < G; c++) add4(y, part[c * RG + tid]);
             g.y0[(size_t)t * MAXR + tid] = y;
         }
     }
@@ -2613,6 +2791,7 @@ public:
         blkcnt_.exact((size_t)ceil_div(n, TREE_BLOCK) * 64);
         blkoff_.exact((size_t)ceil_div(n, TREE_BLOCK) * 64);
         btot_.exact(64);
+        proxies_.exact((size_t)(Dim<D>::L + 1) * PROXY_F4);
         tickets_.exact(N_TICKET);
         done_.exact(1);
         TSNE_CUDA_CHECK(cudaMemsetAsync(tickets_.p, 0, sizeof(int) * N_TICKET, st_));
@@ -2641,6 +2820,7 @@ public:
         if (D == 3) {
             id3_attr<false, 512, ID3_ROWS>();
             id3_attr<true, 512, ID3_ROWS>();
+            id3_attr<true, 512, ID3_MID>();
             id3_attr<true, 256, ID3_SMALL>();
             id3_attr<true, 128, ID3_TINY>();
         }
@@ -2721,6 +2901,7 @@ public:
         hint_ = I.n_int;
         hleaf_ = I.n_small;
         hbig_ = I.n_big;
+        hlarge_ = I.n_large;
         hfine_ = I.n_fine;
         if (max_level_ <= 2) { built_ = false; return 1; }
 
@@ -2815,15 +2996,16 @@ public:
         }
         DepArgs dp{flag_.p, tickets_.p + TICKET_BASES, &info_.p->pad[1], ++epoch_};
         if (D == 3 && id3_) {
-            // recomputed-row decompositions: leaves by size (llist: at most ID3_TINY points;
-            // blist: the others, up to ID3_ROWS; larger leaves, only at the depth limit, take
-            // k_id), then the internal nodes in one dependency-ordered launch
+            // leaves by size (llist: at most ID3_TINY points; blist: at most ID3_SMALL; clist: the
+            // others, up to ID3_ROWS; larger leaves, only at the depth limit, take k_id), then
+            // the internal nodes in one dependency-ordered launch
             if (stats_.max_leaf <= ID3_ROWS) {
-                if (hleaf_ > 0) id3_launch<true, 128, ID3_TINY>(hleaf_, llist_.p, 0, il, dp);
-                if (hbig_ > 0) {
-                    id3_launch<true, 256, ID3_SMALL>(hbig_, blist_.p, ID3_TINY, il, dp);
-                    if (stats_.max_leaf > ID3_SMALL) id3_launch<true, 512, ID3_ROWS>(hbig_, blist_.p, ID3_SMALL, il, dp);
+                if (hlarge_ > 0) {
+                    id3_launch<true, 512, ID3_MID>(hlarge_, clist_.p, ID3_SMALL, 256, il, dp);
+                    if (stats_.max_leaf > ID3_MID) id3_launch<true, 512, ID3_ROWS>(hlarge_, clist_.p, ID3_MID, 512, il, dp);
                 }
+                if (hbig_ > 0) id3_launch<true, 256, ID3_SMALL>(hbig_, blist_.p, ID3_TINY, 256, il, dp);
+                if (hleaf_ > 0) id3_launch<true, 128, ID3_TINY>(hleaf_, llist_.p, 0, 128, il, dp);
             } else {
                 k_id<D, true><<<n_node_ - first, IDG_THREADS, id_smem_bytes<D>(mleaf), st_>>>(MIN_ADM_LEVEL, il, 0,
                                                                                               nullptr, dp);
@@ -2835,7 +3017,7 @@ public:
             if (hint_ > 0) {
                 DepArgs d2 = dp;
                 d2.flag2 = flag2_.p;
-                id3_launch<false, 512, ID3_ROWS>(hint_, ilist_.p, 0, il, d2);
+                id3_launch<false, 512, ID3_ROWS>(hint_, ilist_.p, 0, 512, il, d2);
             }
             near_launch_side();
             mark_end(t_bases, 7);
@@ -2875,7 +3057,7 @@ public:
         k_lists<D><<<std::min(148 * LIST_CTAS, ceil_div(cap_node_, LIST_WARPS)), 32 * LIST_WARPS, 0, st_>>>(
             view(), list_out(), dp);
         const NodeScan q{far_cnt_.p, near_cnt_.p, fine_cnt_.p, far_ptr_.p, near_ptr_.p, rowoff_.p, ilist_.p, llist_.p,
-                         blist_.p, flist_.p, rank_.p, node_blk_.p};
+                         blist_.p, clist_.p, flist_.p, rank_.p, node_blk_.p};
         const int nb = ceil_div(cap_node_, NODE_BLOCK);
         k_node_sums<D><<<nb, NODE_BLOCK, 0, st_>>>(view(), q);
         k_node_scan<D><<<nb, NODE_BLOCK, 0, st_>>>(view(), q);
@@ -2889,7 +3071,7 @@ public:
         nset_cnt_.exact(c + 1);
         far_cnt_.exact(c + 1); near_cnt_.exact(c + 1); fine_cnt_.exact(c + 1);
         far_ptr_.exact(c + 2); near_ptr_.exact(c + 2);
-        ilist_.exact(c + 1); llist_.exact(c + 1); blist_.exact(c + 1); flist_.exact(c + 1);
+        ilist_.exact(c + 1); llist_.exact(c + 1); blist_.exact(c + 1); clist_.exact(D == 3 ? c + 1 : 1); flist_.exact(c + 1);
         rowoff_.exact(c + 2);
         rank_.exact(c);
         node_blk_.exact(ceil_div(c, NODE_BLOCK));
@@ -3096,13 +3278,13 @@ private:
     static void id3_attr()
     {
         TSNE_CUDA_CHECK(cudaFuncSetAttribute(k_id3<LEAVES, THREADS, ROWS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)sizeof(typename Id3<THREADS, ROWS>::Smem)));
+                                             (int)Id3<THREADS, ROWS>::smem()));
     }
     template <bool LEAVES, int THREADS, int ROWS>
-    void id3_launch(int n_item, const int *items, int mlo, const IdArgs &a, const DepArgs &dp)
+    void id3_launch(int n_item, const int *items, int mlo, int chains, const IdArgs &a, const DepArgs &dp)
     {
-        k_id3<LEAVES, THREADS, ROWS><<<n_item, THREADS, sizeof(typename Id3<THREADS, ROWS>::Smem), st_>>>(
-            n_item, items, mlo, a, dp);
+        k_id3<LEAVES, THREADS, ROWS><<<n_item, THREADS, Id3<THREADS, ROWS>::smem(), st_>>>(n_item, items, mlo, chains, a,
+                                                                                           dp);
         launches_++;
     }
 
@@ -3133,7 +3315,7 @@ private:
         TreeView v;
         v.n = n_; v.L = Dim<D>::L; v.leaf_size = leaf_size_; v.cap_node = cap_node_; v.nset_cap = nset_cap_;
         v.keys = keys_.p; v.start = start_.p; v.end = end_.p; v.level = level_.p; v.parent = parent_.p;
-        v.fchild = fchild_.p; v.nchild = nchild_.p; v.leaf = leaf_.p; v.ix = ix_.p; v.rec = rec_.p;
+        v.fchild = fchild_.p; v.nchild = nchild_.p; v.leaf = leaf_.p; v.ix = ix_.p; v.rec = rec_.p; v.proxies = proxies_.p;
         v.delta = delta_.p; v.fm = fm_.p; v.blkcnt = blkcnt_.p; v.blkoff = blkoff_.p;
         v.bset = bset_.p; v.nid = nid_.p; v.btot = btot_.p; v.tickets = tickets_.p;
         v.info = info_.p;
@@ -3294,6 +3476,7 @@ private:
     cudaStream_t st2_ = nullptr;  // side stream: the list write and the near field beside the bases
     cudaEvent_t fork_ev_ = nullptr, near_ev_ = nullptr, lists_ev_ = nullptr;
     bool near_pending_ = false, lists_pending_ = false;
+    DevBuf<float4> proxies_;             // proxy table, a row per level
     DevBuf<int4> rec_;                   // node records of the list pass
     DevBuf<int> far_slot_, near_slot_;   // list entries parked by the count pass
     int epoch_ = 0;
@@ -3302,9 +3485,9 @@ private:
     DevBuf<NodeSums> node_blk_;          // block sums of the node scan
     DevBuf<int> ilist_;                  // internal nodes at level >= 2, in increasing id
     DevBuf<int> llist_;                  // leaves at level >= 2 of at most LEAF_SMALL points
-    DevBuf<int> blist_;                  // the larger leaves at level >= 2
+    DevBuf<int> blist_, clist_;          // the larger leaves at level >= 2
     DevBuf<int> flist_, fine_cnt_;       // leaves with finer far entries, and how many each node has
-    int hint_ = 0, hleaf_ = 0, hbig_ = 0, hfine_ = 0;
+    int hint_ = 0, hleaf_ = 0, hbig_ = 0, hlarge_ = 0, hfine_ = 0;
     cudaEvent_t counts_ev_ = nullptr;   // end of a build's count batch (host waits on it)
     DevBuf<long long> rowoff_;
     DevBuf<int> rank_;

@@ -34,7 +34,7 @@ struct TreeInfo {
     double radius;
     // totals of the list counts and of the basis launches' items
     long long n_rows;
-    int n_far, n_near, n_int, n_small, n_big, n_fine;
+    int n_far, n_near, n_int, n_small, n_big, n_large, n_fine;
 };
 
 // ---- dense per-point kernels (dense.cu) ----
