@@ -893,15 +893,13 @@ __global__ void __launch_bounds__(256) k_lists_compact(TreeView tv, ListOut lo)
 // (its rows of the interpolation matrices: a leaf's points, or the upper bound of the children's
 // skeletons; nodes above MIN_ADM_LEVEL have none), the item lists of the basis launches
 // (ilist: the internal nodes at level >= MIN_ADM_LEVEL; llist / blist: the leaves there of at most
-// LEAF_SMALL points / the larger ones; 3D: at most ID3_TINY_LEAF / ID3_SMALL_LEAF points, and clist
-// the larger ones) and flist, the leaves with far entries
+// TINY_LEAF / SMALL_LEAF points, clist: the larger ones) and flist, the leaves with far entries
 // finer than themselves; each list in increasing node id.
 // Two launches over the nodes there are (block sums, then every block adds the sums before its
 // own): six device-wide scans over the node capacity and their flag and memset launches took
 // 25 launches, 75 us of a rebuild at 20K points and 85 us at 1M.
-constexpr int LEAF_SMALL = 64;
-constexpr int ID3_TINY_LEAF = 32;    // 3D: the leaves of the smallest basis CTAs,
-constexpr int ID3_SMALL_LEAF = 64;   // and of the next
+constexpr int TINY_LEAF = 32;    // the leaves of the smallest basis CTAs,
+constexpr int SMALL_LEAF = 64;   // and of the next
 constexpr int NODE_BLOCK = 1024;
 
 struct NodeSums {
@@ -959,8 +957,8 @@ __device__ __forceinline__ NodeSums node_counts(const TreeView &tv, const NodeSc
     } else {
         const int r = tv.end[t] - tv.start[t];
         c.rows = r;
-        if (r <= (D == 2 ? LEAF_SMALL : ID3_TINY_LEAF)) c.small = 1;
-        else if (D == 2 || r <= ID3_SMALL_LEAF) c.big = 1;
+        if (r <= TINY_LEAF) c.small = 1;
+        else if (r <= SMALL_LEAF) c.big = 1;
         else c.large = 1;
     }
     return c;
@@ -1345,6 +1343,13 @@ __global__ void __launch_bounds__(IDG_THREADS) k_id(int level, IdArgs g, int n_i
 
 
 
+__device__ __forceinline__ float f2_sum(F2 a)
+{
+    float a0, a1;
+    f2_unpack(a, a0, a1);
+    return a0 + a1;
+}
+
 // Warp argmax of (norm, row): the largest norm, ties to the lowest row. Norms are >= 0 or -1
 // (no candidate), so their bit patterns order like the values.
 __device__ __forceinline__ void warp_argmax(float &bv, int &bi)
@@ -1355,38 +1360,66 @@ __device__ __forceinline__ void warp_argmax(float &bv, int &bi)
     bv = __int_as_float(mx);
 }
 
-// Interpolative decompositions of the 2D nodes at level >= 2, one CTA of THREADS threads per
-// node, thread `tid` owning candidate row tid (its row of A = K(candidate - c, proxies) in
-// registers). LEAVES: every leaf (candidates = its points; CTAs of 64 threads for leaves of at
-// most 64 points, which fit seven to an SM, and of 128 for the others). Otherwise every
-// internal node in one dependency-ordered launch (candidates = the children's skeletons):
-// items in decreasing node id (deepest level first), so a node's internal children come
-// before it; it waits for their first flags (skeleton and rank, published right after their
+// Interpolative decompositions of the 2D nodes at level >= 2, one CTA per node, two lanes per
+// candidate row of A = K(candidate - c, proxies): lane l holds the row's entries of the proxies
+// 4j + 2l, 4j + 2l + 1 as pairs for the paired FP32 instructions, NS rows per pair of lanes.
+// LEAVES: the leaves of `items` (candidates = their points).
+// Otherwise every internal node in one dependency-ordered launch (candidates = the children's
+// skeletons): items in decreasing node id (deepest level first), so a node's internal children
+// come before it; it waits for their first flags (skeleton and rank, published right after their
 // Gram-Schmidt steps) and, before its own upward sums, for their second flags (coefficients,
-// published last), and reads all of these through L2 (CTAs of 128 threads). When the children's ranks add up to more than 128, thread
-// tid also owns row 128 + tid, kept in global memory (in the node's first U rows, unused until
-// the end).
+// published last), and reads all of these through L2. When the children's ranks add up to more
+// than 128, thread tid < 128 also owns row 128 + tid, kept in global memory (in the node's first U
+// rows, unused until the end).
 // Column-pivoted Gram-Schmidt until the largest residual row norm is <= tol * the largest
 // initial one (ties: the lower row); the dot products of every step are kept in shared
 // memory (row-major, stride MAXR + 1), R11 is gathered from the pivot rows into shared
-// memory, and the back substitution U = [I ; R11^-1 R12]^T runs there. Then U goes out to
-// global memory, with the skeleton and the rank, and the upward coefficients
-// y0 = U^T (the leaf's [1 | x] | the children's y0) are summed by all threads in a fixed order.
-constexpr int ID2_THREADS = 128;                  // internal nodes and leaves of 65..128 points
-constexpr int ID2_SMALL = 64;                     // leaves of at most 64 points
+// memory, and the back substitution U = [I ; R11^-1 R12]^T runs there, two columns per lane and
+// four at a time. Then U goes out to global memory, with the skeleton and the
+// rank, and the upward coefficients y0 = U^T (the leaf's [1 | x] | the children's y0) are summed
+// in a fixed order (yt threads).
+// What bounds it is a node's serial chain (rank x (pivot, barrier, dot product, update, argmax,
+// barrier)) and, along the tree, the levels' chain. With a row per thread a step was 64 loads,
+// 192 FMAs and the pivot's 64 stores by one thread, and a node's rows took 8,000 cycles to evaluate
+// (one long stretch of code); two lanes have 48 paired FMAs (the same four partial sums p mod 4,
+// joined in the same order). Four lanes per row had the same chain and twice the instructions (leaves at 1M
+// points 563 us a rebuild). From a row per thread: leaves 62 -> 36 us at 20K points and 538 -> 443 us at
+// 1M, internal nodes 143 -> 103 us and 537 -> 426 us (three CTAs of 168 registers per SM; four of 128
+// spilled 184 bytes: 131 and 555 us).
 constexpr int ID2_DSTRIDE = Dim<2>::MAXR + 1;
-constexpr size_t id2_smem(int threads) { return sizeof(float) * threads * ID2_DSTRIDE; }   // dot products
+constexpr int ID2_HELD = 128;                     // rows in registers of the internal nodes' CTAs
+constexpr int ID2_TINY = 32, ID2_SMALL = 64;      // leaves of the smaller CTAs
+constexpr int ID2_ONE_LAUNCH = 148 * 4;           // leaves that one launch of the largest CTAs runs at once
+template <int THREADS, int NS> constexpr size_t id2_smem() { return sizeof(float) * (THREADS / 2 * NS) * ID2_DSTRIDE; }
+template <bool LEAVES, int THREADS, int NS>
+constexpr int id2_min_blocks() { return !LEAVES ? 3 : NS == 2 ? 4 : (THREADS == 128 ? 5 : 10); }
+// the leaves of a launch: the items of up to three lists, one after another
+struct LeafItems {
+    const int *list[3];
+    int n[3];
+};
+__device__ __forceinline__ int leaf_item(const LeafItems &x, int i)
+{
+    if (i < x.n[0]) return x.list[0][i];
+    i -= x.n[0];
+    if (i < x.n[1]) return x.list[1][i];
+    return x.list[2][i - x.n[1]];
+}
+static_assert(ID2_TINY == TINY_LEAF && ID2_SMALL == SMALL_LEAF, "the leaf lists are the launches'");
 
-template <bool LEAVES, int THREADS>
-__global__ void __launch_bounds__(THREADS, THREADS == ID2_SMALL ? 7 : 4)
-k_id2d(int n_item, const int *__restrict__ items, IdArgs g, DepArgs dp)
+template <bool LEAVES, int THREADS, int NS>
+__global__ void __launch_bounds__(THREADS, id2_min_blocks<LEAVES, THREADS, NS>())
+k_id2d(int n_item, const int *__restrict__ items, LeafItems leaves, IdArgs g, DepArgs dp)
 {
     constexpr int P = Dim<2>::NPROXY, MAXR = Dim<2>::MAXR, NW = THREADS / 32;
-    constexpr int ROWS = LEAVES ? THREADS : 2 * THREADS;   // candidate rows a CTA can hold
-    static_assert(LEAVES || (ROWS >= 4 * MAXR && P == MAXR), "overflow rows reuse U rows of MAXR floats");
-    extern __shared__ float dots[];            // [THREADS][ID2_DSTRIDE]
-    __shared__ float prox[P * 2];
-    __shared__ float qsh[P];
+    constexpr int PAIRS = THREADS / 2, HELD = PAIRS * NS, E = P / 4;
+    constexpr int ROWS = LEAVES ? HELD : 4 * MAXR;   // candidate rows a CTA can hold
+    constexpr int QS = 36;                           // stride of a lane's share of the pivot row
+    static_assert(LEAVES || (HELD == ID2_HELD && ROWS <= 2 * HELD && P == MAXR), "overflow rows reuse U rows of MAXR floats");
+    static_assert(P == 64 && NW <= 32 && THREADS >= MAXR, "16 pairs per lane");
+    extern __shared__ float dots[];            // [HELD][ID2_DSTRIDE]
+    __shared__ __align__(8) float px[P], py[P];
+    __shared__ __align__(16) float qsh[2 * QS];   // the pivot row: proxy 4j + 2l + e at l QS + 2j + e
     __shared__ float rdiag[MAXR];
     __shared__ int piv[MAXR];
     __shared__ float R11[MAXR * (MAXR + 1) / 2];   // column jj at jj (jj + 1) / 2
@@ -1398,7 +1431,7 @@ k_id2d(int n_item, const int *__restrict__ items, IdArgs g, DepArgs dp)
     __shared__ float s_lmax[NW];
     __shared__ int s_crank[4], s_item;
     const TreeView &tv = g.tv;
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, ln = tid & 1;
     // internal nodes by level (items == nullptr): one launch per level, node n_item + block,
     // its children finished by the launches before, so nothing waits or publishes
     const bool bylevel = !LEAVES && items == nullptr;
@@ -1411,31 +1444,33 @@ k_id2d(int n_item, const int *__restrict__ items, IdArgs g, DepArgs dp)
     } else {
         const int item = LEAVES ? (int)blockIdx.x : s_item;
         if (item >= n_item) return;
-        t = items[LEAVES ? item : n_item - 1 - item];
+        t = LEAVES ? leaf_item(leaves, item) : items[n_item - 1 - item];
     }
     const int lvl = tv.level[t];
     const float2 *xt = (const float2 *)g.xt;
     float2 *skel = (float2 *)g.skel;
     const int cfirst = tv.fchild[t], nch = LEAVES ? 0 : tv.nchild[t];
+    const int s0 = tv.start[t];
+    const long long roff = g.rowoff[t];
+    float *U = g.U + roff * MAXR;
+    const double h = tv.info->radius / (double)(1LL << lvl);
+    if (tid < P) {
+        const float2 y = reinterpret_cast<const float2 *>(tv.proxies + (size_t)lvl * PROXY_F4)[tid];
+        px[tid] = y.x;
+        py[tid] = y.y;
+    }
+    const float cx = (float)(tv.info->corner[0] + (double)(2 * tv.ix[(size_t)t * 3 + 0] + 1) * h);
+    const float cy = (float)(tv.info->corner[1] + (double)(2 * tv.ix[(size_t)t * 3 + 1] + 1) * h);
     if (!LEAVES && tid < nch) {
         if (!bylevel && !tv.leaf[cfirst + tid]) dep_wait(dp, cfirst + tid);   // leaves: the launch before
         s_crank[tid] = __ldcg(g.rank + cfirst + tid);
     }
     __syncthreads();
     int m = 0;
-    if (LEAVES) m = tv.end[t] - tv.start[t];
+    if (LEAVES) m = tv.end[t] - s0;
     else for (int c = 0; c < nch; c++) m += s_crank[c];
-    const int s0 = tv.start[t];
-    const long long roff = g.rowoff[t];
-    float *U = g.U + roff * MAXR;
-    const double h = tv.info->radius / (double)(1LL << lvl);
-    for (int p = tid; p < P; p += THREADS) proxy_point<2>(p, h, prox + p * 2);
-    const float cx = (float)(tv.info->corner[0] + (double)(2 * tv.ix[(size_t)t * 3 + 0] + 1) * h);
-    const float cy = (float)(tv.info->corner[1] + (double)(2 * tv.ix[(size_t)t * 3 + 1] + 1) * h);
     // candidates and the upward-pass inputs
-    for (int q = 0; q < 2; q++) {
-        const int a = tid + THREADS * q;
-        if (a >= m) break;
+    for (int a = tid; a < m; a += THREADS) {
         float2 pt;
         if (LEAVES) {
             pt = xt[s0 + a];
@@ -1450,72 +1485,93 @@ k_id2d(int n_item, const int *__restrict__ items, IdArgs g, DepArgs dp)
     }
     __syncthreads();
 
-    const bool valid = tid < m;
-    const bool big = !LEAVES && m > THREADS;   // uniform over the block
-    const bool xvalid = big && THREADS + tid < m;
-    float row[P];
-    int pos = valid ? -1 : -2, xpos = xvalid ? -1 : -2;
-    float nrm = -1.f, xnrm = -1.f, lmax = 0.f;
-    {
-        const float2 x = valid ? sxy[tid] : make_float2(0.f, 0.f);
-        const float rx = x.x - cx, ry = x.y - cy;
-        float s4[4] = {0.f, 0.f, 0.f, 0.f};
+    const int a0 = tid >> 1;                     // the lanes' rows: a0 + PAIRS s
+    const int w0 = wid * 16;                     // the warp's first row; a set whose w0 + PAIRS s >= m is empty
+    const bool big = !LEAVES && m > HELD;        // uniform over the block
+    const bool xvalid = big && HELD + tid < m;
+    F2 row[NS][E];
+    float nrm[NS];
+    int pos[NS], xpos = xvalid ? -1 : -2;        // -1: open row, -2: no row, >= 0: pivot position
+    float xnrm = -1.f, lmax = 0.f, bv = -1.f;
+    int bi = INT_MAX;
 #pragma unroll
-        for (int p = 0; p < P; p++) {
-            const float dx = rx - prox[2 * p], dy = ry - prox[2 * p + 1];
-            const float w = valid ? rkernel(fmaf(dx, dx, dy * dy)) : 0.f;
-            row[p] = w;
-            s4[p & 3] = fmaf(w, w, s4[p & 3]);
+    for (int s = 0; s < NS; s++) {
+        const int a = a0 + PAIRS * s;
+        const bool valid = a < m;
+        pos[s] = valid ? -1 : -2;
+        nrm[s] = -1.f;
+        if (w0 + PAIRS * s >= m) continue;
+        const float2 x = sxy[valid ? a : 0];
+        const F2 rx = f2_pack(x.x - cx, x.x - cx), ry = f2_pack(x.y - cy, x.y - cy);
+        F2 zz = f2_pack(0.f, 0.f);
+#pragma unroll
+        for (int j = 0; j < E; j++) {
+            const float2 qx = *reinterpret_cast<const float2 *>(px + 4 * j + 2 * ln);
+            const float2 qy = *reinterpret_cast<const float2 *>(py + 4 * j + 2 * ln);
+            const F2 dx = f2_sub(rx, f2_pack(qx.x, qx.y)), dy = f2_sub(ry, f2_pack(qy.x, qy.y));
+            const F2 d = f2_add(f2_pack(1.f, 1.f), f2_fma(dx, dx, f2_mul(dy, dy)));
+            float d0, d1;
+            f2_unpack(d, d0, d1);
+            const F2 w = f2_pack(fast_rcp(d0), fast_rcp(d1));
+            row[s][j] = f2_mul(w, w);
+            zz = f2_fma(row[s][j], row[s][j], zz);
         }
-        if (valid) nrm = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-        lmax = fmaxf(lmax, fmaxf(nrm, 0.f));
+        float z = f2_sum(zz);
+        z += __shfl_xor_sync(0xffffffffu, z, 1);
+        if (valid) {
+            nrm[s] = z;
+            if (z > bv) { bv = z; bi = a; }
+        }
     }
     float *xr = U + (size_t)tid * MAXR;   // overflow row, in the node's first U rows
     if (xvalid) {
-        const float2 xx = sxy[THREADS + tid];
+        const float2 xx = sxy[HELD + tid];
         const float qx = xx.x - cx, qy = xx.y - cy;
         float z2 = 0.f;
         for (int p = 0; p < P; p++) {
-            const float dx = qx - prox[2 * p], dy = qy - prox[2 * p + 1];
+            const float dx = qx - px[p], dy = qy - py[p];
             const float w = rkernel(fmaf(dx, dx, dy * dy));
             xr[p] = w;
             z2 = fmaf(w, w, z2);
         }
         xnrm = z2;
-        lmax = fmaxf(lmax, z2);
+        if (xnrm > bv) { bv = xnrm; bi = HELD + tid; }
     }
-    float bv = nrm;
-    int bi = valid ? tid : INT_MAX;
-    if (xnrm > bv) { bv = xnrm; bi = THREADS + tid; }
+    lmax = fmaxf(lmax, bv);
     lmax = __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(lmax)));
     warp_argmax(bv, bi);
     if (lane == 0) { s_lmax[wid] = lmax; s_bv[0][wid] = bv; s_bi[0][wid] = bi; }
     __syncthreads();
-    float n0 = 0.f;
-    for (int w = 0; w < NW; w++) n0 = fmaxf(n0, s_lmax[w]);
+    const float n0 = __int_as_float(__reduce_max_sync(0xffffffffu, __float_as_int(lane < NW ? s_lmax[lane] : 0.f)));
     const float stop2 = g.tol2 * n0;
     const int rmax = min(min(m, P), MAXR);
-    float *drow = dots + (size_t)tid * ID2_DSTRIDE;
     int r = 0, buf = 0;
     while (r < rmax) {
-        float v = s_bv[buf][0];
-        int best = s_bi[buf][0];
-        for (int w = 1; w < NW; w++)
-            if (s_bv[buf][w] > v || (s_bv[buf][w] == v && s_bi[buf][w] < best)) { v = s_bv[buf][w]; best = s_bi[buf][w]; }
+        float v = lane < NW ? s_bv[buf][lane] : -1.f;
+        int best = lane < NW ? s_bi[buf][lane] : INT_MAX;
+        warp_argmax(v, best);
         if (best == INT_MAX || !(v > stop2) || !(v > 0.f)) break;
-        if (best == tid) {
-            const float rr = sqrtf(nrm);
-            const float inv = 1.0f / rr;
 #pragma unroll
-            for (int p = 0; p < P; p++) qsh[p] = row[p] * inv;
-            rdiag[r] = rr;
-            piv[r] = best;
-            pos = r;
-            nrm = -1.f;
-        } else if (best == THREADS + tid) {
-            const float rr = sqrtf(xnrm);
-            const float inv = 1.0f / rr;
-            for (int p = 0; p < P; p++) qsh[p] = xr[p] * inv;
+        for (int s = 0; s < NS; s++)
+            if (best == a0 + PAIRS * s) {
+                const float rr = __fsqrt_rn(nrm[s]);
+                const float inv = __frcp_rn(rr);
+                const F2 i2 = f2_pack(inv, inv);
+#pragma unroll
+                for (int j = 0; j < E; j += 2) {
+                    float4 y;
+                    f2_unpack(f2_mul(row[s][j], i2), y.x, y.y);
+                    f2_unpack(f2_mul(row[s][j + 1], i2), y.z, y.w);
+                    *reinterpret_cast<float4 *>(qsh + ln * QS + 2 * j) = y;
+                }
+                if (ln == 0) { rdiag[r] = rr; piv[r] = best; }
+                pos[s] = r;
+                nrm[s] = -1.f;
+            }
+        if (xvalid && best == HELD + tid) {
+            const float rr = __fsqrt_rn(xnrm);
+            const float inv = __frcp_rn(rr);
+            for (int p = 0; p < P; p++) qsh[((p >> 1) & 1) * QS + 2 * (p >> 2) + (p & 1)] = xr[p] * inv;
             rdiag[r] = rr;
             piv[r] = best;
             xpos = r;
@@ -1524,35 +1580,49 @@ k_id2d(int n_item, const int *__restrict__ items, IdArgs g, DepArgs dp)
         __syncthreads();
         bv = -1.f;
         bi = INT_MAX;
-        if (pos == -1) {
-            float d4[4] = {0.f, 0.f, 0.f, 0.f};
+        if (w0 < m) {   // uniform over the warp
+            F2 q[E];
 #pragma unroll
-            for (int p = 0; p < P; p++) d4[p & 3] = fmaf(qsh[p], row[p], d4[p & 3]);
-            const float dot = (d4[0] + d4[1]) + (d4[2] + d4[3]);
-            asm volatile("" ::: "memory");   // reload q below instead of holding 64 more registers
-            float s4[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-            for (int p = 0; p < P; p++) {
-                row[p] = fmaf(-dot, qsh[p], row[p]);
-                s4[p & 3] = fmaf(row[p], row[p], s4[p & 3]);
+            for (int j = 0; j < E; j += 2) {
+                const float4 y = *reinterpret_cast<const float4 *>(qsh + ln * QS + 2 * j);
+                q[j] = f2_pack(y.x, y.y);
+                q[j + 1] = f2_pack(y.z, y.w);
             }
-            nrm = (s4[0] + s4[1]) + (s4[2] + s4[3]);
-            drow[r] = dot;
-            bv = nrm;
-            bi = tid;
+#pragma unroll
+            for (int s = 0; s < NS; s++) {
+                if (w0 + PAIRS * s >= m) continue;
+                F2 d2 = f2_pack(0.f, 0.f), zz = d2;
+#pragma unroll
+                for (int j = 0; j < E; j++) d2 = f2_fma(q[j], row[s][j], d2);
+                float dot = f2_sum(d2);
+                dot += __shfl_xor_sync(0xffffffffu, dot, 1);
+                const F2 nd = f2_pack(-dot, -dot);
+#pragma unroll
+                for (int j = 0; j < E; j++) {
+                    row[s][j] = f2_fma(nd, q[j], row[s][j]);
+                    zz = f2_fma(row[s][j], row[s][j], zz);
+                }
+                float z = f2_sum(zz);
+                z += __shfl_xor_sync(0xffffffffu, z, 1);
+                if (pos[s] == -1) {
+                    nrm[s] = z;
+                    if (ln == 0) dots[(a0 + PAIRS * s) * ID2_DSTRIDE + r] = dot;
+                    if (z > bv) { bv = z; bi = a0 + PAIRS * s; }
+                }
+            }
         }
         if (xpos == -1) {
             float dot = 0.f;
-            for (int p = 0; p < P; p++) dot = fmaf(qsh[p], xr[p], dot);
+            for (int p = 0; p < P; p++) dot = fmaf(qsh[((p >> 1) & 1) * QS + 2 * (p >> 2) + (p & 1)], xr[p], dot);
             float s2 = 0.f;
             for (int p = 0; p < P; p++) {
-                const float y = fmaf(-dot, qsh[p], xr[p]);
+                const float y = fmaf(-dot, qsh[((p >> 1) & 1) * QS + 2 * (p >> 2) + (p & 1)], xr[p]);
                 xr[p] = y;
                 s2 = fmaf(y, y, s2);
             }
             xnrm = s2;
-            U[(size_t)(THREADS + tid) * MAXR + r] = dot;
-            if (s2 > bv) { bv = s2; bi = THREADS + tid; }
+            U[(size_t)(HELD + tid) * MAXR + r] = dot;
+            if (s2 > bv) { bv = s2; bi = HELD + tid; }
         }
         warp_argmax(bv, bi);
         buf ^= 1;
@@ -1562,16 +1632,16 @@ k_id2d(int n_item, const int *__restrict__ items, IdArgs g, DepArgs dp)
     }
     __syncthreads();
     // skeleton and rank; R11 from the pivot rows' dot products (column jj: its entries k < jj)
-    if (pos >= 0) skel[(size_t)t * MAXR + pos] = sxy[tid];
-    if (xpos >= 0) skel[(size_t)t * MAXR + xpos] = sxy[THREADS + tid];
+#pragma unroll
+    for (int s = 0; s < NS; s++)
+        if (ln == 0 && pos[s] >= 0) skel[(size_t)t * MAXR + pos[s]] = sxy[a0 + PAIRS * s];
+    if (xpos >= 0) skel[(size_t)t * MAXR + xpos] = sxy[HELD + tid];
     if (tid == 0) g.rank[t] = r;
-    for (int idx = tid; idx < r * r; idx += THREADS) {
-        const int jj = idx / r, k = idx % r;
-        if (k > jj) continue;
+    for (int jj = wid; jj < r; jj += NW) {
         const int pr = piv[jj];
-        R11[jj * (jj + 1) / 2 + k] = k == jj ? rdiag[jj]
-                                             : (pr < THREADS ? dots[(size_t)pr * ID2_DSTRIDE + k]
-                                                                 : U[(size_t)pr * MAXR + k]);
+        for (int k = lane; k <= jj; k += 32)
+            R11[jj * (jj + 1) / 2 + k] = k == jj ? rdiag[jj]
+                                                 : (pr < HELD ? dots[pr * ID2_DSTRIDE + k] : U[(size_t)pr * MAXR + k]);
     }
     __syncthreads();
     // the skeleton and the rank are what the parent's decomposition needs: published here;
@@ -1580,55 +1650,81 @@ k_id2d(int n_item, const int *__restrict__ items, IdArgs g, DepArgs dp)
         if (tid == 0) dep_publish(dp, t);
         if (tid < nch && !tv.leaf[cfirst + tid]) dep_wait_y0(dp, cfirst + tid);
         __syncthreads();
-        for (int q = 0; q < 2; q++) {
-            const int a = tid + THREADS * q;
-            if (a >= m) break;
+        for (int a = tid; a < m; a += THREADS) {
             int c = 0, aa = a;
             while (aa >= s_crank[c]) { aa -= s_crank[c]; c++; }
             sin_[a] = __ldcg(g.y0 + (size_t)(cfirst + c) * MAXR + aa);
         }
     }
-    // back substitution of the non-pivot rows, column by column (independent updates)
-    if (pos == -1) {
-        for (int k = r - 1; k >= 0; k--) {
-            const float *col = R11 + k * (k + 1) / 2;
-            const float uk = drow[k] / col[k];
-            drow[k] = uk;
-            for (int i = 0; i < k; i++) drow[i] = fmaf(-col[i], uk, drow[i]);
+    // back substitution of the open rows: columns top, top - 1 by the first lane, top - 2, top - 3 by
+    // the second, each column taking the later columns k in decreasing order, then its division
+#pragma unroll
+    for (int s = 0; s < NS; s++) {
+        if (w0 + PAIRS * s >= m) continue;
+        float *u = dots + (a0 + PAIRS * s) * ID2_DSTRIDE;
+        const bool open = pos[s] == -1;
+        for (int top = r - 1; top >= 0; top -= 4) {
+            const int ca = max(top - 2 * ln, 0), cb = max(top - 2 * ln - 1, 0);
+            float acc0 = u[ca], acc1 = u[cb];
+            const float *col = R11 + (r - 1) * r / 2;   // column r - 1; column k - 1 lies k before column k
+            for (int k = r - 1; k > top; col -= k, k--) {
+                const float uk = u[k];
+                acc0 = fmaf(-col[ca], uk, acc0);
+                acc1 = fmaf(-col[cb], uk, acc1);
+            }
+#pragma unroll
+            for (int z = 0; z < 4; z++) {
+                if (top - z < 0) break;
+                const float *cz = R11 + (top - z) * (top - z + 1) / 2;
+                const float uk = __shfl_sync(0xffffffffu, ((z & 1) ? acc1 : acc0) / cz[top - z], z >> 1, 2);
+                if (ln == z >> 1 && open) u[top - z] = uk;
+                if (2 * ln > z) acc0 = fmaf(-cz[ca], uk, acc0);
+                if (2 * ln + 1 > z) acc1 = fmaf(-cz[cb], uk, acc1);
+            }
+            __syncwarp();
         }
+        if (pos[s] >= 0)   // pivot rows are rows of the identity
+            for (int k = ln; k < r; k += 2) u[k] = k == pos[s] ? 1.f : 0.f;
     }
     if (xpos == -1) {
-        float *u = U + (size_t)(THREADS + tid) * MAXR;
+        float *u = U + (size_t)(HELD + tid) * MAXR;
         for (int k = r - 1; k >= 0; k--) {
             float acc = u[k];
             for (int jj = k + 1; jj < r; jj++) acc = fmaf(-R11[jj * (jj + 1) / 2 + k], u[jj], acc);
             u[k] = acc / R11[k * (k + 1) / 2 + k];
         }
     }
-    __syncthreads();
-    // pivot rows are rows of the identity
-    if (pos >= 0)
-        for (int k = 0; k < r; k++) drow[k] = k == pos ? 1.f : 0.f;
     if (xpos >= 0)
-        for (int k = 0; k < r; k++) U[(size_t)(THREADS + tid) * MAXR + k] = k == xpos ? 1.f : 0.f;
+        for (int k = 0; k < r; k++) U[(size_t)(HELD + tid) * MAXR + k] = k == xpos ? 1.f : 0.f;
     __syncthreads();
-    // U rows 0 .. min(m, THREADS) - 1 out of shared memory (over the overflow rows' scratch)
-    const int mm = min(m, THREADS);
-    for (int idx = tid; idx < mm * r; idx += THREADS) {
-        const int a = idx / r, k = idx % r;
-        U[(size_t)a * MAXR + k] = dots[(size_t)a * ID2_DSTRIDE + k];
-    }
-    // y0[k] = sum_a U[a][k] in[a]: groups of RG threads over k, C = THREADS / RG groups over a
-    const int RG = r <= 16 ? 16 : (r <= 32 ? 32 : 64);
-    const int C = THREADS / RG, kk = tid % RG, cg = tid / RG;
-    float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (kk < r) {
-        for (int a = cg; a < m; a += C) {
-            const float w = a < THREADS ? dots[(size_t)a * ID2_DSTRIDE + kk] : U[(size_t)a * MAXR + kk];
-            fma4(acc, w, sin_[a]);
+    // U rows 0 .. min(m, HELD) - 1 out of shared memory (over the overflow rows' scratch)
+#pragma unroll
+    for (int s = 0; s < NS; s++) {
+        const int a = a0 + PAIRS * s;
+        if (a >= m) continue;
+        const float *u = dots + a * ID2_DSTRIDE;
+        float *o = U + (size_t)a * MAXR;
+        for (int k = 4 * ln; k < r; k += 8) {
+            if (k + 3 < r) *reinterpret_cast<float4 *>(o + k) = make_float4(u[k], u[k + 1], u[k + 2], u[k + 3]);
+            else
+                for (int z = k; z < r; z++) o[z] = u[z];
         }
     }
-    part[tid] = acc;
+    // y0[k] = sum_a U[a][k] in[a]: groups of RG threads over k, C = yt / RG groups over a
+    const int yt = LEAVES && m <= ID2_SMALL ? 64 : 128;
+    const int RG = r <= 16 ? 16 : (r <= 32 ? 32 : 64);
+    const int C = yt / RG, kk = tid & (RG - 1), cg = tid / RG;
+    static_assert(THREADS >= (LEAVES && HELD <= ID2_SMALL ? 64 : 128), "a thread per part");
+    if (tid < yt) {
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (kk < r) {
+            for (int a = cg; a < m; a += C) {
+                const float w = a < HELD ? dots[a * ID2_DSTRIDE + kk] : U[(size_t)a * MAXR + kk];
+                fma4(acc, w, sin_[a]);
+            }
+        }
+        part[tid] = acc;
+    }
     __syncthreads();
     if (tid < r) {
         float4 y = part[tid];
@@ -1689,7 +1785,7 @@ constexpr int ID3_SMALL = 64;                // leaves of the 256-thread CTAs
 constexpr int ID3_MID = 128;                 // leaves whose rows a 512-thread CTA holds in registers
 constexpr int ID3_HELD = 28;                 // most pairs per lane
 constexpr int ID3_VP = 400;                  // the residual in the lanes' order (id3_place)
-static_assert(ID3_TINY == ID3_TINY_LEAF && ID3_SMALL == ID3_SMALL_LEAF, "the leaf lists are the launches'");
+static_assert(ID3_TINY == TINY_LEAF && ID3_SMALL == SMALL_LEAF, "the leaf lists are the launches'");
 static_assert(ID3_P % 8 == 0 && ID3_QS >= ID3_P && ID3_QS % 4 == 0, "proxy pairs, 16-byte rows");
 
 template <int THREADS, int ROWS>
@@ -1762,12 +1858,6 @@ __device__ __forceinline__ F2 id3_v(const float *v, int j)
 {
     const float2 x = *reinterpret_cast<const float2 *>(v + 2 * j);
     return f2_pack(x.x, x.y);
-}
-__device__ __forceinline__ float f2_sum(F2 a)
-{
-    float a0, a1;
-    f2_unpack(a, a0, a1);
-    return a0 + a1;
 }
 
 // The lane's part of a row in registers. S >= 4: a lane per chain, lane q holds the pairs q + S i.
@@ -2811,12 +2901,12 @@ public:
                                              (int)id_smem_bytes<D>(id_mcap())));
         TSNE_CUDA_CHECK(cudaFuncSetAttribute(k_id<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)id_smem_bytes<D>(id_mcap())));
-        TSNE_CUDA_CHECK(cudaFuncSetAttribute(k_id2d<true, ID2_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)id2_smem(ID2_SMALL)));
-        TSNE_CUDA_CHECK(cudaFuncSetAttribute(k_id2d<true, ID2_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)id2_smem(ID2_THREADS)));
-        TSNE_CUDA_CHECK(cudaFuncSetAttribute(k_id2d<false, ID2_THREADS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                             (int)id2_smem(ID2_THREADS)));
+        if (D == 2) {
+            id2_attr<true, 64, 1>();
+            id2_attr<true, 128, 1>();
+            id2_attr<true, 128, 2>();
+            id2_attr<false, 128, 2>();
+        }
         if (D == 3) {
             id3_attr<false, 512, ID3_ROWS>();
             id3_attr<true, 512, ID3_ROWS>();
@@ -2959,14 +3049,21 @@ public:
         IdArgs il{view(), xt_.p, skel_.p, rank_.p, rowoff_.p, U_.p, gA_.p, gnrm_.p, gsel_.p, gcand_.p, mleaf, tol2,
                   y0_.p};
         const int first = I.level_begin[MIN_ADM_LEVEL];
-        if (D == 2 && stats_.max_leaf <= ID2_THREADS) {
+        if (D == 2 && stats_.max_leaf <= ID2_HELD) {
             // leaves in one launch, then the internal nodes of every level in one
             // dependency-ordered launch
             DepArgs dp{flag_.p, tickets_.p + TICKET_BASES, &info_.p->pad[1], ++epoch_};
-            if (hleaf_ > 0)
-                k_id2d<true, ID2_SMALL><<<hleaf_, ID2_SMALL, id2_smem(ID2_SMALL), st_>>>(hleaf_, llist_.p, il, dp);
-            if (hbig_ > 0)
-                k_id2d<true, ID2_THREADS><<<hbig_, ID2_THREADS, id2_smem(ID2_THREADS), st_>>>(hbig_, blist_.p, il, dp);
+            // few leaves: one launch of the CTAs that take any size, so that all run at once;
+            // more than fill the GPU: by size, so that small leaves do not take large CTAs
+            const int *none = nullptr;
+            if (hleaf_ + hbig_ + hlarge_ <= ID2_ONE_LAUNCH) {
+                const LeafItems all{{clist_.p, blist_.p, llist_.p}, {hlarge_, hbig_, hleaf_}};
+                if (hleaf_ + hbig_ + hlarge_ > 0) id2_launch<true, 128, 2>(hleaf_ + hbig_ + hlarge_, none, all, il, dp);
+            } else {
+                if (hlarge_ > 0) id2_launch<true, 128, 2>(hlarge_, none, {{clist_.p, none, none}, {hlarge_, 0, 0}}, il, dp);
+                if (hbig_ > 0) id2_launch<true, 128, 1>(hbig_, none, {{blist_.p, none, none}, {hbig_, 0, 0}}, il, dp);
+                if (hleaf_ > 0) id2_launch<true, 64, 1>(hleaf_, none, {{llist_.p, none, none}, {hleaf_, 0, 0}}, il, dp);
+            }
             mark_end(t_bases, 2);
             t_bases = mark_begin();
             near_fork_point();
@@ -2975,16 +3072,13 @@ public:
                 for (int l = max_level_; l >= MIN_ADM_LEVEL; l--) {
                     const int nl = I.n_level_nodes[l];
                     if (nl <= 0) continue;
-                    k_id2d<false, ID2_THREADS><<<nl, ID2_THREADS, id2_smem(ID2_THREADS), st_>>>(
-                        I.level_begin[l], nullptr, il, dp);
-                    launches_++;
+                    id2_launch<false, 128, 2>(I.level_begin[l], nullptr, LeafItems{}, il, dp, nl);
                 }
             } else if (hint_ > 0) {
                 DepArgs d2 = dp;
                 d2.flag2 = flag2_.p;
-                k_id2d<false, ID2_THREADS><<<hint_, ID2_THREADS, id2_smem(ID2_THREADS), st_>>>(hint_, ilist_.p, il, d2);
+                id2_launch<false, 128, 2>(hint_, ilist_.p, LeafItems{}, il, d2);
             }
-            launches_ += 2;
             near_launch_side();
             mark_end(t_bases, 7);
             if (timing_) TSNE_CUDA_CHECK(cudaStreamSynchronize(st_));
@@ -3071,7 +3165,7 @@ public:
         nset_cnt_.exact(c + 1);
         far_cnt_.exact(c + 1); near_cnt_.exact(c + 1); fine_cnt_.exact(c + 1);
         far_ptr_.exact(c + 2); near_ptr_.exact(c + 2);
-        ilist_.exact(c + 1); llist_.exact(c + 1); blist_.exact(c + 1); clist_.exact(D == 3 ? c + 1 : 1); flist_.exact(c + 1);
+        ilist_.exact(c + 1); llist_.exact(c + 1); blist_.exact(c + 1); clist_.exact(c + 1); flist_.exact(c + 1);
         rowoff_.exact(c + 2);
         rank_.exact(c);
         node_blk_.exact(ceil_div(c, NODE_BLOCK));
@@ -3274,6 +3368,20 @@ private:
         marks_.push_back({a, b, phase});
     }
 
+    template <bool LEAVES, int THREADS, int NS>
+    static void id2_attr()
+    {
+        TSNE_CUDA_CHECK(cudaFuncSetAttribute(k_id2d<LEAVES, THREADS, NS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)id2_smem<THREADS, NS>()));
+    }
+    template <bool LEAVES, int THREADS, int NS>
+    void id2_launch(int n_item, const int *items, const LeafItems &leaves, const IdArgs &a, const DepArgs &dp,
+                    int ctas = 0)
+    {
+        k_id2d<LEAVES, THREADS, NS><<<ctas > 0 ? ctas : n_item, THREADS, id2_smem<THREADS, NS>(), st_>>>(n_item, items,
+                                                                                                         leaves, a, dp);
+        launches_++;
+    }
     template <bool LEAVES, int THREADS, int ROWS>
     static void id3_attr()
     {
@@ -3484,7 +3592,7 @@ private:
     DevBuf<int> far_alt_, near_alt_;   // segmented-sort partners of the 3D lists
     DevBuf<NodeSums> node_blk_;          // block sums of the node scan
     DevBuf<int> ilist_;                  // internal nodes at level >= 2, in increasing id
-    DevBuf<int> llist_;                  // leaves at level >= 2 of at most LEAF_SMALL points
+    DevBuf<int> llist_;                  // leaves at level >= 2 of at most TINY_LEAF points
     DevBuf<int> blist_, clist_;          // the larger leaves at level >= 2
     DevBuf<int> flist_, fine_cnt_;       // leaves with finer far entries, and how many each node has
     int hint_ = 0, hleaf_ = 0, hbig_ = 0, hlarge_ = 0, hfine_ = 0;
