@@ -31,14 +31,21 @@ __device__ __forceinline__ Vec<D> vzero()
     return v;
 }
 
-// Streamed P entries: read once per pass, kept out of L1 so Y stays cached.
+// Streamed P entries: read once per pass, not allocated in L1, which is left to the gathers of Y
+// (with evict-first loads the window form took 0.528 ms at 1M points instead of 0.511).
 __device__ __forceinline__ int4 ld_stream_i4(const int *p)
 {
-    return __ldcs(reinterpret_cast<const int4 *>(p));
+    int4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
 }
 __device__ __forceinline__ float4 ld_stream_f4(const float *p)
 {
-    return __ldcs(reinterpret_cast<const float4 *>(p));
+    float4 v;
+    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
 }
 
 template <int D>
@@ -136,6 +143,11 @@ constexpr int ATTR_PIPE_MINB = 5;
 constexpr int ATTR_PIPE_GRID = 148 * ATTR_PIPE_MINB;
 constexpr int ATTR_PIPE3_MINB = 6;
 constexpr int ATTR_PIPE3_GRID = 148 * ATTR_PIPE3_MINB;
+// The table of row ranges (k_attr_ranges) is as fine as form 3's grid; the window form's CTAs take
+// ATTR_RANGES_PER_SM of them each.
+constexpr int ATTR_RANGES = ATTR_PIPE3_GRID;
+constexpr int ATTR_RANGES_PER_SM = ATTR_PIPE3_MINB;
+static_assert(ATTR_RANGES + 1 == ATTR_RANGE_TABLE, "the table the workspace holds");
 
 // PF (TSNE_ATTR_PIPE=1): each lane loads its next step's 4 entries of the row before the
 // gathers of the current step; PF = 2 (TSNE_ATTR_PIPE=3): only the next step's 4 columns
@@ -146,7 +158,8 @@ __device__ __forceinline__ void
 attr_update_rows(int n, const int *__restrict__ rp, const int *__restrict__ col, const float *__restrict__ val,
                  const Vec<D> *__restrict__ Y, Vec<D> *__restrict__ Yn, Vec<D> *__restrict__ uY,
                  Vec<D> *__restrict__ gains, const Vec<D> *__restrict__ rep, const int *__restrict__ rep_flag,
-                 float exag4, float mom, float lr, double *__restrict__ partials, Vec<D> *__restrict__ attr)
+                 float exag4, float mom, float lr, double *__restrict__ partials, Vec<D> *__restrict__ attr,
+                 const int *__restrict__ ranges)
 {
     const int lane = threadIdx.x & 31, hl = lane & 15;
     const int half = (blockIdx.x * ROW_BLOCK + threadIdx.x) >> 4;
@@ -159,7 +172,11 @@ attr_update_rows(int n, const int *__restrict__ rp, const int *__restrict__ col,
     // over them, so that one SM's gathers come from one neighbourhood of the tree order
     __shared__ int s_rng[2];
     int r0 = 0, r1 = n, rounds;
-    if constexpr (CONTIG) {
+    if constexpr (CONTIG && PF == 2) {   // (the grid is the table's)
+        r0 = ranges[blockIdx.x];
+        r1 = ranges[blockIdx.x + 1];
+        rounds = (r1 - r0 + (ROW_BLOCK >> 4) - 1) / (ROW_BLOCK >> 4);
+    } else if constexpr (CONTIG) {
         if (threadIdx.x < 2) {
             const int c = blockIdx.x + threadIdx.x;
             int lo = 0;
@@ -310,17 +327,18 @@ k_attr_update(int n, const int *__restrict__ rp, const int *__restrict__ col, co
               float exag4, float mom, float lr, double *__restrict__ partials, Vec<D> *__restrict__ attr)
 {
     attr_update_rows<D, MODE, CONTIG, 0>(n, rp, col, val, Y, Yn, uY, gains, rep, rep_flag, exag4, mom, lr,
-                                         partials, attr);
+                                         partials, attr, nullptr);
 }
 template <int D, int MODE, bool CONTIG, int PF>
 __global__ void __launch_bounds__(ROW_BLOCK, PF == 1 ? ATTR_PIPE_MINB : ATTR_PIPE3_MINB)
 k_attr_update_pf(int n, const int *__restrict__ rp, const int *__restrict__ col, const float *__restrict__ val,
                  const Vec<D> *__restrict__ Y, Vec<D> *__restrict__ Yn, Vec<D> *__restrict__ uY,
                  Vec<D> *__restrict__ gains, const Vec<D> *__restrict__ rep, const int *__restrict__ rep_flag,
-                 float exag4, float mom, float lr, double *__restrict__ partials, Vec<D> *__restrict__ attr)
+                 float exag4, float mom, float lr, double *__restrict__ partials, Vec<D> *__restrict__ attr,
+                 const int *__restrict__ ranges)
 {
     attr_update_rows<D, MODE, CONTIG, PF>(n, rp, col, val, Y, Yn, uY, gains, rep, rep_flag, exag4, mom, lr,
-                                          partials, attr);
+                                          partials, attr, ranges);
 }
 
 // The update of a rebuild iteration from its stored attractive sums, for the forms with more
@@ -675,152 +693,198 @@ k_attr_pair(int n, const int *__restrict__ rp, const int *__restrict__ col, cons
     block_sum_warps<D>(acc, partials + (size_t)blockIdx.x * D);
 }
 
-// The same step with the Y gathers served from shared memory (TSNE_ATTR_WINDOW=1 or 2; off by
-// default). One CTA per SM (form 2: two) owns a contiguous range of rows holding an equal
-// share of P's entries and stages the window of Y centred on it (WINP points: 128 KB, form 2
-// 64 KB) once; a column
-// inside the window is read from shared memory, one outside it through L1/L2. After the
-// renumbering in tree order about three quarters of a point's neighbours lie inside a
-// 16K-point window around it (200K-point 2D embedding of the benchmark mixture), so most
-// gathers skip the L1 tag stage that bounds k_attr_update. Measured at 1M points, 2D: 0.651 ms
-// per launch against k_attr_update's 0.636 ms, so not faster (it keeps 32 warps per SM
-// resident instead of 64, and about a quarter of the gathers still go to L1/L2), hence off by
-// default. Splitting rows by equal counts instead of equal entries made it 1.25 ms: row
-// lengths follow the tree order's clusters. Used while the average CTA's row range fits in
-// half a window (n <= 148 * win_pts / 2). The row of each half-warp and the summation order
-// are fixed, so results are bit-reproducible, and the three modes give the same bits as one
-// another.
+// The step with the Y gathers served from shared memory: one CTA of 1,024 threads per SM takes a
+// contiguous range of rows holding an equal share of P's entries and stages the window of Y
+// centred on it (WIN points, 96 KB), which holds many of the neighbours once the points are
+// renumbered in tree order. A column inside the window is read from shared memory, one outside
+// it through L1/L2, by a predicated load each. What bounds the forms without a window is the
+// L1's tag stage: a gather of 32 lanes looks up 32 lines, one per cycle, and the launch takes
+// one cycle per entry and SM (1.19 M entries per SM: 0.68 ms at 1M points). The window takes the
+// lookups of the neighbours inside it away (about half of them at 1M points, three quarters at
+// 200K, all up to WIN points); what is left is those outside, and shared-memory bank conflicts.
+// So that 64 half-warps per SM keep enough entries in flight, the columns and values of a half-
+// warp's next step are loaded before the current gathers, across rows too (the next row's
+// pointers and Y when a row starts, its first entries in the row's last step), and a CTA's row
+// range comes from a table. Rows are dealt to half-warps and summed over lanes as in
+// k_attr_update (same bits per row).
+// Per launch, form 3 -> this one: 1M points 0.679 -> 0.511 ms, 200K 0.134 -> 0.106, 300K in the
+// exaggeration phase 0.196 -> 0.156, 20K 26.7 -> 20.8 us, 2K 14.3 -> 10.3 us, 100K 3D 96.8 ->
+// 87.6 us. The window's size at 1M (before the P loads passed by L1): 64 KB 0.548 ms, 96 KB
+// 0.528, 128 KB 0.555, 160 KB 0.611, 224 KB 1.259: what the window takes is missing in L1 for
+// the lines in flight of the gathers outside it.
 constexpr int WIN_THREADS = 1024;
 constexpr int WIN_GRID = 148;
-template <int D> constexpr int win_pts() { return D == 2 ? 16384 : 8192; }
+template <int D> constexpr int win_pts() { return D == 2 ? 12288 : 6144; }
 
-// first row i in [0, n] with rp[i] >= x (rp non-decreasing, rp[0] = 0)
-__device__ __forceinline__ int first_row_at(const int *__restrict__ rp, int n, long long x)
+// Y[c] from the window (byte address win, first point w0, wl points) or from global memory
+template <int D>
+__device__ __forceinline__ Vec<D> win_gather(unsigned win, int w0, int wl, const Vec<D> *Y, int c)
 {
-    int lo = 0, hi = n;
-    while (lo < hi) {
-        const int mid = (lo + hi) >> 1;
-        if ((long long)rp[mid] < x) lo = mid + 1;
-        else hi = mid;
-    }
-    return lo;
+    const unsigned off = (unsigned)(c - w0), sa = win + off * (unsigned)sizeof(Vec<D>);
+    Vec<D> v;
+    if constexpr (D == 2)
+        asm volatile("{ .reg .pred p; setp.lt.u32 p, %2, %3;\n"
+                     "@p ld.shared.v2.f32 {%0, %1}, [%4];\n"
+                     "@!p ld.global.nc.v2.f32 {%0, %1}, [%5]; }"
+                     : "=f"(v.x), "=f"(v.y) : "r"(off), "r"(wl), "r"(sa), "l"(Y + c));
+    else
+        asm volatile("{ .reg .pred p; setp.lt.u32 p, %4, %5;\n"
+                     "@p ld.shared.v4.f32 {%0, %1, %2, %3}, [%6];\n"
+                     "@!p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%7]; }"
+                     : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(off), "r"(wl), "r"(sa), "l"(Y + c));
+    return v;
+}
+template <int D>
+__device__ __forceinline__ void attr_acc_y(const Vec<D> &yi, const Vec<D> &yj, float p, float (&a)[D])
+{
+    float df[D], r2 = 0.f;
+#pragma unroll
+    for (int k = 0; k < D; k++) { df[k] = vget(yi, k) - vget(yj, k); r2 = fmaf(df[k], df[k], r2); }
+    const float q = p * fast_rcp(1.0f + r2);
+#pragma unroll
+    for (int k = 0; k < D; k++) a[k] = fmaf(q, df[k], a[k]);
 }
 
-template <int D, int MODE, int WINP, int MINB>
-__global__ void __launch_bounds__(WIN_THREADS, MINB)
-k_attr_window(int n, const int *__restrict__ rp, const int *__restrict__ col, const float *__restrict__ val,
-              const Vec<D> *__restrict__ Y, Vec<D> *__restrict__ Yn, Vec<D> *__restrict__ uY,
-              Vec<D> *__restrict__ gains, const Vec<D> *__restrict__ rep, const int *__restrict__ rep_flag,
-              float exag4, float mom, float lr, double *__restrict__ partials, Vec<D> *__restrict__ attr)
+template <int D, int MODE>
+__global__ void __launch_bounds__(WIN_THREADS, 1)
+k_attr_window(int n, const int *__restrict__ ranges, const int *__restrict__ rp, const int *__restrict__ col,
+              const float *__restrict__ val, const Vec<D> *__restrict__ Y, Vec<D> *__restrict__ Yn,
+              Vec<D> *__restrict__ uY, Vec<D> *__restrict__ gains, const Vec<D> *__restrict__ rep,
+              const int *__restrict__ rep_flag, float exag4, float mom, float lr, double *__restrict__ partials,
+              Vec<D> *__restrict__ attr)
 {
-    constexpr int WIN = WINP;
-    constexpr int NH = WIN_THREADS / 16;   // half-warps per CTA
+    static_assert(MODE != ATTR_UPDATE, "the update of a rebuild iteration is k_update_rows");
+    constexpr int WIN = win_pts<D>();
+    constexpr int NHC = WIN_THREADS >> 4;   // half-warps per CTA
     extern __shared__ __align__(16) unsigned char win_raw[];
-    Vec<D> *win = reinterpret_cast<Vec<D> *>(win_raw);
-    const int lane = threadIdx.x & 31, hl = lane & 15, hw = threadIdx.x >> 4;
-    // CTA b takes the rows whose entries start in [b nnz / G, (b + 1) nnz / G): equal shares of
-    // P, since row lengths follow the clusters of the tree order and equal row counts would not
-    // balance; the last CTA also takes the empty rows at the end
-    const long long nnz = rp[n];
-    const int rb = first_row_at(rp, n, (long long)blockIdx.x * nnz / gridDim.x);
-    const int re = blockIdx.x + 1 == gridDim.x ? n : first_row_at(rp, n, (long long)(blockIdx.x + 1) * nnz / gridDim.x);
-    int w0 = rb + (re - rb) / 2 - WIN / 2;
-    w0 = max(0, min(w0, n - WIN));
+    const int lane = threadIdx.x & 31, hl = lane & 15;
+    const int r0 = ranges[blockIdx.x * ATTR_RANGES_PER_SM], r1 = ranges[(blockIdx.x + 1) * ATTR_RANGES_PER_SM];
+    int w0 = (r0 + (r1 - r0) / 2 - WIN / 2) & ~1;   // an even point: 16-byte copies
+    w0 = max(0, min(w0, (n - WIN + 1) & ~1));
     const int wl = min(WIN, n - w0);
-    if (MODE != ATTR_UPDATE) {
-        for (int k = threadIdx.x; k < wl; k += WIN_THREADS) win[k] = Y[w0 + k];
-        __syncthreads();
+    {
+        const float4 *src = reinterpret_cast<const float4 *>(Y + w0);
+        float4 *dst = reinterpret_cast<float4 *>(win_raw);
+        constexpr int PER = 16 / (int)sizeof(Vec<D>);   // points per copy
+        for (int k = threadIdx.x; k < wl / PER; k += WIN_THREADS) dst[k] = src[k];
+        if (PER == 2 && (wl & 1) && threadIdx.x == 0) reinterpret_cast<Vec<D> *>(win_raw)[wl - 1] = Y[w0 + wl - 1];
     }
+    const unsigned win = (unsigned)__cvta_generic_to_shared(win_raw);
     const int use_rep = (MODE != ATTR_GRAD && rep != nullptr) ? *rep_flag : 0;
     double acc[D];
     for (int k = 0; k < D; k++) acc[k] = 0.0;
-    // every half-warp of the CTA runs the same number of rounds (full-warp shuffles)
-    const int rounds = (re - rb + NH - 1) / NH;
+    const int rounds = (r1 - r0 + NHC - 1) / NHC;   // the same for the half-warps of a warp
+    // the current row (i) and its first entries
+    int i = r0 + ((int)threadIdx.x >> 4);
+    Vec<D> yi = vzero<D>();
+    int b = 0, e = 0;
+    if (i < r1) { yi = Y[i]; b = rp[i]; e = rp[i + 1]; }
+    int4 c4 = make_int4(0, 0, 0, 0);
+    float4 p4 = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (b + 4 * hl < e) { c4 = ld_stream_i4(col + b + 4 * hl); p4 = ld_stream_f4(val + b + 4 * hl); }
+    __syncthreads();
     for (int rd = 0; rd < rounds; rd++) {
-        const int i = rb + rd * NH + hw;
-        const bool live = i < re;
-        Vec<D> yi = vzero<D>(), opnd = vzero<D>();
-        int b = 0, e = 0;
-        if (live) {
-            yi = Y[i];
-            b = rp[i];
-            e = rp[i + 1];
-            if (MODE != ATTR_GRAD) {
-                if (hl == 1) opnd = uY[i];
-                else if (hl == 2) opnd = gains[i];
-                else if (hl == 3 && use_rep) opnd = rep[i];
-            }
+        const bool live = i < r1;
+        const int i_n = i + NHC;
+        Vec<D> yi_n = vzero<D>(), opnd = vzero<D>();
+        int nb = 0, ne = 0;
+        if (i_n < r1) { yi_n = Y[i_n]; nb = rp[i_n]; ne = rp[i_n + 1]; }
+        if (MODE != ATTR_GRAD && live) {
+            if (hl == 1) opnd = uY[i];
+            else if (hl == 2) opnd = gains[i];
+            else if (hl == 3 && use_rep) opnd = rep[i];
         }
         float a[D];
 #pragma unroll
         for (int k = 0; k < D; k++) a[k] = 0.f;
-        if (MODE == ATTR_UPDATE) {
-            if (live && hl == 0) {
-                const Vec<D> s = attr[i];
-#pragma unroll
-                for (int k = 0; k < D; k++) a[k] = vget(s, k);
+        int base = b + 4 * hl;
+        const int last = max(b, e - 1) - (max(b, e - 1) - b) % 64 + 4 * hl;   // this lane's place in the row's last step
+        for (;; base += 64) {
+            const bool on = base < e, fin = base >= last;
+            const int na = fin ? nb + 4 * hl : base + 64, nae = fin ? ne : e;
+            int4 cn = make_int4(0, 0, 0, 0);
+            float4 pn = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (na < nae) { cn = ld_stream_i4(col + na); pn = ld_stream_f4(val + na); }
+            if (on) {
+                const Vec<D> y0 = win_gather<D>(win, w0, wl, Y, c4.x), y1 = win_gather<D>(win, w0, wl, Y, c4.y);
+                const Vec<D> y2 = win_gather<D>(win, w0, wl, Y, c4.z), y3 = win_gather<D>(win, w0, wl, Y, c4.w);
+                attr_acc_y<D>(yi, y0, p4.x, a);
+                attr_acc_y<D>(yi, y1, p4.y, a);
+                attr_acc_y<D>(yi, y2, p4.z, a);
+                attr_acc_y<D>(yi, y3, p4.w, a);
             }
-        } else {
-            for (int base = b + 4 * hl; base < e; base += 64) {
-                const int4 c4 = ld_stream_i4(col + base);
-                const float4 p4 = ld_stream_f4(val + base);
-                const int cs[4] = {c4.x, c4.y, c4.z, c4.w};
-                const float ps[4] = {p4.x, p4.y, p4.z, p4.w};
-#pragma unroll
-                for (int q = 0; q < 4; q++) {
-                    const unsigned int off = (unsigned int)(cs[q] - w0);
-                    const Vec<D> yj = off < (unsigned int)wl ? win[off] : __ldg(Y + cs[q]);
-                    float df[D], r2 = 0.f;
-#pragma unroll
-                    for (int k = 0; k < D; k++) { df[k] = vget(yi, k) - vget(yj, k); r2 = fmaf(df[k], df[k], r2); }
-                    const float w = ps[q] * fast_rcp(1.0f + r2);
-#pragma unroll
-                    for (int k = 0; k < D; k++) a[k] = fmaf(w, df[k], a[k]);
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < D; k++)
-                for (int o = 8; o > 0; o >>= 1) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
+            c4 = cn;
+            p4 = pn;
+            if (fin) break;
         }
+        __syncwarp();
+#pragma unroll
+        for (int k = 0; k < D; k++)
+            for (int o = 8; o > 0; o >>= 1) a[k] += __shfl_xor_sync(0xffffffffu, a[k], o);
         if (MODE == ATTR_GRAD) {
             if (live && hl == 0) {
-                Vec<D> s = vzero<D>();
+                Vec<D> v = vzero<D>();
 #pragma unroll
-                for (int k = 0; k < D; k++) vset(s, k, a[k]);
-                attr[i] = s;
+                for (int k = 0; k < D; k++) vset(v, k, a[k]);
+                attr[i] = v;
             }
-            continue;
-        }
-        const int src = lane & 16;
-        Vec<D> u = vzero<D>(), g = vzero<D>(), r = vzero<D>();
-#pragma unroll
-        for (int k = 0; k < D; k++) {
-            vset(u, k, __shfl_sync(0xffffffffu, vget(opnd, k), src + 1));
-            vset(g, k, __shfl_sync(0xffffffffu, vget(opnd, k), src + 2));
-            vset(r, k, __shfl_sync(0xffffffffu, vget(opnd, k), src + 3));
-        }
-        if (live && hl == 0) {
-            Vec<D> yn = yi;
+        } else {
+            const int src = lane & 16;
+            Vec<D> u = vzero<D>(), g = vzero<D>(), r = vzero<D>();
 #pragma unroll
             for (int k = 0; k < D; k++) {
-                const float gk = exag4 * a[k] - vget(r, k);
-                const float uk = vget(u, k);
-                float gain = (uk * gk < 0.f) ? vget(g, k) + 0.2f : vget(g, k) * 0.8f;
-                gain = fmaxf(gain, 0.01f);
-                const float un = mom * uk - lr * (gk * gain);
-                vset(g, k, gain);
-                vset(u, k, un);
-                vset(yn, k, vget(yi, k) + un);
-                acc[k] += (double)vget(yn, k);
+                vset(u, k, __shfl_sync(0xffffffffu, vget(opnd, k), src + 1));
+                vset(g, k, __shfl_sync(0xffffffffu, vget(opnd, k), src + 2));
+                vset(r, k, __shfl_sync(0xffffffffu, vget(opnd, k), src + 3));
             }
-            uY[i] = u;
-            gains[i] = g;
-            Yn[i] = yn;
+            if (live && hl == 0) {
+                Vec<D> yn = yi;
+#pragma unroll
+                for (int k = 0; k < D; k++) {
+                    const float gk = exag4 * a[k] - vget(r, k);
+                    const float uk = vget(u, k);
+                    float gain = (uk * gk < 0.f) ? vget(g, k) + 0.2f : vget(g, k) * 0.8f;
+                    gain = fmaxf(gain, 0.01f);
+                    const float un = mom * uk - lr * (gk * gain);
+                    vset(g, k, gain);
+                    vset(u, k, un);
+                    vset(yn, k, vget(yi, k) + un);
+                    acc[k] += (double)vget(yn, k);
+                }
+                uY[i] = u;
+                gains[i] = g;
+                Yn[i] = yn;
+            }
         }
+        i = i_n;
+        yi = yi_n;
+        b = nb;
+        e = ne;
     }
     if (MODE == ATTR_GRAD) return;
     for (int k = 0; k < D; k++) acc[k] += __shfl_down_sync(0xffffffffu, acc[k], 16);
     block_sum_warps<D, WIN_THREADS / 32>(acc, partials + (size_t)blockIdx.x * D);
+}
+
+// The row ranges of the attractive step's CTAs: ranges[c] is the first row whose entries start at
+// or after c / ATTR_RANGES of P's (ATTR_RANGES + 1 entries). They depend on P alone, so they are
+// laid out once per numbering; every CTA's own search was a chain of up to 20 dependent loads.
+__global__ void k_attr_ranges(int n, const int *__restrict__ rp, int *__restrict__ ranges)
+{
+    const int c = blockIdx.x * blockDim.x + threadIdx.x;
+    if (c > ATTR_RANGES) return;
+    int lo = 0;
+    if (c == ATTR_RANGES) lo = n;
+    else {
+        const long long target = (long long)c * rp[n] / ATTR_RANGES;
+        int hi = n;
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (rp[mid] < target) lo = mid + 1;
+            else hi = mid;
+        }
+    }
+    ranges[c] = lo;
 }
 
 // Centring (reference tsne_h2pack.c:1978-1984): Y = Ynext - mean(Ynext), the mean summed
@@ -1145,26 +1209,19 @@ inline int ew_grid(int n) { int g = ceil_div(n, EW_BLOCK); return g < 1 ? 1 : (g
 // ---------------------------------------------------------------------------------
 // launchers
 // ---------------------------------------------------------------------------------
-// The shared-memory window forms of the attractive step (k_attr_window), chosen by
-// TSNE_ATTR_WINDOW: 1, one CTA per SM with a 128 KB window; 2 (2D; 3D takes form 1, its
-// update spills at 32 registers), two CTAs per SM with 64 KB windows (at most 32 registers
-// per thread, so twice the resident warps). A form is taken
-// while the average CTA's row range fits in half its window; all three modes and the
-// centring follow the same rule, so a step's kernels always agree on the row split. 0 (the
-// default): k_attr_update. Measured at 1M points, 2D: form 2 takes 1.40 ms per launch, form 1
-// 0.651 ms, k_attr_update 0.62 ms.
-template <int D>
-int window_form(int n)
+// Every CTA of the attractive step takes a contiguous range of rows (equal shares of P's
+// entries) instead of rows dealt round-robin, so one SM's gathers come from one neighbourhood of
+// the tree order (measured at 1M points: 0.622 ms per launch against 0.634 round-robin);
+// TSNE_ATTR_CONTIG=0 restores the round-robin split. All three modes follow the same split.
+int attr_contig()
 {
-    static const int form = [] {
-        const char *e = getenv("TSNE_ATTR_WINDOW");
-        const int v = e != nullptr ? atoi(e) : 0;
-        return (v == 1 || v == 2) ? v : 0;
+    static const int v = [] {
+        const char *e = getenv("TSNE_ATTR_CONTIG");
+        return e != nullptr && atoi(e) == 0 ? 0 : 1;
     }();
-    const int f = (D == 3 && form == 2) ? 1 : form;
-    if (f == 0) return 0;
-    return ceil_div(n, f * WIN_GRID) <= win_pts<D>() / f / 2 ? f : 0;
+    return v;
 }
+
 // Form of the attractive step, TSNE_ATTR_PIPE: 0 k_attr_update (32 registers in 2D, eight CTAs
 // per SM); 1 the same with the next step's entries loaded ahead (48 registers, five CTAs per
 // SM); 2 k_attr_pair (two rows per half-warp, five CTAs per SM); 3 the next step's columns
@@ -1182,66 +1239,33 @@ int attr_pipe()
     const int x = atoi(e);
     return (x >= 1 && x <= 4) ? x : 0;
 }
+// The window form (k_attr_window): always in 2D; in 3D once the points are renumbered in tree order,
+// or while all of them fit the window. With the points in their first order hardly any neighbour
+// lies in the window of a large set: in 2D the form is still the faster one (0.732 against 0.753 ms
+// at 1M points, 0.157 against 0.169 at 200K, both with TSNE_REORDER=0), in 3D the other is (0.102
+// against 0.105 ms at 100K; renumbered 0.097 against 0.088).
+// TSNE_ATTR_WINDOW=0 turns it off, and so does a form asked for by TSNE_ATTR_PIPE. Every kernel of
+// a step follows the same rule, so they agree on the number of partial sums.
 template <int D>
-int attr_blocks(int n)
+bool attr_window(int n, const AttrRows &rows)
 {
-    const int form = window_form<D>(n);
-    if (form != 0) return form * WIN_GRID;
+    const char *e = getenv("TSNE_ATTR_WINDOW");
+    const bool off = (e != nullptr && atoi(e) == 0) || getenv("TSNE_ATTR_PIPE") != nullptr || !attr_contig();
+    return !off && rows.ranges != nullptr && (D == 2 || rows.tree_order || n <= win_pts<D>());
+}
+template <int D>
+int attr_blocks(int n, const AttrRows &rows)
+{
+    if (attr_window<D>(n, rows)) return WIN_GRID;
     const int pipe = attr_pipe<D>();
     return pipe == 3 ? ATTR_PIPE3_GRID : pipe != 0 ? ATTR_PIPE_GRID : ROW_GRID;
 }
-template <int D, int MODE, int FORM>
-void launch_window_form(cudaStream_t st, int n, const int *rp, const int *col, const float *val, const void *Y,
-                        void *Ynext, void *uY, void *gains, const void *rep, const int *rep_flag, float exag4,
-                        float mom, float lr, double *partials, void *attr)
-{
-    constexpr int WINP = win_pts<D>() / FORM;
-    constexpr size_t smem = MODE == ATTR_UPDATE ? 0 : sizeof(Vec<D>) * (size_t)WINP;
-    // the window's shared memory, and (two CTAs per SM) a carve-out that holds both windows
-    static const cudaError_t attr_set =
-        FORM == 2 ? (cudaFuncSetAttribute(k_attr_window<D, MODE, WINP, FORM>,
-                                          cudaFuncAttributePreferredSharedMemoryCarveout,
-                                          (int)cudaSharedmemCarveoutMaxShared),
-                     cudaFuncSetAttribute(k_attr_window<D, MODE, WINP, FORM>,
-                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem))
-                  : cudaFuncSetAttribute(k_attr_window<D, MODE, WINP, FORM>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    (void)attr_set;
-    k_attr_window<D, MODE, WINP, FORM><<<FORM * WIN_GRID, WIN_THREADS, smem, st>>>(
-        n, rp, col, val, (const Vec<D> *)Y, (Vec<D> *)Ynext, (Vec<D> *)uY, (Vec<D> *)gains, (const Vec<D> *)rep,
-        rep_flag, exag4, mom, lr, partials, (Vec<D> *)attr);
-}
-template <int D, int MODE>
-void launch_window(cudaStream_t st, int n, const int *rp, const int *col, const float *val, const void *Y,
-                   void *Ynext, void *uY, void *gains, const void *rep, const int *rep_flag, float exag4, float mom,
-                   float lr, double *partials, void *attr)
-{
-    if (window_form<D>(n) == 1)
-        launch_window_form<D, MODE, 1>(st, n, rp, col, val, Y, Ynext, uY, gains, rep, rep_flag, exag4, mom, lr,
-                                       partials, attr);
-    else
-        launch_window_form<D, MODE, 2>(st, n, rp, col, val, Y, Ynext, uY, gains, rep, rep_flag, exag4, mom, lr,
-                                       partials, attr);
-}
-
-// Every CTA of the attractive step takes a contiguous range of rows (equal shares of P's
-// entries) instead of rows dealt round-robin, so one SM's gathers come from one neighbourhood of
-// the tree order (measured at 1M points: 0.622 ms per launch against 0.634 round-robin);
-// TSNE_ATTR_CONTIG=0 restores the round-robin split. All three modes follow the same split.
-int attr_contig()
-{
-    static const int v = [] {
-        const char *e = getenv("TSNE_ATTR_CONTIG");
-        return e != nullptr && atoi(e) == 0 ? 0 : 1;
-    }();
-    return v;
-}
-
 template <int D, int MODE, bool CONTIG>
-void launch_attr_rows(cudaStream_t st, int n, const int *rp, const int *col, const float *val, const void *Y,
+void launch_attr_rows(cudaStream_t st, int n, const AttrRows &rows, const int *col, const float *val, const void *Y,
                       void *Ynext, void *uY, void *gains, const void *rep, const int *rep_flag, float exag4,
                       float mom, float lr, double *partials, void *attr)
 {
+    const int *rp = rows.rp;
     const int pipe = attr_pipe<D>();
     if constexpr (MODE != ATTR_UPDATE) {
         if (pipe == 4) {
@@ -1258,80 +1282,80 @@ void launch_attr_rows(cudaStream_t st, int n, const int *rp, const int *col, con
     else if (pipe == 3)
         k_attr_update_pf<D, MODE, CONTIG, 2><<<ATTR_PIPE3_GRID, ROW_BLOCK, 0, st>>>(
             n, rp, col, val, (const Vec<D> *)Y, (Vec<D> *)Ynext, (Vec<D> *)uY, (Vec<D> *)gains,
-            (const Vec<D> *)rep, rep_flag, exag4, mom, lr, partials, (Vec<D> *)attr);
+            (const Vec<D> *)rep, rep_flag, exag4, mom, lr, partials, (Vec<D> *)attr, rows.ranges);
     else if (pipe == 1)
         k_attr_update_pf<D, MODE, CONTIG, 1><<<ATTR_PIPE_GRID, ROW_BLOCK, 0, st>>>(
             n, rp, col, val, (const Vec<D> *)Y, (Vec<D> *)Ynext, (Vec<D> *)uY, (Vec<D> *)gains,
-            (const Vec<D> *)rep, rep_flag, exag4, mom, lr, partials, (Vec<D> *)attr);
+            (const Vec<D> *)rep, rep_flag, exag4, mom, lr, partials, (Vec<D> *)attr, nullptr);
     else
         k_attr_update<D, MODE, CONTIG><<<ROW_GRID, ROW_BLOCK, 0, st>>>(
             n, rp, col, val, (const Vec<D> *)Y, (Vec<D> *)Ynext, (Vec<D> *)uY, (Vec<D> *)gains,
             (const Vec<D> *)rep, rep_flag, exag4, mom, lr, partials, (Vec<D> *)attr);
 }
 template <int D, int MODE>
-void launch_attr_any(cudaStream_t st, int n, const int *rp, const int *col, const float *val, const void *Y,
+void launch_attr_any(cudaStream_t st, int n, const AttrRows &rows, const int *col, const float *val, const void *Y,
                      void *Ynext, void *uY, void *gains, const void *rep, const int *rep_flag, float exag4,
                      float mom, float lr, double *partials, void *attr)
 {
+    if constexpr (MODE != ATTR_UPDATE) {
+        if (attr_window<D>(n, rows)) {
+            constexpr size_t smem = sizeof(Vec<D>) * (size_t)win_pts<D>();
+            TSNE_CUDA_CHECK(cudaFuncSetAttribute(k_attr_window<D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)smem));
+            k_attr_window<D, MODE><<<WIN_GRID, WIN_THREADS, smem, st>>>(
+                n, rows.ranges, rows.rp, col, val, (const Vec<D> *)Y, (Vec<D> *)Ynext, (Vec<D> *)uY, (Vec<D> *)gains,
+                (const Vec<D> *)rep, rep_flag, exag4, mom, lr, partials, (Vec<D> *)attr);
+            return;
+        }
+    }
     if (attr_contig())
-        launch_attr_rows<D, MODE, true>(st, n, rp, col, val, Y, Ynext, uY, gains, rep, rep_flag, exag4, mom, lr,
+        launch_attr_rows<D, MODE, true>(st, n, rows, col, val, Y, Ynext, uY, gains, rep, rep_flag, exag4, mom, lr,
                                         partials, attr);
     else
-        launch_attr_rows<D, MODE, false>(st, n, rp, col, val, Y, Ynext, uY, gains, rep, rep_flag, exag4, mom, lr,
+        launch_attr_rows<D, MODE, false>(st, n, rows, col, val, Y, Ynext, uY, gains, rep, rep_flag, exag4, mom, lr,
                                          partials, attr);
 }
 
 template <int D>
-void launch_attr_update(cudaStream_t st, int n, const int *rp, const int *col, const float *val,
+void launch_attr_update(cudaStream_t st, int n, const AttrRows &rows, const int *col, const float *val,
                         const void *Y, void *Ynext, void *uY, void *gains, const void *rep,
                         const int *rep_flag, float exag4, float mom, float lr, double *partials)
 {
-    if (window_form<D>(n) != 0) {
-        launch_window<D, ATTR_FUSED>(st, n, rp, col, val, Y, Ynext, uY, gains, rep, rep_flag, exag4, mom, lr,
-                                     partials, nullptr);
-        return;
-    }
-    launch_attr_any<D, ATTR_FUSED>(st, n, rp, col, val, Y, Ynext, uY, gains, rep, rep_flag, exag4, mom, lr,
+    launch_attr_any<D, ATTR_FUSED>(st, n, rows, col, val, Y, Ynext, uY, gains, rep, rep_flag, exag4, mom, lr,
                                    partials, nullptr);
 }
 template <int D>
-void launch_attr_grad(cudaStream_t st, int n, const int *rp, const int *col, const float *val, const void *Y,
+void launch_attr_grad(cudaStream_t st, int n, const AttrRows &rows, const int *col, const float *val, const void *Y,
                       void *attr)
 {
-    if (window_form<D>(n) != 0) {
-        launch_window<D, ATTR_GRAD>(st, n, rp, col, val, Y, nullptr, nullptr, nullptr, nullptr, nullptr, 0.f, 0.f,
-                                    0.f, nullptr, attr);
-        return;
-    }
-    launch_attr_any<D, ATTR_GRAD>(st, n, rp, col, val, Y, nullptr, nullptr, nullptr, nullptr, nullptr, 0.f, 0.f,
+    launch_attr_any<D, ATTR_GRAD>(st, n, rows, col, val, Y, nullptr, nullptr, nullptr, nullptr, nullptr, 0.f, 0.f,
                                   0.f, nullptr, attr);
 }
 template <int D>
-void launch_update(cudaStream_t st, int n, const int *rp, const void *Y, void *Ynext, void *uY, void *gains,
+void launch_update(cudaStream_t st, int n, const AttrRows &rows, const void *Y, void *Ynext, void *uY, void *gains,
                    const void *rep, const int *rep_flag, const void *attr, float exag4, float mom, float lr,
                    double *partials)
 {
-    if (window_form<D>(n) != 0) {
-        launch_window<D, ATTR_UPDATE>(st, n, rp, nullptr, nullptr, Y, Ynext, uY, gains, rep, rep_flag, exag4, mom,
-                                      lr, partials, const_cast<void *>(attr));
-        return;
-    }
-    if (attr_pipe<D>() != 0) {
-        k_update_rows<D><<<attr_blocks<D>(n), ROW_BLOCK, 0, st>>>(
+    if (attr_window<D>(n, rows) || attr_pipe<D>() != 0) {
+        k_update_rows<D><<<attr_blocks<D>(n, rows), ROW_BLOCK, 0, st>>>(
             n, (const Vec<D> *)Y, (Vec<D> *)Ynext, (Vec<D> *)uY, (Vec<D> *)gains, (const Vec<D> *)rep, rep_flag,
             (const Vec<D> *)attr, exag4, mom, lr, partials);
         return;
     }
-    launch_attr_any<D, ATTR_UPDATE>(st, n, rp, nullptr, nullptr, Y, Ynext, uY, gains, rep, rep_flag, exag4, mom,
+    launch_attr_any<D, ATTR_UPDATE>(st, n, rows, nullptr, nullptr, Y, Ynext, uY, gains, rep, rep_flag, exag4, mom,
                                     lr, partials, const_cast<void *>(attr));
+}
+void launch_attr_ranges(cudaStream_t st, int n, const int *rp, int *ranges)
+{
+    k_attr_ranges<<<ceil_div(ATTR_RANGES + 1, 128), 128, 0, st>>>(n, rp, ranges);
 }
 
 template <int D>
-void launch_center(cudaStream_t st, int n, const void *Ynext, void *Ycur, const double *partials,
-                   DevScalars *sc, const void *, double *)
+void launch_center(cudaStream_t st, int n, const AttrRows &rows, const void *Ynext, void *Ycur, const double *partials,
+                   DevScalars *sc)
 {
-    const int nblk = attr_blocks<D>(n);
-    k_center<D><<<ew_grid(n), RED_BLOCK, 0, st>>>(n, (const Vec<D> *)Ynext, (Vec<D> *)Ycur, partials, nblk, sc);
+    k_center<D><<<ew_grid(n), RED_BLOCK, 0, st>>>(n, (const Vec<D> *)Ynext, (Vec<D> *)Ycur, partials,
+                                                  attr_blocks<D>(n, rows), sc);
 }
 
 template <int D>
@@ -1417,16 +1441,16 @@ void launch_pcal(cudaStream_t st, int n, const int *indptr, const double *dist, 
 }
 
 #define TSNE_INST(D)                                                                              \
-    template void launch_attr_update<D>(cudaStream_t, int, const int *, const int *, const float *,  \
+    template void launch_attr_update<D>(cudaStream_t, int, const AttrRows &, const int *, const float *, \
                                         const void *, void *, void *, void *, const void *,          \
                                         const int *, float, float, float, double *);                 \
-    template void launch_attr_grad<D>(cudaStream_t, int, const int *, const int *, const float *,    \
+    template void launch_attr_grad<D>(cudaStream_t, int, const AttrRows &, const int *, const float *, \
                                       const void *, void *);                                         \
-    template void launch_update<D>(cudaStream_t, int, const int *, const void *, void *, void *,     \
+    template void launch_update<D>(cudaStream_t, int, const AttrRows &, const void *, void *, void *, \
                                    void *, const void *, const int *, const void *, float, float,    \
                                    float, double *);                                                 \
-    template void launch_center<D>(cudaStream_t, int, const void *, void *, const double *,         \
-                                   DevScalars *, const void *, double *);                            \
+    template void launch_center<D>(cudaStream_t, int, const AttrRows &, const void *, void *,        \
+                                   const double *, DevScalars *);                                    \
     template void launch_exact_sv<D>(cudaStream_t, int, const void *, float4 *);                    \
     template void launch_z_force<D>(cudaStream_t, int, const void *, const float4 *, const int *,   \
                                     void *, DevScalars *, double *, int, int);          \

@@ -127,6 +127,7 @@ struct tsne_workspace {
 
     cudaStream_t st = nullptr;
     DevBuf<int> rp, col, rp2, col2, len, inv, order, order2;
+    DevBuf<int> ranges;             // row ranges of the attractive step's CTAs, for this numbering
     long long padded_nnz = 0;
     DevBuf<float> val, val2;
     DevBuf<unsigned char> Y, Yn, uY, gains, rep, frc, tmpv, Yconv;
@@ -296,8 +297,9 @@ void pad_P(tsne_workspace *ws, const int *rp0, const int *ci0, const V *pv0)
     ws->val.exact(std::max(padded, 4));
     ws->padded_nnz = padded;
     k_pad_copy<V><<<ROW_GRID, ROW_BLOCK, 0, st>>>(n, rp0, ci0, pv0, ws->rp.p, ws->col.p, ws->val.p);
+    launch_attr_ranges(st, n, ws->rp.p, ws->ranges.exact(ATTR_RANGE_TABLE));
     TSNE_CUDA_CHECK(cudaStreamSynchronize(st));
-    ws->n_launch += 3;
+    ws->n_launch += 4;
 }
 
 template <int D>
@@ -391,6 +393,7 @@ void renumber_impl(tsne_workspace *ws, const int *ord_dev)
     ws->val2.exact(std::max<long long>(nnz, 4));
     launch_row_gather(st, n, ord_dev, ws->inv.p, ws->rp.p, ws->col.p, ws->val.p, ws->rp2.p, ws->col2.p, ws->val2.p);
     ws->rp.swap(ws->rp2);
+    launch_attr_ranges(st, n, ws->rp.p, ws->ranges.exact(ATTR_RANGE_TABLE));
     ws->col.swap(ws->col2);
     ws->val.swap(ws->val2);
     ws->tmpv.exact(ws->vbytes * n);
@@ -405,7 +408,7 @@ void renumber_impl(tsne_workspace *ws, const int *ord_dev)
     ws->order.swap(ws->order2);
     ws->has_order = true;
     ws->tiles.valid = false;        // rows changed: the tile format is rebuilt by the caller
-    ws->n_launch += 11;
+    ws->n_launch += 12;
 }
 
 void renumber(tsne_workspace *ws, const int *ord_dev)
@@ -425,13 +428,7 @@ void exact_force(tsne_workspace *ws)
     ws->n_launch += 3;
 }
 
-// the shared-memory window forms (TSNE_ATTR_WINDOW) are off: the CSR kernels that the tile
-// form pairs with (the update after a rebuild, the centring) use the ROW_GRID row split
-bool window_off()
-{
-    const char *e = getenv("TSNE_ATTR_WINDOW");
-    return e == nullptr || atoi(e) == 0;
-}
+AttrRows attr_rows(const tsne_workspace *ws) { return {ws->rp.p, ws->ranges.p, ws->has_order}; }
 
 bool next_reorder_due(tsne_workspace *ws, int iter, const int *iters, int n_reorder)
 {
@@ -469,7 +466,7 @@ int run_range_impl(tsne_workspace *ws, int it_begin, int it_end)
     }
     // the shared-column tile form of the 2D attractive pass (TSNE_ATTR_TILES=1; off by default
     // until it measures faster), built at the renumberings from iteration tiles_from on
-    const bool tiles_on = env_int("TSNE_ATTR_TILES", 0) != 0 && window_off() && getenv("TSNE_ATTR_PIPE") != nullptr &&
+    const bool tiles_on = env_int("TSNE_ATTR_TILES", 0) != 0 && getenv("TSNE_ATTR_PIPE") != nullptr &&
                           env_int("TSNE_ATTR_PIPE", 0) == 0;
     const int tiles_from = env_int("TSNE_ATTR_TILES_FROM", 100);
     const int tile_rows = env_int("TSNE_ATTR_TILE_ROWS", 64), tile_umax = env_int("TSNE_ATTR_TILE_UMAX", 6144);
@@ -532,7 +529,7 @@ int run_range_impl(tsne_workspace *ws, int it_begin, int it_end)
                 if (D == 2 && ws->tiles.valid)
                     launch_attr_tile_grad(st, n, ws->tiles, ws->rp.p, ws->col.p, ws->val.p, ws->Y.p, ws->attr.p);
                 else
-                    launch_attr_grad<D>(st, n, ws->rp.p, ws->col.p, ws->val.p, ws->Y.p, ws->attr.p);
+                    launch_attr_grad<D>(st, n, attr_rows(ws), ws->col.p, ws->val.p, ws->Y.p, ws->attr.p);
                 attr_ready = true;
                 ws->n_launch++;
             };
@@ -596,7 +593,7 @@ int run_range_impl(tsne_workspace *ws, int it_begin, int it_end)
         size_t e2 = evused;
         if (prof) stage_event(ws, evpool, evused);
         if (attr_ready) {
-            launch_update<D>(st, n, ws->rp.p, ws->Y.p, ws->Yn.p, ws->uY.p, ws->gains.p, force, flag, ws->attr.p,
+            launch_update<D>(st, n, attr_rows(ws), ws->Y.p, ws->Yn.p, ws->uY.p, ws->gains.p, force, flag, ws->attr.p,
                              (float)(4.0 * exag), (float)mom, (float)lr, ws->part.p);
         } else {
             if (ktime) stage_event(ws, kev, kused);
@@ -605,7 +602,7 @@ int run_range_impl(tsne_workspace *ws, int it_begin, int it_end)
                                         ws->uY.p, ws->gains.p, force, flag, (float)(4.0 * exag), (float)mom,
                                         (float)lr, ws->part.p);
             else
-                launch_attr_update<D>(st, n, ws->rp.p, ws->col.p, ws->val.p, ws->Y.p, ws->Yn.p, ws->uY.p,
+                launch_attr_update<D>(st, n, attr_rows(ws), ws->col.p, ws->val.p, ws->Y.p, ws->Yn.p, ws->uY.p,
                                       ws->gains.p, force, flag, (float)(4.0 * exag), (float)mom, (float)lr,
                                       ws->part.p);
             if (ktime) stage_event(ws, kev, kused);
@@ -613,7 +610,7 @@ int run_range_impl(tsne_workspace *ws, int it_begin, int it_end)
         if (prof) { stage_event(ws, evpool, evused); stages.push_back({iter, 0, e2, evused - 1}); }
         size_t e3 = evused;
         if (prof) stage_event(ws, evpool, evused);
-        launch_center<D>(st, n, ws->Yn.p, ws->Y.p, ws->part.p, ws->sc.p, nullptr, nullptr);
+        launch_center<D>(st, n, attr_rows(ws), ws->Yn.p, ws->Y.p, ws->part.p, ws->sc.p);
         ws->n_launch += 2;
 
         if (p.enable_early_stopping && iter >= p.min_iter - 1) {

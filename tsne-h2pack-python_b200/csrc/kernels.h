@@ -38,21 +38,31 @@ struct TreeInfo {
 };
 
 // ---- dense per-point kernels (dense.cu) ----
+// P's rows as the attractive step takes them: row pointers, the table of its CTAs' row ranges
+// (launch_attr_ranges, ATTR_RANGE_TABLE entries; null: none), and whether the points are numbered
+// in the order of an H2 tree.
+struct AttrRows {
+    const int *rp;
+    const int *ranges;
+    bool tree_order;
+};
+constexpr int ATTR_RANGE_TABLE = 148 * 6 + 1;
+void launch_attr_ranges(cudaStream_t st, int n, const int *rp, int *ranges);
 template <int D>
-void launch_attr_update(cudaStream_t st, int n, const int *rp, const int *col, const float *val,
+void launch_attr_update(cudaStream_t st, int n, const AttrRows &rows, const int *col, const float *val,
                         const void *Y, void *Ynext, void *uY, void *gains, const void *rep,
                         const int *rep_flag, float exag4, float mom, float lr, double *partials);
 // the attractive sums alone (into attr), and the update from them (same bits as the fused step)
 template <int D>
-void launch_attr_grad(cudaStream_t st, int n, const int *rp, const int *col, const float *val, const void *Y,
+void launch_attr_grad(cudaStream_t st, int n, const AttrRows &rows, const int *col, const float *val, const void *Y,
                       void *attr);
 template <int D>
-void launch_update(cudaStream_t st, int n, const int *rp, const void *Y, void *Ynext, void *uY, void *gains,
+void launch_update(cudaStream_t st, int n, const AttrRows &rows, const void *Y, void *Ynext, void *uY, void *gains,
                    const void *rep, const int *rep_flag, const void *attr, float exag4, float mom, float lr,
                    double *partials);
 template <int D>
-void launch_center(cudaStream_t st, int n, const void *Ynext, void *Ycur, const double *partials,
-                   DevScalars *sc, const void *Yprev_conv, double *conv_partials);
+void launch_center(cudaStream_t st, int n, const AttrRows &rows, const void *Ynext, void *Ycur, const double *partials,
+                   DevScalars *sc);
 template <int D>
 void launch_exact_sv(cudaStream_t st, int n, const void *Y, float4 *sv);
 template <int D>
