@@ -13,6 +13,8 @@
 #include <math.h>
 #include <stdlib.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "kernels.h"
 
@@ -1316,13 +1318,15 @@ void launch_attr_any(cudaStream_t st, int n, const AttrRows &rows, const int *co
                                          partials, attr);
 }
 
+// the number of partial sums a step leaves for the centring
 template <int D>
-void launch_attr_update(cudaStream_t st, int n, const AttrRows &rows, const int *col, const float *val,
-                        const void *Y, void *Ynext, void *uY, void *gains, const void *rep,
-                        const int *rep_flag, float exag4, float mom, float lr, double *partials)
+int launch_attr_update(cudaStream_t st, int n, const AttrRows &rows, const int *col, const float *val,
+                       const void *Y, void *Ynext, void *uY, void *gains, const void *rep,
+                       const int *rep_flag, float exag4, float mom, float lr, double *partials)
 {
     launch_attr_any<D, ATTR_FUSED>(st, n, rows, col, val, Y, Ynext, uY, gains, rep, rep_flag, exag4, mom, lr,
                                    partials, nullptr);
+    return attr_blocks<D>(n, rows);
 }
 template <int D>
 void launch_attr_grad(cudaStream_t st, int n, const AttrRows &rows, const int *col, const float *val, const void *Y,
@@ -1332,18 +1336,22 @@ void launch_attr_grad(cudaStream_t st, int n, const AttrRows &rows, const int *c
                                   0.f, nullptr, attr);
 }
 template <int D>
-void launch_update(cudaStream_t st, int n, const AttrRows &rows, const void *Y, void *Ynext, void *uY, void *gains,
-                   const void *rep, const int *rep_flag, const void *attr, float exag4, float mom, float lr,
-                   double *partials)
+int launch_update(cudaStream_t st, int n, const AttrRows &rows, const void *Y, void *Ynext, void *uY, void *gains,
+                  const void *rep, const int *rep_flag, const void *attr, float exag4, float mom, float lr,
+                  double *partials)
 {
-    if (attr_window<D>(n, rows) || attr_pipe<D>() != 0) {
-        k_update_rows<D><<<attr_blocks<D>(n, rows), ROW_BLOCK, 0, st>>>(
+    const bool window = attr_window<D>(n, rows);
+    if (window || attr_pipe<D>() != 0) {
+        // the window form's rows are a thread each here: as many CTAs as rows fill, up to six per SM
+        const int blocks = window ? std::min(ATTR_PIPE3_GRID, ceil_div(n, ROW_BLOCK)) : attr_blocks<D>(n, rows);
+        k_update_rows<D><<<blocks, ROW_BLOCK, 0, st>>>(
             n, (const Vec<D> *)Y, (Vec<D> *)Ynext, (Vec<D> *)uY, (Vec<D> *)gains, (const Vec<D> *)rep, rep_flag,
             (const Vec<D> *)attr, exag4, mom, lr, partials);
-        return;
+        return blocks;
     }
     launch_attr_any<D, ATTR_UPDATE>(st, n, rows, nullptr, nullptr, Y, Ynext, uY, gains, rep, rep_flag, exag4, mom,
                                     lr, partials, const_cast<void *>(attr));
+    return attr_blocks<D>(n, rows);
 }
 void launch_attr_ranges(cudaStream_t st, int n, const int *rp, int *ranges)
 {
@@ -1351,11 +1359,10 @@ void launch_attr_ranges(cudaStream_t st, int n, const int *rp, int *ranges)
 }
 
 template <int D>
-void launch_center(cudaStream_t st, int n, const AttrRows &rows, const void *Ynext, void *Ycur, const double *partials,
+void launch_center(cudaStream_t st, int n, const void *Ynext, void *Ycur, const double *partials, int n_partial,
                    DevScalars *sc)
 {
-    k_center<D><<<ew_grid(n), RED_BLOCK, 0, st>>>(n, (const Vec<D> *)Ynext, (Vec<D> *)Ycur, partials,
-                                                  attr_blocks<D>(n, rows), sc);
+    k_center<D><<<ew_grid(n), RED_BLOCK, 0, st>>>(n, (const Vec<D> *)Ynext, (Vec<D> *)Ycur, partials, n_partial, sc);
 }
 
 template <int D>
@@ -1441,16 +1448,16 @@ void launch_pcal(cudaStream_t st, int n, const int *indptr, const double *dist, 
 }
 
 #define TSNE_INST(D)                                                                              \
-    template void launch_attr_update<D>(cudaStream_t, int, const AttrRows &, const int *, const float *, \
-                                        const void *, void *, void *, void *, const void *,          \
-                                        const int *, float, float, float, double *);                 \
+    template int launch_attr_update<D>(cudaStream_t, int, const AttrRows &, const int *, const float *, \
+                                       const void *, void *, void *, void *, const void *,           \
+                                       const int *, float, float, float, double *);                  \
     template void launch_attr_grad<D>(cudaStream_t, int, const AttrRows &, const int *, const float *, \
                                       const void *, void *);                                         \
-    template void launch_update<D>(cudaStream_t, int, const AttrRows &, const void *, void *, void *, \
-                                   void *, const void *, const int *, const void *, float, float,    \
-                                   float, double *);                                                 \
-    template void launch_center<D>(cudaStream_t, int, const AttrRows &, const void *, void *,        \
-                                   const double *, DevScalars *);                                    \
+    template int launch_update<D>(cudaStream_t, int, const AttrRows &, const void *, void *, void *, \
+                                  void *, const void *, const int *, const void *, float, float,     \
+                                  float, double *);                                                  \
+    template void launch_center<D>(cudaStream_t, int, const void *, void *, const double *, int,     \
+                                   DevScalars *);                                                    \
     template void launch_exact_sv<D>(cudaStream_t, int, const void *, float4 *);                    \
     template void launch_z_force<D>(cudaStream_t, int, const void *, const float4 *, const int *,   \
                                     void *, DevScalars *, double *, int, int);          \

@@ -592,8 +592,9 @@ int run_range_impl(tsne_workspace *ws, int it_begin, int it_end)
 
         size_t e2 = evused;
         if (prof) stage_event(ws, evpool, evused);
+        int n_partial = ROW_GRID;   // the tile form's
         if (attr_ready) {
-            launch_update<D>(st, n, attr_rows(ws), ws->Y.p, ws->Yn.p, ws->uY.p, ws->gains.p, force, flag, ws->attr.p,
+            n_partial = launch_update<D>(st, n, attr_rows(ws), ws->Y.p, ws->Yn.p, ws->uY.p, ws->gains.p, force, flag, ws->attr.p,
                              (float)(4.0 * exag), (float)mom, (float)lr, ws->part.p);
         } else {
             if (ktime) stage_event(ws, kev, kused);
@@ -602,7 +603,7 @@ int run_range_impl(tsne_workspace *ws, int it_begin, int it_end)
                                         ws->uY.p, ws->gains.p, force, flag, (float)(4.0 * exag), (float)mom,
                                         (float)lr, ws->part.p);
             else
-                launch_attr_update<D>(st, n, attr_rows(ws), ws->col.p, ws->val.p, ws->Y.p, ws->Yn.p, ws->uY.p,
+                n_partial = launch_attr_update<D>(st, n, attr_rows(ws), ws->col.p, ws->val.p, ws->Y.p, ws->Yn.p, ws->uY.p,
                                       ws->gains.p, force, flag, (float)(4.0 * exag), (float)mom, (float)lr,
                                       ws->part.p);
             if (ktime) stage_event(ws, kev, kused);
@@ -610,7 +611,7 @@ int run_range_impl(tsne_workspace *ws, int it_begin, int it_end)
         if (prof) { stage_event(ws, evpool, evused); stages.push_back({iter, 0, e2, evused - 1}); }
         size_t e3 = evused;
         if (prof) stage_event(ws, evpool, evused);
-        launch_center<D>(st, n, attr_rows(ws), ws->Yn.p, ws->Y.p, ws->part.p, ws->sc.p);
+        launch_center<D>(st, n, ws->Yn.p, ws->Y.p, ws->part.p, n_partial, ws->sc.p);
         ws->n_launch += 2;
 
         if (p.enable_early_stopping && iter >= p.min_iter - 1) {

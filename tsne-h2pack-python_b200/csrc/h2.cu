@@ -49,7 +49,6 @@ struct TreeView {
     int *start, *end, *level, *parent, *fchild, *nchild, *leaf, *ix;
     int4 *rec;               // per node, packed for the list pass: see node_rec
     float4 *proxies;         // per level: see proxy_table
-    signed char *delta;      // shared leading digits with the previous key (n + 1)
     int *fm;                 // per point: first | last level << 8 of the nodes it starts, or -1
     int *blkcnt, *blkoff;    // per block of TREE_BLOCK points, 2 x 32 counts / offsets
     int *bset, *nid;         // per level l: boundary starts B_l and their node ids (stride cap_node)
@@ -181,17 +180,17 @@ __device__ void root_from_parts(int n, int nblk, const double *part, const TreeV
     tv.ix[0] = tv.ix[1] = tv.ix[2] = 0;
 }
 
+// Morton keys of the cells at depth L, FP64 with IEEE operations only
 template <int D>
-__global__ void k_keys(int n, int L, const Vec<D> *__restrict__ Y, const TreeInfo *__restrict__ info,
-                       unsigned long long *__restrict__ keys, int *__restrict__ idx)
-{
-    const double R = info->radius;
-    const double cell = 2.0 * R / (double)(1LL << L);
-    const double qmax = (double)((1LL << L) - 1);
-    double corner[D];
-    for (int k = 0; k < D; k++) corner[k] = info->corner[k];
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const Vec<D> y = Y[i];
+struct KeyMaker {
+    double cell, qmax, corner[D];
+    __device__ __forceinline__ KeyMaker(const TreeInfo *info, int L)
+        : cell(2.0 * info->radius / (double)(1LL << L)), qmax((double)((1LL << L) - 1))
+    {
+        for (int k = 0; k < D; k++) corner[k] = info->corner[k];
+    }
+    __device__ __forceinline__ unsigned long long key(const Vec<D> &y, int L) const
+    {
         unsigned int q[D];
         for (int k = 0; k < D; k++) {
             const double t = ((double)vget(y, k) - corner[k]) / cell;
@@ -204,9 +203,86 @@ __global__ void k_keys(int n, int L, const Vec<D> *__restrict__ Y, const TreeInf
         unsigned long long key = 0;
         for (int b = L - 1; b >= 0; b--)
             for (int k = D - 1; k >= 0; k--) key = (key << 1) | ((q[k] >> b) & 1u);
-        keys[i] = key;
+        return key;
+    }
+};
+
+template <int D>
+__global__ void k_keys(int n, int L, const Vec<D> *__restrict__ Y, const TreeInfo *__restrict__ info,
+                       unsigned long long *__restrict__ keys, int *__restrict__ idx)
+{
+    const KeyMaker<D> km(info, L);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        keys[i] = km.key(Y[i], L);
         idx[i] = i;
     }
+}
+
+// The sort of up to SORT_MOST points. The device-wide radix sort is nine launches with the keys'
+// whatever the size, about 70 us at 20K points; this is two, 36 us. Tiles of SORT_TILE points are
+// made (keys and all) and sorted by a CTA each, stably; a point's place in the whole order is its
+// place in its tile plus, for every other tile, the keys there that come before it: those <= its
+// key in the tiles before (equal keys keep their order), those < its key in the tiles after. The
+// bisections grow with the square of the points: a rebuild gains 35 us at 50K and at 66K points and
+// 17 us at 131K; beyond, the radix sort.
+constexpr int SORT_THREADS = 512, SORT_ITEMS = 4, SORT_TILE = SORT_THREADS * SORT_ITEMS;
+constexpr int SORT_MOST = 131072;
+
+struct KeyLess {
+    __device__ bool operator()(unsigned long long a, unsigned long long b) const { return a < b; }
+};
+
+template <int D>
+__global__ void __launch_bounds__(SORT_THREADS)
+k_tile_sort(int n, int L, const Vec<D> *__restrict__ Y, const TreeInfo *__restrict__ info,
+            unsigned long long *__restrict__ keys, int *__restrict__ idx)
+{
+    using Sort = cub::BlockMergeSort<unsigned long long, SORT_THREADS, SORT_ITEMS, int>;
+    __shared__ typename Sort::TempStorage tmp;
+    const KeyMaker<D> km(info, L);
+    const int base = blockIdx.x * SORT_TILE + threadIdx.x * SORT_ITEMS;
+    unsigned long long k[SORT_ITEMS];
+    int v[SORT_ITEMS];
+#pragma unroll
+    for (int q = 0; q < SORT_ITEMS; q++) {   // past the end: above every key (a key has 60 bits at most)
+        v[q] = base + q;
+        k[q] = base + q < n ? km.key(Y[base + q], L) : ~0ULL;
+    }
+    Sort(tmp).StableSort(k, v, KeyLess());
+#pragma unroll
+    for (int q = 0; q < SORT_ITEMS; q++)
+        if (base + q < n) {
+            keys[base + q] = k[q];
+            idx[base + q] = v[q];
+        }
+}
+
+__global__ void __launch_bounds__(256) k_tile_rank(int n, const unsigned long long *__restrict__ tk,
+                                                   const int *__restrict__ ti, unsigned long long *__restrict__ keys,
+                                                   int *__restrict__ perm)
+{
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i >= n) return;
+    const unsigned long long k = tk[i];
+    const int mine = i / SORT_TILE, tiles = (n + SORT_TILE - 1) / SORT_TILE;
+    int rank = i % SORT_TILE;
+    constexpr int T = 4;   // bisections side by side: each step is a dependent load
+    for (int t0 = 0; t0 < tiles; t0 += T) {
+        int pos[T];
+#pragma unroll
+        for (int q = 0; q < T; q++) pos[q] = 0;
+        // keys of tile t that come before point i: those < k + 1 before its own tile, < k after
+        for (int step = SORT_TILE; step > 0; step >>= 1)
+#pragma unroll
+            for (int q = 0; q < T; q++) {
+                const int t = t0 + q, p = t * SORT_TILE + pos[q] + step;   // (past the last tile: p > n)
+                if (pos[q] + step <= SORT_TILE && p <= n && tk[p - 1] < (t < mine ? k + 1 : k)) pos[q] += step;
+            }
+#pragma unroll
+        for (int q = 0; q < T; q++) rank += t0 + q == mine ? 0 : pos[q];
+    }
+    keys[rank] = k;
+    perm[rank] = ti[i];
 }
 
 // ---------------------------------------------------------------------------------
@@ -235,32 +311,31 @@ __device__ __forceinline__ int shared_digits(unsigned long long a, unsigned long
     return (__clzll((long long)x) - (64 - D * L)) / D;
 }
 
+// coordinate k of a key: every D-th bit, brought together by halving steps
 template <int D>
-__device__ __forceinline__ unsigned int key_coord(unsigned long long key, int k, int L)
+__device__ __forceinline__ unsigned int key_coord(unsigned long long key, int k)
 {
-    unsigned int q = 0;
-    for (int b = 0; b < L; b++) q |= (unsigned int)((key >> (D * b + k)) & 1ULL) << b;
-    return q;
-}
-
-// tree-order coordinates, and delta (with its sentinel)
-template <int D>
-__global__ void k_gather(int n, int L, const int *__restrict__ perm, const Vec<D> *__restrict__ Y,
-                         Vec<D> *__restrict__ xt, const unsigned long long *__restrict__ keys,
-                         signed char *__restrict__ delta)
-{
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= n; i += gridDim.x * blockDim.x) {
-        if (i == n) {
-            delta[n] = -1;
-            continue;
-        }
-        xt[i] = Y[perm[i]];
-        delta[i] = i == 0 ? (signed char)-1 : (signed char)shared_digits<D>(keys[i - 1], keys[i], L);
+    unsigned long long x = key >> k;
+    if constexpr (D == 2) {
+        x &= 0x5555555555555555ULL;
+        x = (x | x >> 1) & 0x3333333333333333ULL;
+        x = (x | x >> 2) & 0x0f0f0f0f0f0f0f0fULL;
+        x = (x | x >> 4) & 0x00ff00ff00ff00ffULL;
+        x = (x | x >> 8) & 0x0000ffff0000ffffULL;
+        x = (x | x >> 16) & 0x00000000ffffffffULL;
+    } else {
+        x &= 0x1249249249249249ULL;
+        x = (x | x >> 2) & 0x10c30c30c30c30c3ULL;
+        x = (x | x >> 4) & 0x100f00f00f00f00fULL;
+        x = (x | x >> 8) & 0x001f0000ff0000ffULL;
+        x = (x | x >> 16) & 0x001f00000000ffffULL;
+        x = (x | x >> 32) & 0x00000000001fffffULL;
     }
+    return (unsigned int)x;
 }
 
 // per point: E, f, m packed in fm (-1: starts no node); per block and level the number of
-// node starts and of boundary starts
+// node starts and of boundary starts; the tree-order coordinates
 __device__ __forceinline__ void tree_bits(int fm, int l, bool &bn, bool &bb)
 {
     const int f = fm & 0xff, m = fm >> 8;
@@ -268,43 +343,72 @@ __device__ __forceinline__ void tree_bits(int fm, int l, bool &bn, bool &bb)
     bn = bb && l <= m;
 }
 
+// In the sorted keys the least delta of (a, b] is the number of digits key[a] and key[b] share, so
+// neither question needs a walk: the run of points that share delta[s] digits with s starts at p,
+// found by bisection over the leaf_size points before s, and E_s is whether point p + leaf_size
+// still belongs to it; m_s comes from the digits that points s and s + leaf_size share. The
+// block's keys and leaf_size on each side are staged in shared memory while that fits. Walking
+// point by point, up to leaf_size each way, took 82 us at 1M points and 18 at 20K with a launch of
+// its own for the coordinates (10 and 4 us); this takes 37 and 9 us.
+constexpr int TREE_HALO = 256;     // longest leaf_size whose keys are staged
+
 template <int D>
-__global__ void __launch_bounds__(TREE_BLOCK) k_tree_marks(TreeView tv)
+__global__ void __launch_bounds__(TREE_BLOCK) k_tree_marks(TreeView tv, const int *__restrict__ perm,
+                                                           const Vec<D> *__restrict__ Y, Vec<D> *__restrict__ xt)
 {
     __shared__ int wc[2][32][TREE_BLOCK / 32];
+    __shared__ int s_max[TREE_BLOCK / 32];
+    __shared__ unsigned long long sk[TREE_BLOCK + 2 * TREE_HALO];
     const int n = tv.n, L = tv.L, leaf = tv.leaf_size;
-    const signed char *delta = tv.delta;
-    const int s = blockIdx.x * TREE_BLOCK + threadIdx.x;
+    const int b0 = blockIdx.x * TREE_BLOCK, s = b0 + threadIdx.x;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const bool staged = leaf <= TREE_HALO;
+    if (staged)
+        for (int i = max(0, b0 - leaf) + threadIdx.x; i < min(n, b0 + TREE_BLOCK + leaf); i += TREE_BLOCK)
+            sk[i - b0 + TREE_HALO] = tv.keys[i];
+    if (s < n) xt[s] = Y[perm[s]];
+    __syncthreads();
+    auto key = [&](int i) { return staged ? sk[i - b0 + TREE_HALO] : tv.keys[i]; };
     int fm = -1;
     if (s < n) {
-        const int ds = delta[s], f = ds + 1;
+        const unsigned long long ks = key(s);
+        const int ds = s == 0 ? -1 : shared_digits<D>(key(s - 1), ks, L), f = ds + 1;
         bool E = s == 0;
         if (s > 0) {
-            int j = s - 1;
-            while (delta[j] >= ds && s - j <= leaf) j--;   // delta[0] = -1 ends the walk
-            const int left = s - j;
-            if (left > leaf) E = true;
+            auto with_s = [&](int i) { return shared_digits<D>(key(i), ks, L) >= ds; };
+            if (s >= leaf && with_s(s - leaf)) E = true;
             else {
-                int k = s + 1;
-                while (k < n && delta[k] >= ds && left + (k - s) <= leaf) k++;
-                E = left + (k - s) > leaf;
+                int lo = max(0, s - leaf), p = s - 1;   // point s - 1 shares delta[s] digits
+                while (lo < p) {
+                    const int mid = (lo + p) >> 1;
+                    if (with_s(mid)) p = mid;
+                    else lo = mid + 1;
+                }
+                E = leaf < n - p && with_s(p + leaf);
             }
         }
         if (f > L) E = false;
         if (E) {
-            int mu = L + 1;
-            const int last = min(s + leaf, n);
-            for (int j = s + 1; j <= last && mu >= f; j++) mu = min(mu, (int)delta[j]);
-            const int m = min(L, max(f, mu + 1));
-            fm = f | (m << 8);
+            const int mu = leaf < n - s ? shared_digits<D>(ks, key(s + leaf), L) : -1;
+            fm = f | (min(L, max(f, mu + 1)) << 8);
         }
         tv.fm[s] = fm;
     }
+    // counts of the levels up to the block's deepest node; below it every mark is a boundary
+    int mm = fm >= 0 ? fm >> 8 : -1;
+    mm = __reduce_max_sync(0xffffffffu, mm);
+    const unsigned marks = __ballot_sync(0xffffffffu, fm >= 0);
+    if (lane == 0) s_max[w] = mm;
+    __syncthreads();
+    const int deepest = __reduce_max_sync(0xffffffffu, s_max[lane]);
     for (int l = 0; l <= L; l++) {
-        bool bn, bb;
-        tree_bits(fm, l, bn, bb);
-        const unsigned vn = __ballot_sync(0xffffffffu, bn), vb = __ballot_sync(0xffffffffu, bb);
+        unsigned vn = 0, vb = marks;
+        if (l <= deepest) {
+            bool bn, bb;
+            tree_bits(fm, l, bn, bb);
+            vn = __ballot_sync(0xffffffffu, bn);
+            vb = __ballot_sync(0xffffffffu, bb);
+        }
         if (lane == 0) { wc[0][l][w] = __popc(vn); wc[1][l][w] = __popc(vb); }
     }
     __syncthreads();
@@ -370,7 +474,7 @@ template <int D>
 __global__ void __launch_bounds__(TREE_BLOCK) k_tree_emit(TreeView tv)
 {
     __shared__ int wo[2][32][TREE_BLOCK / 32];
-    __shared__ int sboff[2][32], slb[32], s_over;
+    __shared__ int sboff[2][32], slb[32], s_over, s_deep;
     const int n = tv.n, L = tv.L;
     const int s = blockIdx.x * TREE_BLOCK + threadIdx.x;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -385,7 +489,7 @@ __global__ void __launch_bounds__(TREE_BLOCK) k_tree_emit(TreeView tv)
         const unsigned used = __ballot_sync(0xffffffffu, c > 0);
         const int over = total > tv.cap_node;   // node table full: the host regrows it; nothing downstream runs
         slb[lane] = x - c;
-        if (lane == 0) s_over = over;
+        if (lane == 0) { s_over = over; s_deep = 31 - __clz((int)used); }
         if (blockIdx.x == 0) {
             TreeInfo *info = tv.info;
             info->level_begin[lane] = x - c;
@@ -400,9 +504,10 @@ __global__ void __launch_bounds__(TREE_BLOCK) k_tree_emit(TreeView tv)
     }
     __syncthreads();
     if (s_over) return;
+    const int deepest = s_deep;   // no level below it has a node: its boundaries are not needed
     const unsigned lt = (1u << lane) - 1u;
     const int fm = s < n ? tv.fm[s] : -1;
-    for (int l = 0; l <= L; l++) {
+    for (int l = 0; l <= deepest; l++) {
         bool bn, bb;
         tree_bits(fm, l, bn, bb);
         const unsigned vn = __ballot_sync(0xffffffffu, bn), vb = __ballot_sync(0xffffffffu, bb);
@@ -411,7 +516,7 @@ __global__ void __launch_bounds__(TREE_BLOCK) k_tree_emit(TreeView tv)
     __syncthreads();
     if (threadIdx.x < 64) {   // exclusive scan over the warps, per array and level
         const int arr = threadIdx.x >> 5, l = threadIdx.x & 31;
-        if (l <= L) {
+        if (l <= deepest) {
             int run = 0;
             for (int k = 0; k < TREE_BLOCK / 32; k++) { const int c = wo[arr][l][k]; wo[arr][l][k] = run; run += c; }
         }
@@ -422,8 +527,11 @@ __global__ void __launch_bounds__(TREE_BLOCK) k_tree_emit(TreeView tv)
     const size_t cap = (size_t)tv.cap_node;
     const unsigned long long key = s < n ? tv.keys[s] : 0ULL;
     const int f = fm & 0xff, m = fm >> 8;
+    unsigned int q[3] = {0, 0, 0};
+    if (fm >= 0)
+        for (int k = 0; k < D; k++) q[k] = key_coord<D>(key, k);
     int prev_br = 0, prev_id = -1;
-    for (int l = 0; l <= L; l++) {
+    for (int l = 0; l <= deepest; l++) {
         bool bn, bb;
         tree_bits(fm, l, bn, bb);
         const unsigned vn = __ballot_sync(0xffffffffu, bn), vb = __ballot_sync(0xffffffffu, bb);
@@ -436,8 +544,7 @@ __global__ void __launch_bounds__(TREE_BLOCK) k_tree_emit(TreeView tv)
                 tv.start[id] = s;
                 tv.level[id] = l;
                 tv.leaf[id] = l == m ? 1 : 0;
-                for (int k = 0; k < 3; k++)
-                    tv.ix[(size_t)id * 3 + k] = k < D ? (int)(key_coord<D>(key, k, L) >> (L - l)) : 0;
+                for (int k = 0; k < 3; k++) tv.ix[(size_t)id * 3 + k] = (int)(q[k] >> (L - l));
                 tv.end[id] = br;
                 tv.parent[id] = l == 0 ? -1 : (f <= l - 1 ? prev_br : prev_br - 1);
                 tv.fchild[id] = -1;
@@ -2876,7 +2983,6 @@ public:
         keys_in_.exact(n); keys_.exact(n); idx_in_.exact(n); perm_.exact(n); xt_.exact(n);
         yp_.exact(n);
         bbox_part_.exact((size_t)BBOX_BLOCKS * (2 * D + 1));
-        delta_.exact((size_t)n + 1);
         fm_.exact(n);
         blkcnt_.exact((size_t)ceil_div(n, TREE_BLOCK) * 64);
         blkoff_.exact((size_t)ceil_div(n, TREE_BLOCK) * 64);
@@ -2933,17 +3039,26 @@ public:
             if (!tree_ok) {
                 const int nblk = ceil_div(n_, TREE_BLOCK);
                 k_bbox<D><<<BBOX_BLOCKS, 256, 0, st_>>>(n_, (const Vec<D> *)Y, bbox_part_.p, view(), done_.p);
-                k_keys<D><<<grid_for(n_, 256), 256, 0, st_>>>(n_, L, (const Vec<D> *)Y, info_.p, keys_in_.p, idx_in_.p);
-                size_t bytes = sort_bytes_;
-                TSNE_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(cub_tmp_.p, bytes, keys_in_.p, keys_.p, idx_in_.p,
-                                                                perm_.p, n_, 0, D * L, st_));
-                k_gather<D><<<grid_for(n_ + 1, 256), 256, 0, st_>>>(n_, L, perm_.p, (const Vec<D> *)Y,
-                                                                     (Vec<D> *)xt_.p, keys_.p, delta_.p);
-                k_tree_marks<D><<<nblk, TREE_BLOCK, 0, st_>>>(view());
+                if (n_ <= SORT_MOST) {
+                    const int tiles = ceil_div(n_, SORT_TILE);
+                    const bool one = tiles == 1;
+                    k_tile_sort<D><<<tiles, SORT_THREADS, 0, st_>>>(n_, L, (const Vec<D> *)Y, info_.p,
+                                                                    one ? keys_.p : keys_in_.p, one ? perm_.p : idx_in_.p);
+                    if (!one)
+                        k_tile_rank<<<ceil_div(n_, 256), 256, 0, st_>>>(n_, keys_in_.p, idx_in_.p, keys_.p, perm_.p);
+                    launches_ += 2;
+                } else {
+                    k_keys<D><<<grid_for(n_, 256), 256, 0, st_>>>(n_, L, (const Vec<D> *)Y, info_.p, keys_in_.p, idx_in_.p);
+                    size_t bytes = sort_bytes_;
+                    TSNE_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(cub_tmp_.p, bytes, keys_in_.p, keys_.p, idx_in_.p,
+                                                                    perm_.p, n_, 0, D * L, st_));
+                    launches_ += 1 + 4;
+                }
+                k_tree_marks<D><<<nblk, TREE_BLOCK, 0, st_>>>(view(), perm_.p, (const Vec<D> *)Y, xt_.p);
                 k_tree_scan<<<64, TREE_SCAN_THREADS, 0, st_>>>(nblk, view());
                 k_tree_emit<D><<<nblk, TREE_BLOCK, 0, st_>>>(view());
                 k_tree_finish<D><<<grid_for(cap_node_, 256, 148 * 8), 256, 0, st_>>>(view());
-                launches_ += 8 + 4;
+                launches_ += 5;
                 tree_ok = true;
             }
             launch_list_counts();
@@ -3424,7 +3539,7 @@ private:
         v.n = n_; v.L = Dim<D>::L; v.leaf_size = leaf_size_; v.cap_node = cap_node_; v.nset_cap = nset_cap_;
         v.keys = keys_.p; v.start = start_.p; v.end = end_.p; v.level = level_.p; v.parent = parent_.p;
         v.fchild = fchild_.p; v.nchild = nchild_.p; v.leaf = leaf_.p; v.ix = ix_.p; v.rec = rec_.p; v.proxies = proxies_.p;
-        v.delta = delta_.p; v.fm = fm_.p; v.blkcnt = blkcnt_.p; v.blkoff = blkoff_.p;
+        v.fm = fm_.p; v.blkcnt = blkcnt_.p; v.blkoff = blkoff_.p;
         v.bset = bset_.p; v.nid = nid_.p; v.btot = btot_.p; v.tickets = tickets_.p;
         v.info = info_.p;
         return v;
@@ -3576,7 +3691,6 @@ private:
     DevBuf<TreeInfo> info_;
     HostPinned<TreeInfo> hinfo_;
     DevBuf<int> start_, end_, level_, parent_, fchild_, nchild_, leaf_, ix_;
-    DevBuf<signed char> delta_;
     DevBuf<int> fm_, blkcnt_, blkoff_, bset_, nid_, btot_;
     DevBuf<int> flag_, tickets_;  // dependency-ordered launches
     DevBuf<int> done_;            // finished blocks of the bounding-box launch

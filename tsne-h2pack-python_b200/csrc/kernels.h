@@ -48,20 +48,21 @@ struct AttrRows {
 };
 constexpr int ATTR_RANGE_TABLE = 148 * 6 + 1;
 void launch_attr_ranges(cudaStream_t st, int n, const int *rp, int *ranges);
+// (returns the number of partial sums it leaves in `partials` for launch_center)
 template <int D>
-void launch_attr_update(cudaStream_t st, int n, const AttrRows &rows, const int *col, const float *val,
-                        const void *Y, void *Ynext, void *uY, void *gains, const void *rep,
-                        const int *rep_flag, float exag4, float mom, float lr, double *partials);
+int launch_attr_update(cudaStream_t st, int n, const AttrRows &rows, const int *col, const float *val,
+                       const void *Y, void *Ynext, void *uY, void *gains, const void *rep,
+                       const int *rep_flag, float exag4, float mom, float lr, double *partials);
 // the attractive sums alone (into attr), and the update from them (same bits as the fused step)
 template <int D>
 void launch_attr_grad(cudaStream_t st, int n, const AttrRows &rows, const int *col, const float *val, const void *Y,
                       void *attr);
 template <int D>
-void launch_update(cudaStream_t st, int n, const AttrRows &rows, const void *Y, void *Ynext, void *uY, void *gains,
-                   const void *rep, const int *rep_flag, const void *attr, float exag4, float mom, float lr,
-                   double *partials);
+int launch_update(cudaStream_t st, int n, const AttrRows &rows, const void *Y, void *Ynext, void *uY, void *gains,
+                  const void *rep, const int *rep_flag, const void *attr, float exag4, float mom, float lr,
+                  double *partials);
 template <int D>
-void launch_center(cudaStream_t st, int n, const AttrRows &rows, const void *Ynext, void *Ycur, const double *partials,
+void launch_center(cudaStream_t st, int n, const void *Ynext, void *Ycur, const double *partials, int n_partial,
                    DevScalars *sc);
 template <int D>
 void launch_exact_sv(cudaStream_t st, int n, const void *Y, float4 *sv);
