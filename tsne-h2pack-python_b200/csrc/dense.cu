@@ -354,6 +354,7 @@ k_update_rows(int n, const Vec<D> *__restrict__ Y, Vec<D> *__restrict__ Yn, Vec<
               Vec<D> *__restrict__ gains, const Vec<D> *__restrict__ rep, const int *__restrict__ rep_flag,
               const Vec<D> *__restrict__ attr, float exag4, float mom, float lr, double *__restrict__ partials)
 {
+    after_previous();
     const int use_rep = rep != nullptr ? *rep_flag : 0;
     double acc[D];
 #pragma unroll
@@ -755,6 +756,7 @@ k_attr_window(int n, const int *__restrict__ ranges, const int *__restrict__ rp,
               const int *__restrict__ rep_flag, float exag4, float mom, float lr, double *__restrict__ partials,
               Vec<D> *__restrict__ attr)
 {
+    after_previous();
     static_assert(MODE != ATTR_UPDATE, "the update of a rebuild iteration is k_update_rows");
     constexpr int WIN = win_pts<D>();
     constexpr int NHC = WIN_THREADS >> 4;   // half-warps per CTA
@@ -896,6 +898,7 @@ __global__ void __launch_bounds__(RED_BLOCK)
 k_center(int n, const Vec<D> *__restrict__ Yn, Vec<D> *__restrict__ Y, const double *__restrict__ partials,
          int nblk, DevScalars *sc)
 {
+    after_previous();
     __shared__ double mean[D];
     reduce_partials<D>(partials, nblk, mean);
     if (threadIdx.x == 0) {
@@ -939,6 +942,7 @@ template <int D>
 __global__ void __launch_bounds__(32 * EXACT_WARPS)
 k_exact_sv(int n, const Vec<D> *__restrict__ Y, float4 *__restrict__ sv)
 {
+    after_previous();
     __shared__ Vec<D> sh[EXACT_WARPS][EXACT_TILE];
     __shared__ float part[2][D + 1][EXACT_WARPS][32];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -988,6 +992,7 @@ template <int D>
 __global__ void __launch_bounds__(RED_BLOCK)
 k_z_part(int n, const Vec<D> *__restrict__ Yp, const float4 *__restrict__ sv, double *__restrict__ partials)
 {
+    after_previous();
     double t[3] = {0.0, 0.0, 0.0};
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const Vec<D> y = Yp[i];
@@ -1023,6 +1028,7 @@ __global__ void __launch_bounds__(RED_BLOCK)
 k_force(int n, const Vec<D> *__restrict__ Yp, const float4 *__restrict__ sv, const int *__restrict__ perm,
         Vec<D> *__restrict__ F, DevScalars *sc, const double *__restrict__ partials, int nblk, int h2_path, int keep_rep)
 {
+    after_previous();
     __shared__ double tz[3];
     reduce_partials<3>(partials, nblk, tz);
     const double Z = tz[0] + 2.0 * tz[1] - 2.0 * tz[2];
@@ -1331,8 +1337,7 @@ void launch_attr_any(cudaStream_t st, int n, const AttrRows &rows, const int *co
             constexpr size_t smem = sizeof(Vec<D>) * (size_t)win_pts<D>();
             TSNE_CUDA_CHECK(cudaFuncSetAttribute(k_attr_window<D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)smem));
-            k_attr_window<D, MODE><<<WIN_GRID, WIN_THREADS, smem, st>>>(
-                n, rows.ranges, rows.rp, col, val, (const Vec<D> *)Y, (Vec<D> *)Ynext, (Vec<D> *)uY, (Vec<D> *)gains,
+            launch_early(k_attr_window<D, MODE>, WIN_GRID, WIN_THREADS, smem, st, n, rows.ranges, rows.rp, col, val, (const Vec<D> *)Y, (Vec<D> *)Ynext, (Vec<D> *)uY, (Vec<D> *)gains,
                 (const Vec<D> *)rep, rep_flag, exag4, mom, lr, partials, (Vec<D> *)attr);
             return;
         }
@@ -1371,8 +1376,7 @@ int launch_update(cudaStream_t st, int n, const AttrRows &rows, const void *Y, v
     if (window || attr_pipe<D>() != 0) {
         // the window form's rows are a thread each here: as many CTAs as rows fill, up to six per SM
         const int blocks = window ? std::min(ATTR_PIPE3_GRID, ceil_div(n, ROW_BLOCK)) : attr_blocks<D>(n, rows);
-        k_update_rows<D><<<blocks, ROW_BLOCK, 0, st>>>(
-            n, (const Vec<D> *)Y, (Vec<D> *)Ynext, (Vec<D> *)uY, (Vec<D> *)gains, (const Vec<D> *)rep, rep_flag,
+        launch_early(k_update_rows<D>, blocks, ROW_BLOCK, 0, st, n, (const Vec<D> *)Y, (Vec<D> *)Ynext, (Vec<D> *)uY, (Vec<D> *)gains, (const Vec<D> *)rep, rep_flag,
             (const Vec<D> *)attr, exag4, mom, lr, partials);
         return blocks;
     }
@@ -1389,13 +1393,13 @@ template <int D>
 void launch_center(cudaStream_t st, int n, const void *Ynext, void *Ycur, const double *partials, int n_partial,
                    DevScalars *sc)
 {
-    k_center<D><<<ew_grid(n), RED_BLOCK, 0, st>>>(n, (const Vec<D> *)Ynext, (Vec<D> *)Ycur, partials, n_partial, sc);
+    launch_early(k_center<D>, ew_grid(n), RED_BLOCK, 0, st, n, (const Vec<D> *)Ynext, (Vec<D> *)Ycur, partials, n_partial, sc);
 }
 
 template <int D>
 void launch_exact_sv(cudaStream_t st, int n, const void *Y, float4 *sv)
 {
-    k_exact_sv<D><<<ceil_div(n, 32), 32 * EXACT_WARPS, 0, st>>>(n, (const Vec<D> *)Y, sv);
+    launch_early(k_exact_sv<D>, ceil_div(n, 32), 32 * EXACT_WARPS, 0, st, n, (const Vec<D> *)Y, sv);
 }
 
 template <int D>
@@ -1404,8 +1408,8 @@ void launch_z_force(cudaStream_t st, int n, const void *Ypts, const float4 *sv,
                     int keep_rep)
 {
     const int nblk = 148 * 2;
-    k_z_part<D><<<nblk, RED_BLOCK, 0, st>>>(n, (const Vec<D> *)Ypts, sv, partials);
-    k_force<D><<<ew_grid(n), RED_BLOCK, 0, st>>>(n, (const Vec<D> *)Ypts, sv, perm, (Vec<D> *)rep, sc, partials, nblk, h2_path, keep_rep);
+    launch_early(k_z_part<D>, nblk, RED_BLOCK, 0, st, n, (const Vec<D> *)Ypts, sv, partials);
+    launch_early(k_force<D>, ew_grid(n), RED_BLOCK, 0, st, n, (const Vec<D> *)Ypts, sv, perm, (Vec<D> *)rep, sc, partials, nblk, h2_path, keep_rep);
 }
 
 template <int D>

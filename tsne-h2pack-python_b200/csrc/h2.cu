@@ -80,6 +80,7 @@ template <int D>
 __global__ void __launch_bounds__(256) k_bbox(int n, const Vec<D> *__restrict__ Y, double *__restrict__ part,
                                               TreeView tv, int *__restrict__ done)
 {
+    after_previous();
     float lo[D], hi[D];
     int bad = 0;
     for (int k = 0; k < D; k++) { lo[k] = INFINITY; hi[k] = -INFINITY; }
@@ -211,6 +212,7 @@ template <int D>
 __global__ void k_keys(int n, int L, const Vec<D> *__restrict__ Y, const TreeInfo *__restrict__ info,
                        unsigned long long *__restrict__ keys, int *__restrict__ idx)
 {
+    after_previous();
     const KeyMaker<D> km(info, L);
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         keys[i] = km.key(Y[i], L);
@@ -237,6 +239,7 @@ __global__ void __launch_bounds__(SORT_THREADS)
 k_tile_sort(int n, int L, const Vec<D> *__restrict__ Y, const TreeInfo *__restrict__ info,
             unsigned long long *__restrict__ keys, int *__restrict__ idx)
 {
+    after_previous();
     using Sort = cub::BlockMergeSort<unsigned long long, SORT_THREADS, SORT_ITEMS, int>;
     __shared__ typename Sort::TempStorage tmp;
     const KeyMaker<D> km(info, L);
@@ -261,6 +264,7 @@ __global__ void __launch_bounds__(256) k_tile_rank(int n, const unsigned long lo
                                                    const int *__restrict__ ti, unsigned long long *__restrict__ keys,
                                                    int *__restrict__ perm)
 {
+    after_previous();
     const int i = blockIdx.x * 256 + threadIdx.x;
     if (i >= n) return;
     const unsigned long long k = tk[i];
@@ -356,6 +360,7 @@ template <int D>
 __global__ void __launch_bounds__(TREE_BLOCK) k_tree_marks(TreeView tv, const int *__restrict__ perm,
                                                            const Vec<D> *__restrict__ Y, Vec<D> *__restrict__ xt)
 {
+    after_previous();
     __shared__ int wc[2][32][TREE_BLOCK / 32];
     __shared__ int s_max[TREE_BLOCK / 32];
     __shared__ unsigned long long sk[TREE_BLOCK + 2 * TREE_HALO];
@@ -430,6 +435,7 @@ constexpr int TREE_SCAN_THREADS = 1024;
 
 __global__ void __launch_bounds__(TREE_SCAN_THREADS) k_tree_scan(int nblk, TreeView tv)
 {
+    after_previous();
     __shared__ int wsum[TREE_SCAN_THREADS / 32];
     const int col = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
     const int per = (nblk + TREE_SCAN_THREADS - 1) / TREE_SCAN_THREADS;
@@ -473,6 +479,7 @@ __global__ void __launch_bounds__(TREE_SCAN_THREADS) k_tree_scan(int nblk, TreeV
 template <int D>
 __global__ void __launch_bounds__(TREE_BLOCK) k_tree_emit(TreeView tv)
 {
+    after_previous();
     __shared__ int wo[2][32][TREE_BLOCK / 32];
     __shared__ int sboff[2][32], slb[32], s_over, s_deep;
     const int n = tv.n, L = tv.L;
@@ -652,6 +659,7 @@ __device__ __forceinline__ void proxy_table(int l, double radius, float4 *table)
 template <int D>
 __global__ void k_tree_finish(TreeView tv)
 {
+    after_previous();
     TreeInfo *info = tv.info;
     if (info->pad[0]) return;
     for (int l = blockIdx.x; l <= tv.L; l += gridDim.x) proxy_table<D>(l, info->radius, tv.proxies);
@@ -740,6 +748,7 @@ __device__ __forceinline__ void dep_publish_y0(const DepArgs &dp, int node)
 // one bounded wait for `node` (the failure path of the dependency-ordered launches, for tests)
 __global__ void k_dep_probe(DepArgs dp, int node)
 {
+    after_previous();
     if (threadIdx.x == 0) dep_wait(dp, node);
 }
 
@@ -805,6 +814,7 @@ __device__ void descend(const TreeView &tv, ListOut &lo, int t, const NodeRec &r
 template <int D>
 __global__ void __launch_bounds__(128) k_lists_write(int n_node, TreeView tv, ListOut lo)
 {
+    after_previous();
     for (int t = blockIdx.x * blockDim.x + threadIdx.x; t < n_node; t += gridDim.x * blockDim.x) {
         const NodeRec rt = node_rec(tv, t);
         int fc = 0, nc = 0;
@@ -859,6 +869,7 @@ template <int D> constexpr int list_stack() { return 1024 + 32 * (1 << D); }
 template <int D>
 __global__ void __launch_bounds__(32 * LIST_WARPS) k_lists(TreeView tv, ListOut lo, DepArgs dp)
 {
+    after_previous();
     constexpr int NCH = 1 << D, G = 32 / NCH, FS = far_slots(D);
     __shared__ int stack_[LIST_WARPS][list_stack<D>()];
     int *stack = stack_[threadIdx.x >> 5];
@@ -985,6 +996,7 @@ __device__ __forceinline__ void warp_copy_sorted(const int *slot, int cnt, int *
 template <int D>
 __global__ void __launch_bounds__(256) k_lists_compact(TreeView tv, ListOut lo)
 {
+    after_previous();
     constexpr int FS = far_slots(D);
     __shared__ int stage_[8][FS > NEAR_SLOTS ? FS : NEAR_SLOTS];
     const int n_node = tv.info->n_node;
@@ -1098,6 +1110,7 @@ __device__ __forceinline__ NodeSums node_block_scan(NodeSums x, NodeSums *sh, No
 template <int D>
 __global__ void __launch_bounds__(NODE_BLOCK) k_node_sums(TreeView tv, NodeScan q)
 {
+    after_previous();
     __shared__ NodeSums sh[32];
     const int n_node = tv.info->n_node, t = blockIdx.x * NODE_BLOCK + threadIdx.x;
     if (blockIdx.x * NODE_BLOCK >= n_node) return;
@@ -1109,6 +1122,7 @@ __global__ void __launch_bounds__(NODE_BLOCK) k_node_sums(TreeView tv, NodeScan 
 template <int D>
 __global__ void __launch_bounds__(NODE_BLOCK) k_node_scan(TreeView tv, NodeScan q)
 {
+    after_previous();
     __shared__ NodeSums sh[32];
     TreeInfo *info = tv.info;
     const int n_node = info->n_node, t = blockIdx.x * NODE_BLOCK + threadIdx.x;
@@ -1229,6 +1243,7 @@ template <int D, bool LEAVES>
 __global__ void __launch_bounds__(IDG_THREADS) k_id(int level, IdArgs g, int n_item, const int *__restrict__ items,
                                                     DepArgs dp)
 {
+    after_previous();
     constexpr int P = Dim<D>::NPROXY, PP = P + 1, MAXR = Dim<D>::MAXR, NCH = 1 << D;
     extern __shared__ __align__(16) unsigned char smraw[];
     const TreeView &tv = g.tv;
@@ -1518,6 +1533,7 @@ template <bool LEAVES, int THREADS, int NS>
 __global__ void __launch_bounds__(THREADS, id2_min_blocks<LEAVES, THREADS, NS>())
 k_id2d(int n_item, const int *__restrict__ items, LeafItems leaves, IdArgs g, DepArgs dp)
 {
+    after_previous();
     constexpr int P = Dim<2>::NPROXY, MAXR = Dim<2>::MAXR, NW = THREADS / 32;
     constexpr int PAIRS = THREADS / 2, HELD = PAIRS * NS, E = P / 4;
     constexpr int ROWS = LEAVES ? HELD : 4 * MAXR;   // candidate rows a CTA can hold
@@ -2083,6 +2099,7 @@ template <bool LEAVES, int THREADS, int ROWS>
 __global__ void __launch_bounds__(THREADS, id3_min_blocks<THREADS>())
 k_id3(int n_item, const int *__restrict__ items, int mlo, int chains, IdArgs g, DepArgs dp)
 {
+    after_previous();
     using K = Id3<THREADS, ROWS>;
     using SM = typename K::Smem;
     constexpr int P = ID3_P, MAXR = Dim<3>::MAXR, QR = K::QR, CS = K::CS, NW = K::NW, NK = K::NK;
@@ -2445,6 +2462,7 @@ __device__ __forceinline__ float4 input_at(const ProdArgs &g, const typename Dim
 template <int D>
 __global__ void __launch_bounds__(256) k_up(int level, ProdArgs g)
 {
+    after_previous();
     constexpr int MAXR = Dim<D>::MAXR;
     const TreeView &tv = g.tv;
     const Vec<D> *xt = (const Vec<D> *)g.xt;
@@ -2592,6 +2610,7 @@ constexpr int far_halves(int d) { return (d == 2 ? MAX_RANK_2D : MAX_RANK_3D) / 
 template <int D>
 __global__ void __launch_bounds__(32 * FAR_WARPS) k_far_c(int first, int n_node, ProdArgs g)
 {
+    after_previous();
     constexpr int MAXR = Dim<D>::MAXR, HALVES = far_halves(D);
     __shared__ SrcBuf<D> bufs[FAR_WARPS];
     const TreeView &tv = g.tv;
@@ -2658,6 +2677,7 @@ constexpr int NEAR_ALL = 0, NEAR_BLOCKS = 1;
 template <int D, int NC, int PART = NEAR_ALL>
 __global__ void __launch_bounds__(NEAR_THREADS) k_near(ProdArgs g)
 {
+    after_previous();
     constexpr int MAXR = Dim<D>::MAXR;
     const TreeView &tv = g.tv;
     const int t = blockIdx.x;
@@ -2725,6 +2745,7 @@ constexpr int NEAR2_TILE = 2 * NEAR2_THREADS;
 template <int PART = NEAR_ALL>
 __global__ void __launch_bounds__(NEAR2_THREADS) k_near2d(ProdArgs g)
 {
+    after_previous();
     constexpr int MAXR = Dim<2>::MAXR;
     const TreeView &tv = g.tv;
     const int t = blockIdx.x;
@@ -2820,6 +2841,7 @@ __global__ void __launch_bounds__(NEAR2_THREADS) k_near2d(ProdArgs g)
 template <int D>
 __global__ void __launch_bounds__(32 * FAR_WARPS) k_fine(const int *__restrict__ items, ProdArgs g)
 {
+    after_previous();
     __shared__ SrcBuf<D> bufs[FAR_WARPS];
     const TreeView &tv = g.tv;
     const Vec<D> *xt = (const Vec<D> *)g.xt;
@@ -2916,6 +2938,7 @@ template <int D>
 __global__ void __launch_bounds__(256) k_down_internal(int n_item, const int *__restrict__ items, ProdArgs g,
                                                         DepArgs dp)
 {
+    after_previous();
     __shared__ float4 sy[256 / 32][Dim<D>::MAXR];
     const int lane = threadIdx.x & 31;
     for (;;) {
@@ -2937,6 +2960,7 @@ __global__ void __launch_bounds__(256) k_down_internal(int n_item, const int *__
 template <int D>
 __global__ void __launch_bounds__(256) k_down_leaves(ProdArgs g)
 {
+    after_previous();
     __shared__ float4 sy[256 / 32][Dim<D>::MAXR];
     const TreeView &tv = g.tv;
     const int lb = tv.info->level_begin[MIN_ADM_LEVEL];
@@ -3038,26 +3062,26 @@ public:
         for (int attempt = 0; attempt < 12; attempt++) {
             if (!tree_ok) {
                 const int nblk = ceil_div(n_, TREE_BLOCK);
-                k_bbox<D><<<BBOX_BLOCKS, 256, 0, st_>>>(n_, (const Vec<D> *)Y, bbox_part_.p, view(), done_.p);
+                launch_early(k_bbox<D>, BBOX_BLOCKS, 256, 0, st_, n_, (const Vec<D> *)Y, bbox_part_.p, view(), done_.p);
                 if (n_ <= SORT_MOST) {
                     const int tiles = ceil_div(n_, SORT_TILE);
                     const bool one = tiles == 1;
-                    k_tile_sort<D><<<tiles, SORT_THREADS, 0, st_>>>(n_, L, (const Vec<D> *)Y, info_.p,
+                    launch_early(k_tile_sort<D>, tiles, SORT_THREADS, 0, st_, n_, L, (const Vec<D> *)Y, info_.p,
                                                                     one ? keys_.p : keys_in_.p, one ? perm_.p : idx_in_.p);
                     if (!one)
-                        k_tile_rank<<<ceil_div(n_, 256), 256, 0, st_>>>(n_, keys_in_.p, idx_in_.p, keys_.p, perm_.p);
+                        launch_early(k_tile_rank, ceil_div(n_, 256), 256, 0, st_, n_, keys_in_.p, idx_in_.p, keys_.p, perm_.p);
                     launches_ += 2;
                 } else {
-                    k_keys<D><<<grid_for(n_, 256), 256, 0, st_>>>(n_, L, (const Vec<D> *)Y, info_.p, keys_in_.p, idx_in_.p);
+                    launch_early(k_keys<D>, grid_for(n_, 256), 256, 0, st_, n_, L, (const Vec<D> *)Y, info_.p, keys_in_.p, idx_in_.p);
                     size_t bytes = sort_bytes_;
                     TSNE_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(cub_tmp_.p, bytes, keys_in_.p, keys_.p, idx_in_.p,
                                                                     perm_.p, n_, 0, D * L, st_));
                     launches_ += 1 + 4;
                 }
-                k_tree_marks<D><<<nblk, TREE_BLOCK, 0, st_>>>(view(), perm_.p, (const Vec<D> *)Y, xt_.p);
-                k_tree_scan<<<64, TREE_SCAN_THREADS, 0, st_>>>(nblk, view());
-                k_tree_emit<D><<<nblk, TREE_BLOCK, 0, st_>>>(view());
-                k_tree_finish<D><<<grid_for(cap_node_, 256, 148 * 8), 256, 0, st_>>>(view());
+                launch_early(k_tree_marks<D>, nblk, TREE_BLOCK, 0, st_, view(), perm_.p, (const Vec<D> *)Y, xt_.p);
+                launch_early(k_tree_scan, 64, TREE_SCAN_THREADS, 0, st_, nblk, view());
+                launch_early(k_tree_emit<D>, nblk, TREE_BLOCK, 0, st_, view());
+                launch_early(k_tree_finish<D>, grid_for(cap_node_, 256, 148 * 8), 256, 0, st_, view());
                 launches_ += 5;
                 tree_ok = true;
             }
@@ -3128,9 +3152,9 @@ public:
             TSNE_CUDA_CHECK(cudaStreamWaitEvent(st2_, fork_ev_, 0));
             cudaEvent_t t_lists = mark_begin(st2_);
             if (!slot_over) {
-                k_lists_compact<D><<<grid_for((long long)n_node_ * 32, 256, 148 * 8), 256, 0, st2_>>>(view(), list_out());
+                launch_early(k_lists_compact<D>, grid_for((long long)n_node_ * 32, 256, 148 * 8), 256, 0, st2_, view(), list_out());
             } else {
-                k_lists_write<D><<<grid_for(n_node_, 128, 148 * 8), 128, 0, st2_>>>(n_node_, view(), list_out());
+                launch_early(k_lists_write<D>, grid_for(n_node_, 128, 148 * 8), 128, 0, st2_, n_node_, view(), list_out());
                 if (D == 3) {
                     sort_segments(far_idx_, far_alt_, htot_[0], far_ptr_.p, st2_);
                     sort_segments(near_idx_, near_alt_, htot_[1], near_ptr_.p, st2_);
@@ -3216,7 +3240,7 @@ public:
                 if (hbig_ > 0) id3_launch<true, 256, ID3_SMALL>(hbig_, blist_.p, ID3_TINY, 256, il, dp);
                 if (hleaf_ > 0) id3_launch<true, 128, ID3_TINY>(hleaf_, llist_.p, 0, 128, il, dp);
             } else {
-                k_id<D, true><<<n_node_ - first, IDG_THREADS, id_smem_bytes<D>(mleaf), st_>>>(MIN_ADM_LEVEL, il, 0,
+                launch_early(k_id<D, true>, n_node_ - first, IDG_THREADS, id_smem_bytes<D>(mleaf), st_, MIN_ADM_LEVEL, il, 0,
                                                                                               nullptr, dp);
                 launches_++;
             }
@@ -3237,7 +3261,7 @@ public:
             rank_stats_valid_ = false;
             return 0;
         }
-        k_id<D, true><<<n_node_ - first, IDG_THREADS, id_smem_bytes<D>(mleaf), st_>>>(MIN_ADM_LEVEL, il, 0, nullptr, dp);
+        launch_early(k_id<D, true>, n_node_ - first, IDG_THREADS, id_smem_bytes<D>(mleaf), st_, MIN_ADM_LEVEL, il, 0, nullptr, dp);
         launches_++;
         mark_end(t_bases, 2);
         t_bases = mark_begin();
@@ -3246,7 +3270,7 @@ public:
         IdArgs ia = il;
         ia.mcap = mcap;
         if (hint_ > 0) {
-            k_id<D, false><<<hint_, IDG_THREADS, id_smem_bytes<D>(mcap), st_>>>(0, ia, hint_, ilist_.p, dp);
+            launch_early(k_id<D, false>, hint_, IDG_THREADS, id_smem_bytes<D>(mcap), st_, 0, ia, hint_, ilist_.p, dp);
             launches_++;
         }
         mark_end(t_bases, 7);
@@ -3263,13 +3287,12 @@ public:
     void launch_list_counts()
     {
         DepArgs dp{flag_.p, tickets_.p + TICKET_LISTS, &info_.p->pad[1], ++epoch_};
-        k_lists<D><<<std::min(148 * LIST_CTAS, ceil_div(cap_node_, LIST_WARPS)), 32 * LIST_WARPS, 0, st_>>>(
-            view(), list_out(), dp);
+        launch_early(k_lists<D>, std::min(148 * LIST_CTAS, ceil_div(cap_node_, LIST_WARPS)), 32 * LIST_WARPS, 0, st_, view(), list_out(), dp);
         const NodeScan q{far_cnt_.p, near_cnt_.p, fine_cnt_.p, far_ptr_.p, near_ptr_.p, rowoff_.p, ilist_.p, llist_.p,
                          blist_.p, clist_.p, flist_.p, rank_.p, node_blk_.p};
         const int nb = ceil_div(cap_node_, NODE_BLOCK);
-        k_node_sums<D><<<nb, NODE_BLOCK, 0, st_>>>(view(), q);
-        k_node_scan<D><<<nb, NODE_BLOCK, 0, st_>>>(view(), q);
+        launch_early(k_node_sums<D>, nb, NODE_BLOCK, 0, st_, view(), q);
+        launch_early(k_node_scan<D>, nb, NODE_BLOCK, 0, st_, view(), q);
         launches_ += 3;
     }
 
@@ -3409,7 +3432,7 @@ public:
         if (n_node_ <= 0) return -1;
         // an epoch that no launch has published: the wait runs out after `polls` polls
         DepArgs dp{flag_.p, tickets_.p, &info_.p->pad[1], epoch_ + (1 << 24), polls};
-        k_dep_probe<<<1, 32, 0, st_>>>(dp, 0);
+        launch_early(k_dep_probe, 1, 32, 0, st_, dp, 0);
         launches_++;
         return wait_failed();
     }
@@ -3493,7 +3516,7 @@ private:
     void id2_launch(int n_item, const int *items, const LeafItems &leaves, const IdArgs &a, const DepArgs &dp,
                     int ctas = 0)
     {
-        k_id2d<LEAVES, THREADS, NS><<<ctas > 0 ? ctas : n_item, THREADS, id2_smem<THREADS, NS>(), st_>>>(n_item, items,
+        launch_early(k_id2d<LEAVES, THREADS, NS>, ctas > 0 ? ctas : n_item, THREADS, id2_smem<THREADS, NS>(), st_, n_item, items,
                                                                                                          leaves, a, dp);
         launches_++;
     }
@@ -3506,7 +3529,7 @@ private:
     template <bool LEAVES, int THREADS, int ROWS>
     void id3_launch(int n_item, const int *items, int mlo, int chains, const IdArgs &a, const DepArgs &dp)
     {
-        k_id3<LEAVES, THREADS, ROWS><<<n_item, THREADS, Id3<THREADS, ROWS>::smem(), st_>>>(n_item, items, mlo, chains, a,
+        launch_early(k_id3<LEAVES, THREADS, ROWS>, n_item, THREADS, Id3<THREADS, ROWS>::smem(), st_, n_item, items, mlo, chains, a,
                                                                                            dp);
         launches_++;
     }
@@ -3592,8 +3615,8 @@ private:
     template <int PART>
     void launch_near(const ProdArgs &g, cudaStream_t st)
     {
-        if (D == 2 && g.xin == nullptr) k_near2d<PART><<<n_node_, NEAR2_THREADS, 0, st>>>(g);
-        else k_near<D, 4, PART><<<n_node_, NEAR_THREADS, 0, st>>>(g);
+        if (D == 2 && g.xin == nullptr) launch_early(k_near2d<PART>, n_node_, NEAR2_THREADS, 0, st, g);
+        else launch_early(k_near<D, 4, PART>, n_node_, NEAR_THREADS, 0, st, g);
         launches_++;
     }
     // The near blocks of the force product ([1 | Y] columns) need only the tree, the points and
@@ -3635,7 +3658,7 @@ private:
         if (xin != nullptr || !y0_from_build_) {
             for (int l = max_level_; l >= MIN_ADM_LEVEL; l--) {
                 const int nl = I.n_level_nodes[l];
-                if (nl > 0) { k_up<D><<<grid_for((long long)nl * 32, 256), 256, 0, st_>>>(l, g); launches_++; }
+                if (nl > 0) { launch_early(k_up<D>, grid_for((long long)nl * 32, 256), 256, 0, st_, l, g); launches_++; }
             }
         }
         y0_from_build_ = y0_from_build_ && xin == nullptr;
@@ -3645,13 +3668,12 @@ private:
         if (near_done && hfine_ > 0) {
             TSNE_CUDA_CHECK(cudaEventRecord(fork_ev_, st_));
             TSNE_CUDA_CHECK(cudaStreamWaitEvent(st2_, fork_ev_, 0));
-            k_fine<D><<<hfine_, 32 * FAR_WARPS, 0, st2_>>>(flist_.p, g);
+            launch_early(k_fine<D>, hfine_, 32 * FAR_WARPS, 0, st2_, flist_.p, g);
             TSNE_CUDA_CHECK(cudaEventRecord(near_ev_, st2_));
             launches_++;
         }
         cudaEvent_t t_far = mark_begin();
-        k_far_c<D><<<grid_for((long long)(n_node_ - first) * far_halves(D), FAR_WARPS, 148 * 32), 32 * FAR_WARPS, 0, st_>>>(
-            first, n_node_, g);
+        launch_early(k_far_c<D>, grid_for((long long)(n_node_ - first) * far_halves(D), FAR_WARPS, 148 * 32), 32 * FAR_WARPS, 0, st_, first, n_node_, g);
         mark_end(t_far, 3);
         launches_++;
         cudaEvent_t t_near = mark_begin();
@@ -3660,11 +3682,11 @@ private:
         cudaEvent_t t_down = mark_begin();
         if (hint_ > 0) {
             DepArgs dp{flag_.p, tickets_.p + TICKET_DOWN, &info_.p->pad[1], ++epoch_};
-            k_down_internal<D><<<grid_for((long long)hint_ * 32, 256, 148 * 8), 256, 0, st_>>>(hint_, ilist_.p, g, dp);
+            launch_early(k_down_internal<D>, grid_for((long long)hint_ * 32, 256, 148 * 8), 256, 0, st_, hint_, ilist_.p, g, dp);
             launches_++;
         }
         if (near_done) join_near();
-        k_down_leaves<D><<<grid_for((long long)(n_node_ - first) * 32, 256), 256, 0, st_>>>(g);
+        launch_early(k_down_leaves<D>, grid_for((long long)(n_node_ - first) * 32, 256), 256, 0, st_, g);
         launches_++;
         mark_end(t_down, 5);
     }
