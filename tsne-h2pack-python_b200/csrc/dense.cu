@@ -1108,22 +1108,25 @@ k_attr_only(int n, const int *__restrict__ rp, const int *__restrict__ col, cons
     }
 }
 
+// Host arrays are in the caller's order: a point's place there is ord[i] (i before a renumbering).
 template <int D>
-__global__ void k_soa_to_vec(int n, const double *__restrict__ soa, Vec<D> *__restrict__ v)
+__global__ void k_soa_to_vec(int n, const double *__restrict__ soa, Vec<D> *__restrict__ v, const int *__restrict__ ord)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const int c = ord ? ord[i] : i;
         Vec<D> o = vzero<D>();
-        for (int k = 0; k < D; k++) vset(o, k, (float)soa[(size_t)k * n + i]);
+        for (int k = 0; k < D; k++) vset(o, k, (float)soa[(size_t)k * n + c]);
         v[i] = o;
     }
 }
 
 template <int D>
-__global__ void k_vec_to_soa(int n, const Vec<D> *__restrict__ v, double *__restrict__ soa)
+__global__ void k_vec_to_soa(int n, const Vec<D> *__restrict__ v, double *__restrict__ soa, const int *__restrict__ ord)
 {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const Vec<D> x = v[i];
-        for (int k = 0; k < D; k++) soa[(size_t)k * n + i] = (double)vget(x, k);
+        const int c = ord ? ord[i] : i;
+        for (int k = 0; k < D; k++) soa[(size_t)k * n + c] = (double)vget(x, k);
     }
 }
 
@@ -1428,15 +1431,15 @@ void launch_attr_only(cudaStream_t st, int n, const int *rp, const int *col, con
 }
 
 template <int D>
-void launch_soa_to_vec(cudaStream_t st, int n, const double *soa, void *vec)
+void launch_soa_to_vec(cudaStream_t st, int n, const double *soa, void *vec, const int *ord)
 {
-    k_soa_to_vec<D><<<ew_grid(n), EW_BLOCK, 0, st>>>(n, soa, (Vec<D> *)vec);
+    k_soa_to_vec<D><<<ew_grid(n), EW_BLOCK, 0, st>>>(n, soa, (Vec<D> *)vec, ord);
 }
 
 template <int D>
-void launch_vec_to_soa(cudaStream_t st, int n, const void *vec, double *soa)
+void launch_vec_to_soa(cudaStream_t st, int n, const void *vec, double *soa, const int *ord)
 {
-    k_vec_to_soa<D><<<ew_grid(n), EW_BLOCK, 0, st>>>(n, (const Vec<D> *)vec, soa);
+    k_vec_to_soa<D><<<ew_grid(n), EW_BLOCK, 0, st>>>(n, (const Vec<D> *)vec, soa, ord);
 }
 
 template <int D>
@@ -1496,8 +1499,8 @@ void launch_pcal(cudaStream_t st, int n, const int *indptr, const double *dist, 
                                const void *, double, DevScalars *, double *);                       \
     template void launch_attr_only<D>(cudaStream_t, int, const int *, const int *, const float *,   \
                                       const void *, double, double *);                              \
-    template void launch_soa_to_vec<D>(cudaStream_t, int, const double *, void *);                  \
-    template void launch_vec_to_soa<D>(cudaStream_t, int, const void *, double *);                  \
+    template void launch_soa_to_vec<D>(cudaStream_t, int, const double *, void *, const int *);                \
+    template void launch_vec_to_soa<D>(cudaStream_t, int, const void *, double *, const int *);                \
     template void launch_fill_vec<D>(cudaStream_t, int, void *, float);                             \
     template void launch_permute_vec<D>(cudaStream_t, int, const int *, const void *, void *);
 

@@ -302,40 +302,30 @@ void pad_P(tsne_workspace *ws, const int *rp0, const int *ci0, const V *pv0)
     ws->n_launch += 4;
 }
 
-template <int D>
-void soa_to_device(tsne_workspace *ws, const double *soa_host, void *dst)
+// host SoA double -> device vec: point i of dst is point ord[i] of the host's (its own i without ord)
+void upload_soa(tsne_workspace *ws, const double *soa_host, void *dst, const int *ord = nullptr)
 {
     DevBuf<double> tmp;
-    tmp.exact((size_t)ws->n * D);
-    TSNE_CUDA_CHECK(cudaMemcpyAsync(tmp.p, soa_host, sizeof(double) * ws->n * D, cudaMemcpyHostToDevice, ws->st));
-    launch_soa_to_vec<D>(ws->st, ws->n, tmp.p, dst);
+    tmp.exact((size_t)ws->n * ws->d);
+    TSNE_CUDA_CHECK(cudaMemcpyAsync(tmp.p, soa_host, sizeof(double) * ws->n * ws->d, cudaMemcpyHostToDevice, ws->st));
+    if (ws->d == 2) launch_soa_to_vec<2>(ws->st, ws->n, tmp.p, dst, ord);
+    else launch_soa_to_vec<3>(ws->st, ws->n, tmp.p, dst, ord);
     TSNE_CUDA_CHECK(cudaStreamSynchronize(ws->st));
 }
 
-void upload_soa(tsne_workspace *ws, const double *soa_host, void *dst)
-{
-    if (ws->d == 2) soa_to_device<2>(ws, soa_host, dst);
-    else soa_to_device<3>(ws, soa_host, dst);
-}
-
-// device vec -> host SoA double, in the caller's point order
+// device vec -> host SoA double, in the caller's point order. The conversion's kernel also moves the
+// points to their places, and the copy goes straight to the caller's memory: a second host
+// array filled point by point in a random order, here and at the upload, took 24 of 28 ms at 1M points.
 void download_soa(tsne_workspace *ws, const void *src, double *out)
 {
     const int n = ws->n, d = ws->d;
+    const int *ord = ws->has_order ? ws->order.p : nullptr;
     DevBuf<double> tmp;
     tmp.exact((size_t)n * d);
-    if (d == 2) launch_vec_to_soa<2>(ws->st, n, src, tmp.p);
-    else launch_vec_to_soa<3>(ws->st, n, src, tmp.p);
-    std::vector<double> h((size_t)n * d);
-    TSNE_CUDA_CHECK(cudaMemcpyAsync(h.data(), tmp.p, sizeof(double) * n * d, cudaMemcpyDeviceToHost, ws->st));
-    std::vector<int> ord;
-    if (ws->has_order) {
-        ord.resize(n);
-        TSNE_CUDA_CHECK(cudaMemcpyAsync(ord.data(), ws->order.p, sizeof(int) * n, cudaMemcpyDeviceToHost, ws->st));
-    }
+    if (d == 2) launch_vec_to_soa<2>(ws->st, n, src, tmp.p, ord);
+    else launch_vec_to_soa<3>(ws->st, n, src, tmp.p, ord);
+    TSNE_CUDA_CHECK(cudaMemcpyAsync(out, tmp.p, sizeof(double) * n * d, cudaMemcpyDeviceToHost, ws->st));
     TSNE_CUDA_CHECK(cudaStreamSynchronize(ws->st));
-    for (int k = 0; k < d; k++)
-        for (int j = 0; j < n; j++) out[(size_t)k * n + (ws->has_order ? ord[j] : j)] = h[(size_t)k * n + j];
 }
 
 // Rebuild the H2 matrix for the current embedding (reference update_h2_matrix,
@@ -1346,6 +1336,7 @@ int tsne_h2_probe_dependency_timeout(H2Pack_p h2, int max_polls)
 int tsne_get_state(tsne_workspace_t *ws, double *Y_out, double *rep_out, double *rep_Z)
 {
     if (ws == nullptr) return -1;
+    AllocStream guard(ws->st);
     try {
         if (Y_out) download_soa(ws, ws->Y.p, Y_out);
         if (rep_out) download_soa(ws, ws->rep.p, rep_out);
@@ -1361,18 +1352,9 @@ int tsne_get_state(tsne_workspace_t *ws, double *Y_out, double *rep_out, double 
 int tsne_set_embedding(tsne_workspace_t *ws, const double *Y_in)
 {
     if (ws == nullptr || Y_in == nullptr) return -1;
+    AllocStream guard(ws->st);
     try {
-        std::vector<double> Yc((size_t)ws->n * ws->d);
-        if (ws->has_order) {
-            std::vector<int> ord(ws->n);
-            TSNE_CUDA_CHECK(cudaStreamSynchronize(ws->st));
-            TSNE_CUDA_CHECK(cudaMemcpy(ord.data(), ws->order.p, sizeof(int) * ws->n, cudaMemcpyDeviceToHost));
-            for (int k = 0; k < ws->d; k++)
-                for (int j = 0; j < ws->n; j++) Yc[(size_t)k * ws->n + j] = Y_in[(size_t)k * ws->n + ord[j]];
-        } else {
-            memcpy(Yc.data(), Y_in, sizeof(double) * Yc.size());
-        }
-        upload_soa(ws, Yc.data(), ws->Y.p);
+        upload_soa(ws, Y_in, ws->Y.p, ws->has_order ? ws->order.p : nullptr);
         const size_t vb = ws->vbytes * ws->n;
         TSNE_CUDA_CHECK(cudaMemsetAsync(ws->uY.p, 0, vb, ws->st));
         if (ws->d == 2) launch_fill_vec<2>(ws->st, ws->n, ws->gains.p, 1.0f);

@@ -77,9 +77,9 @@ template <int D>
 void launch_attr_only(cudaStream_t st, int n, const int *rp, const int *col, const float *val,
                       const void *Y, double scale, double *grad_soa);
 template <int D>
-void launch_soa_to_vec(cudaStream_t st, int n, const double *soa, void *vec);
+void launch_soa_to_vec(cudaStream_t st, int n, const double *soa, void *vec, const int *ord);
 template <int D>
-void launch_vec_to_soa(cudaStream_t st, int n, const void *vec, double *soa);
+void launch_vec_to_soa(cudaStream_t st, int n, const void *vec, double *soa, const int *ord);
 template <int D>
 void launch_fill_vec(cudaStream_t st, int n, void *vec, float value);
 template <int D>
