@@ -55,15 +55,18 @@ def data_desc(n, seed=1):
 PEAKS = ROOT / "MEASURED_PEAKS.json"
 # ncu summaries of the roofline kernel on a smaller case (the default 2D form first); the DRAM
 # traffic per algorithmic byte scales the traffic to this workload's launch
-TRAFFIC = [ROOT / "profiles" / "k_attr_update_pf_200k_full.md", ROOT / "profiles" / "k_attr_update_200k_full.md"]
+TRAFFIC = [ROOT / "profiles" / "k_attr_window_200k_full.md", ROOT / "profiles" / "k_attr_update_pf_200k_full.md", ROOT / "profiles" / "k_attr_update_200k_full.md"]
 
-# the attractive step's form (TSNE_ATTR_PIPE; default 3 in 2D, 0 in 3D), as the engine picks it
-ATTR_FORMS = {0: "k_attr_update", 1: "k_attr_update_pf<1> (next step's entries loaded ahead)",
+# the attractive step's form as the engine picks it: the window form (3D: from the first renumbering on) unless
+# TSNE_ATTR_PIPE names another or TSNE_ATTR_WINDOW=0 or TSNE_ATTR_CONTIG=0 turns it off
+ATTR_FORMS = {"window": "k_attr_window (96 KB shared-memory window of Y per SM)", 0: "k_attr_update", 1: "k_attr_update_pf<1> (next step's entries loaded ahead)",
               2: "k_attr_pair (two rows per half-warp)", 3: "k_attr_update_pf<2> (next step's columns loaded ahead)"}
 
 
 def attr_form(d):
     v = os.environ.get("TSNE_ATTR_PIPE", "")
+    if v == "" and "0" not in (os.environ.get("TSNE_ATTR_WINDOW"), os.environ.get("TSNE_ATTR_CONTIG")):
+        return "window"
     if v == "":
         return 3 if d == 2 else 0
     return int(v) if v.isdigit() and int(v) in ATTR_FORMS else 0

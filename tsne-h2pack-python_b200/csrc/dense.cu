@@ -1340,8 +1340,9 @@ void launch_attr_any(cudaStream_t st, int n, const AttrRows &rows, const int *co
             constexpr size_t smem = sizeof(Vec<D>) * (size_t)win_pts<D>();
             TSNE_CUDA_CHECK(cudaFuncSetAttribute(k_attr_window<D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  (int)smem));
-            launch_early(k_attr_window<D, MODE>, WIN_GRID, WIN_THREADS, smem, st, n, rows.ranges, rows.rp, col, val, (const Vec<D> *)Y, (Vec<D> *)Ynext, (Vec<D> *)uY, (Vec<D> *)gains,
-                (const Vec<D> *)rep, rep_flag, exag4, mom, lr, partials, (Vec<D> *)attr);
+            launch_early(k_attr_window<D, MODE>, WIN_GRID, WIN_THREADS, smem, st, n, rows.ranges, rows.rp, col,
+                val, (const Vec<D> *)Y, (Vec<D> *)Ynext, (Vec<D> *)uY, (Vec<D> *)gains, (const Vec<D> *)rep,
+                rep_flag, exag4, mom, lr, partials, (Vec<D> *)attr);
             return;
         }
     }
@@ -1379,8 +1380,9 @@ int launch_update(cudaStream_t st, int n, const AttrRows &rows, const void *Y, v
     if (window || attr_pipe<D>() != 0) {
         // the window form's rows are a thread each here: as many CTAs as rows fill, up to six per SM
         const int blocks = window ? std::min(ATTR_PIPE3_GRID, ceil_div(n, ROW_BLOCK)) : attr_blocks<D>(n, rows);
-        launch_early(k_update_rows<D>, blocks, ROW_BLOCK, 0, st, n, (const Vec<D> *)Y, (Vec<D> *)Ynext, (Vec<D> *)uY, (Vec<D> *)gains, (const Vec<D> *)rep, rep_flag,
-            (const Vec<D> *)attr, exag4, mom, lr, partials);
+        launch_early(k_update_rows<D>, blocks, ROW_BLOCK, 0, st, n, (const Vec<D> *)Y, (Vec<D> *)Ynext, (Vec<D>
+            *)uY, (Vec<D> *)gains, (const Vec<D> *)rep, rep_flag, (const Vec<D> *)attr, exag4, mom, lr,
+            partials);
         return blocks;
     }
     launch_attr_any<D, ATTR_UPDATE>(st, n, rows, nullptr, nullptr, Y, Ynext, uY, gains, rep, rep_flag, exag4, mom,
@@ -1396,7 +1398,8 @@ template <int D>
 void launch_center(cudaStream_t st, int n, const void *Ynext, void *Ycur, const double *partials, int n_partial,
                    DevScalars *sc)
 {
-    launch_early(k_center<D>, ew_grid(n), RED_BLOCK, 0, st, n, (const Vec<D> *)Ynext, (Vec<D> *)Ycur, partials, n_partial, sc);
+    launch_early(k_center<D>, ew_grid(n), RED_BLOCK, 0, st, n, (const Vec<D> *)Ynext, (Vec<D> *)Ycur, partials,
+        n_partial, sc);
 }
 
 template <int D>
@@ -1412,7 +1415,8 @@ void launch_z_force(cudaStream_t st, int n, const void *Ypts, const float4 *sv,
 {
     const int nblk = 148 * 2;
     launch_early(k_z_part<D>, nblk, RED_BLOCK, 0, st, n, (const Vec<D> *)Ypts, sv, partials);
-    launch_early(k_force<D>, ew_grid(n), RED_BLOCK, 0, st, n, (const Vec<D> *)Ypts, sv, perm, (Vec<D> *)rep, sc, partials, nblk, h2_path, keep_rep);
+    launch_early(k_force<D>, ew_grid(n), RED_BLOCK, 0, st, n, (const Vec<D> *)Ypts, sv, perm, (Vec<D> *)rep, sc,
+        partials, nblk, h2_path, keep_rep);
 }
 
 template <int D>

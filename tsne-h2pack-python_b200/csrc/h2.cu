@@ -5,18 +5,17 @@
 // which is absent from the reference checkout. This file is the engine's own design:
 //
 //   tree   : root box = bounding-box midpoint with half-width MIN_HALF_WIDTH * 2^k; 64-bit
-//            Morton keys of the points' cells at depth L; stable radix sort -> tree order;
-//            nodes split level by level (binary search of the child digit inside each node)
-//            while they hold more than leaf_size points. Nodes are numbered level by level
-//            in key order.
+//            Morton keys of the points' cells at depth L; stable sort -> tree order; every
+//            level at once from the digits that neighbouring keys share, nodes split while they
+//            hold more than leaf_size points and are numbered level by level in key order.
 //   lists  : per-target far / near partners of the symmetric dual-tree traversal, derived
-//            level by level from the parent's inadmissible-source set (NSET).
+//            from the parent's inadmissible-source set (NSET), a warp per target.
 //   bases  : for every node at level >= 2, an interpolative decomposition of K(candidates,
-//            proxy points): column-pivoted Gram-Schmidt in shared memory, one CTA per node,
-//            candidates = a leaf's points or the children's skeletons (nested bases).
-//   product: upward pass (warp per node), far field (warp per compressed target), near
-//            field (CTA per leaf, source tiles in shared memory), downward pass, then the Z
-//            identity and the force.
+//            proxy points): column-pivoted Gram-Schmidt, one CTA per node, candidates = a
+//            leaf's points or the children's skeletons (nested bases); the upward sums at its end.
+//   product: far field (warp per compressed target), finer far entries and near field (CTA
+//            per leaf, source tiles in shared memory) on a side stream, downward pass, then the
+//            Z identity and the force.
 // The CPU oracle (oracle/tsne_oracle.c) restates the same design; tree and lists agree bit
 // for bit.
 #include <cub/cub.cuh>
@@ -3062,17 +3061,20 @@ public:
         for (int attempt = 0; attempt < 12; attempt++) {
             if (!tree_ok) {
                 const int nblk = ceil_div(n_, TREE_BLOCK);
-                launch_early(k_bbox<D>, BBOX_BLOCKS, 256, 0, st_, n_, (const Vec<D> *)Y, bbox_part_.p, view(), done_.p);
+                launch_early(k_bbox<D>, BBOX_BLOCKS, 256, 0, st_, n_, (const Vec<D> *)Y, bbox_part_.p, view(),
+                    done_.p);
                 if (n_ <= SORT_MOST) {
                     const int tiles = ceil_div(n_, SORT_TILE);
                     const bool one = tiles == 1;
                     launch_early(k_tile_sort<D>, tiles, SORT_THREADS, 0, st_, n_, L, (const Vec<D> *)Y, info_.p,
-                                                                    one ? keys_.p : keys_in_.p, one ? perm_.p : idx_in_.p);
+                        one ? keys_.p : keys_in_.p, one ? perm_.p : idx_in_.p);
                     if (!one)
-                        launch_early(k_tile_rank, ceil_div(n_, 256), 256, 0, st_, n_, keys_in_.p, idx_in_.p, keys_.p, perm_.p);
+                        launch_early(k_tile_rank, ceil_div(n_, 256), 256, 0, st_, n_, keys_in_.p, idx_in_.p,
+                            keys_.p, perm_.p);
                     launches_ += 2;
                 } else {
-                    launch_early(k_keys<D>, grid_for(n_, 256), 256, 0, st_, n_, L, (const Vec<D> *)Y, info_.p, keys_in_.p, idx_in_.p);
+                    launch_early(k_keys<D>, grid_for(n_, 256), 256, 0, st_, n_, L, (const Vec<D> *)Y, info_.p,
+                        keys_in_.p, idx_in_.p);
                     size_t bytes = sort_bytes_;
                     TSNE_CUDA_CHECK(cub::DeviceRadixSort::SortPairs(cub_tmp_.p, bytes, keys_in_.p, keys_.p, idx_in_.p,
                                                                     perm_.p, n_, 0, D * L, st_));
@@ -3152,9 +3154,11 @@ public:
             TSNE_CUDA_CHECK(cudaStreamWaitEvent(st2_, fork_ev_, 0));
             cudaEvent_t t_lists = mark_begin(st2_);
             if (!slot_over) {
-                launch_early(k_lists_compact<D>, grid_for((long long)n_node_ * 32, 256, 148 * 8), 256, 0, st2_, view(), list_out());
+                launch_early(k_lists_compact<D>, grid_for((long long)n_node_ * 32, 256, 148 * 8), 256, 0, st2_,
+                    view(), list_out());
             } else {
-                launch_early(k_lists_write<D>, grid_for(n_node_, 128, 148 * 8), 128, 0, st2_, n_node_, view(), list_out());
+                launch_early(k_lists_write<D>, grid_for(n_node_, 128, 148 * 8), 128, 0, st2_, n_node_, view(),
+                    list_out());
                 if (D == 3) {
                     sort_segments(far_idx_, far_alt_, htot_[0], far_ptr_.p, st2_);
                     sort_segments(near_idx_, near_alt_, htot_[1], near_ptr_.p, st2_);
@@ -3240,8 +3244,8 @@ public:
                 if (hbig_ > 0) id3_launch<true, 256, ID3_SMALL>(hbig_, blist_.p, ID3_TINY, 256, il, dp);
                 if (hleaf_ > 0) id3_launch<true, 128, ID3_TINY>(hleaf_, llist_.p, 0, 128, il, dp);
             } else {
-                launch_early(k_id<D, true>, n_node_ - first, IDG_THREADS, id_smem_bytes<D>(mleaf), st_, MIN_ADM_LEVEL, il, 0,
-                                                                                              nullptr, dp);
+                launch_early(k_id<D, true>, n_node_ - first, IDG_THREADS, id_smem_bytes<D>(mleaf), st_,
+                    MIN_ADM_LEVEL, il, 0, nullptr, dp);
                 launches_++;
             }
             mark_end(t_bases, 2);
@@ -3261,7 +3265,8 @@ public:
             rank_stats_valid_ = false;
             return 0;
         }
-        launch_early(k_id<D, true>, n_node_ - first, IDG_THREADS, id_smem_bytes<D>(mleaf), st_, MIN_ADM_LEVEL, il, 0, nullptr, dp);
+        launch_early(k_id<D, true>, n_node_ - first, IDG_THREADS, id_smem_bytes<D>(mleaf), st_, MIN_ADM_LEVEL,
+            il, 0, nullptr, dp);
         launches_++;
         mark_end(t_bases, 2);
         t_bases = mark_begin();
@@ -3287,7 +3292,8 @@ public:
     void launch_list_counts()
     {
         DepArgs dp{flag_.p, tickets_.p + TICKET_LISTS, &info_.p->pad[1], ++epoch_};
-        launch_early(k_lists<D>, std::min(148 * LIST_CTAS, ceil_div(cap_node_, LIST_WARPS)), 32 * LIST_WARPS, 0, st_, view(), list_out(), dp);
+        launch_early(k_lists<D>, std::min(148 * LIST_CTAS, ceil_div(cap_node_, LIST_WARPS)), 32 * LIST_WARPS, 0,
+            st_, view(), list_out(), dp);
         const NodeScan q{far_cnt_.p, near_cnt_.p, fine_cnt_.p, far_ptr_.p, near_ptr_.p, rowoff_.p, ilist_.p, llist_.p,
                          blist_.p, clist_.p, flist_.p, rank_.p, node_blk_.p};
         const int nb = ceil_div(cap_node_, NODE_BLOCK);
@@ -3516,8 +3522,8 @@ private:
     void id2_launch(int n_item, const int *items, const LeafItems &leaves, const IdArgs &a, const DepArgs &dp,
                     int ctas = 0)
     {
-        launch_early(k_id2d<LEAVES, THREADS, NS>, ctas > 0 ? ctas : n_item, THREADS, id2_smem<THREADS, NS>(), st_, n_item, items,
-                                                                                                         leaves, a, dp);
+        launch_early(k_id2d<LEAVES, THREADS, NS>, ctas > 0 ? ctas : n_item, THREADS, id2_smem<THREADS, NS>(),
+            st_, n_item, items, leaves, a, dp);
         launches_++;
     }
     template <bool LEAVES, int THREADS, int ROWS>
@@ -3529,8 +3535,8 @@ private:
     template <bool LEAVES, int THREADS, int ROWS>
     void id3_launch(int n_item, const int *items, int mlo, int chains, const IdArgs &a, const DepArgs &dp)
     {
-        launch_early(k_id3<LEAVES, THREADS, ROWS>, n_item, THREADS, Id3<THREADS, ROWS>::smem(), st_, n_item, items, mlo, chains, a,
-                                                                                           dp);
+        launch_early(k_id3<LEAVES, THREADS, ROWS>, n_item, THREADS, Id3<THREADS, ROWS>::smem(), st_, n_item,
+            items, mlo, chains, a, dp);
         launches_++;
     }
 
@@ -3658,7 +3664,8 @@ private:
         if (xin != nullptr || !y0_from_build_) {
             for (int l = max_level_; l >= MIN_ADM_LEVEL; l--) {
                 const int nl = I.n_level_nodes[l];
-                if (nl > 0) { launch_early(k_up<D>, grid_for((long long)nl * 32, 256), 256, 0, st_, l, g); launches_++; }
+                if (nl > 0) { launch_early(k_up<D>, grid_for((long long)nl * 32, 256), 256, 0, st_, l, g);
+                    launches_++; }
             }
         }
         y0_from_build_ = y0_from_build_ && xin == nullptr;
@@ -3673,7 +3680,8 @@ private:
             launches_++;
         }
         cudaEvent_t t_far = mark_begin();
-        launch_early(k_far_c<D>, grid_for((long long)(n_node_ - first) * far_halves(D), FAR_WARPS, 148 * 32), 32 * FAR_WARPS, 0, st_, first, n_node_, g);
+        launch_early(k_far_c<D>, grid_for((long long)(n_node_ - first) * far_halves(D), FAR_WARPS, 148 * 32), 32
+            * FAR_WARPS, 0, st_, first, n_node_, g);
         mark_end(t_far, 3);
         launches_++;
         cudaEvent_t t_near = mark_begin();
@@ -3682,7 +3690,8 @@ private:
         cudaEvent_t t_down = mark_begin();
         if (hint_ > 0) {
             DepArgs dp{flag_.p, tickets_.p + TICKET_DOWN, &info_.p->pad[1], ++epoch_};
-            launch_early(k_down_internal<D>, grid_for((long long)hint_ * 32, 256, 148 * 8), 256, 0, st_, hint_, ilist_.p, g, dp);
+            launch_early(k_down_internal<D>, grid_for((long long)hint_ * 32, 256, 148 * 8), 256, 0, st_, hint_,
+                ilist_.p, g, dp);
             launches_++;
         }
         if (near_done) join_near();
