@@ -38,14 +38,14 @@ __device__ __forceinline__ Vec<D> vzero()
 __device__ __forceinline__ int4 ld_stream_i4(const int *p)
 {
     int4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.v4.s32 {%0, %1, %2, %3}, [%4];"
                  : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
     return v;
 }
 __device__ __forceinline__ float4 ld_stream_f4(const float *p)
 {
     float4 v;
-    asm volatile("ld.global.nc.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
+    asm volatile("ld.global.L1::no_allocate.v4.f32 {%0, %1, %2, %3}, [%4];"
                  : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
     return v;
 }
@@ -103,7 +103,7 @@ __device__ __forceinline__ void block_sum_warps(double (&v)[NV], double *out)
 
 // Fixed-order sum of `count` per-block partials (stride NV) by one block; result in sh_out.
 template <int NV>
-__device__ __forceinline__ void reduce_partials(const double *__restrict__ part, int count, double *sh_out)
+__device__ __forceinline__ void reduce_partials(const double *part, int count, double *sh_out)
 {
     __shared__ double sh[RED_BLOCK][NV];
     double acc[NV];
@@ -350,9 +350,8 @@ k_attr_update_pf(int n, const int *__restrict__ rp, const int *__restrict__ col,
 // loads; this one reads and writes every array coalesced.
 template <int D>
 __global__ void __launch_bounds__(ROW_BLOCK)
-k_update_rows(int n, const Vec<D> *__restrict__ Y, Vec<D> *__restrict__ Yn, Vec<D> *__restrict__ uY,
-              Vec<D> *__restrict__ gains, const Vec<D> *__restrict__ rep, const int *__restrict__ rep_flag,
-              const Vec<D> *__restrict__ attr, float exag4, float mom, float lr, double *__restrict__ partials)
+k_update_rows(int n, const Vec<D> *Y, Vec<D> *Yn, Vec<D> *uY, Vec<D> *gains, const Vec<D> *rep, const int *rep_flag,
+              const Vec<D> *attr, float exag4, float mom, float lr, double *partials)
 {
     after_previous();
     const int use_rep = rep != nullptr ? *rep_flag : 0;
@@ -728,12 +727,12 @@ __device__ __forceinline__ Vec<D> win_gather(unsigned win, int w0, int wl, const
     if constexpr (D == 2)
         asm volatile("{ .reg .pred p; setp.lt.u32 p, %2, %3;\n"
                      "@p ld.shared.v2.f32 {%0, %1}, [%4];\n"
-                     "@!p ld.global.nc.v2.f32 {%0, %1}, [%5]; }"
+                     "@!p ld.global.v2.f32 {%0, %1}, [%5]; }"
                      : "=f"(v.x), "=f"(v.y) : "r"(off), "r"(wl), "r"(sa), "l"(Y + c));
     else
         asm volatile("{ .reg .pred p; setp.lt.u32 p, %4, %5;\n"
                      "@p ld.shared.v4.f32 {%0, %1, %2, %3}, [%6];\n"
-                     "@!p ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%7]; }"
+                     "@!p ld.global.v4.f32 {%0, %1, %2, %3}, [%7]; }"
                      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(off), "r"(wl), "r"(sa), "l"(Y + c));
     return v;
 }
@@ -750,11 +749,9 @@ __device__ __forceinline__ void attr_acc_y(const Vec<D> &yi, const Vec<D> &yj, f
 
 template <int D, int MODE>
 __global__ void __launch_bounds__(WIN_THREADS, 1)
-k_attr_window(int n, const int *__restrict__ ranges, const int *__restrict__ rp, const int *__restrict__ col,
-              const float *__restrict__ val, const Vec<D> *__restrict__ Y, Vec<D> *__restrict__ Yn,
-              Vec<D> *__restrict__ uY, Vec<D> *__restrict__ gains, const Vec<D> *__restrict__ rep,
-              const int *__restrict__ rep_flag, float exag4, float mom, float lr, double *__restrict__ partials,
-              Vec<D> *__restrict__ attr)
+k_attr_window(int n, const int *ranges, const int *rp, const int *col, const float *val, const Vec<D> *Y, Vec<D> *Yn,
+              Vec<D> *uY, Vec<D> *gains, const Vec<D> *rep, const int *rep_flag, float exag4, float mom, float lr,
+              double *partials, Vec<D> *attr)
 {
     after_previous();
     static_assert(MODE != ATTR_UPDATE, "the update of a rebuild iteration is k_update_rows");
@@ -895,8 +892,7 @@ __global__ void k_attr_ranges(int n, const int *__restrict__ rp, int *__restrict
 // in FP64 from the update's fixed per-block partials, identically in every block.
 template <int D>
 __global__ void __launch_bounds__(RED_BLOCK)
-k_center(int n, const Vec<D> *__restrict__ Yn, Vec<D> *__restrict__ Y, const double *__restrict__ partials,
-         int nblk, DevScalars *sc)
+k_center(int n, const Vec<D> *Yn, Vec<D> *Y, const double *partials, int nblk, DevScalars *sc)
 {
     after_previous();
     __shared__ double mean[D];
@@ -940,7 +936,7 @@ __device__ __forceinline__ void exact_tile(const Vec<D> *sh, int cnt, int self, 
 }
 template <int D>
 __global__ void __launch_bounds__(32 * EXACT_WARPS)
-k_exact_sv(int n, const Vec<D> *__restrict__ Y, float4 *__restrict__ sv)
+k_exact_sv(int n, const Vec<D> *Y, float4 *sv)
 {
     after_previous();
     __shared__ Vec<D> sh[EXACT_WARPS][EXACT_TILE];
@@ -990,7 +986,7 @@ __device__ __forceinline__ float sv_v(const float4 &a, int k)
 // three FP64 sums over fixed blocks.
 template <int D>
 __global__ void __launch_bounds__(RED_BLOCK)
-k_z_part(int n, const Vec<D> *__restrict__ Yp, const float4 *__restrict__ sv, double *__restrict__ partials)
+k_z_part(int n, const Vec<D> *Yp, const float4 *sv, double *partials)
 {
     after_previous();
     double t[3] = {0.0, 0.0, 0.0};
@@ -1025,8 +1021,8 @@ k_z_part(int n, const Vec<D> *__restrict__ Yp, const float4 *__restrict__ sv, do
 // non-finite Z skips the force, as the reference does.
 template <int D>
 __global__ void __launch_bounds__(RED_BLOCK)
-k_force(int n, const Vec<D> *__restrict__ Yp, const float4 *__restrict__ sv, const int *__restrict__ perm,
-        Vec<D> *__restrict__ F, DevScalars *sc, const double *__restrict__ partials, int nblk, int h2_path, int keep_rep)
+k_force(int n, const Vec<D> *Yp, const float4 *sv, const int *perm, Vec<D> *F, DevScalars *sc, const double *partials,
+        int nblk, int h2_path, int keep_rep)
 {
     after_previous();
     __shared__ double tz[3];

@@ -76,8 +76,8 @@ __device__ void root_from_parts(int n, int nblk, const double *part, const TreeV
 // them to the root box and writes the root node (`done` counts the finished blocks and is left
 // at zero for the next launch). A second launch for the root alone cost 5 us plus its gap.
 template <int D>
-__global__ void __launch_bounds__(256) k_bbox(int n, const Vec<D> *__restrict__ Y, double *__restrict__ part,
-                                              TreeView tv, int *__restrict__ done)
+__global__ void __launch_bounds__(256) k_bbox(int n, const Vec<D> *Y, double *part, TreeView tv,
+                                              int *done)
 {
     after_previous();
     float lo[D], hi[D];
@@ -208,8 +208,7 @@ struct KeyMaker {
 };
 
 template <int D>
-__global__ void k_keys(int n, int L, const Vec<D> *__restrict__ Y, const TreeInfo *__restrict__ info,
-                       unsigned long long *__restrict__ keys, int *__restrict__ idx)
+__global__ void k_keys(int n, int L, const Vec<D> *Y, const TreeInfo *info, unsigned long long *keys, int *idx)
 {
     after_previous();
     const KeyMaker<D> km(info, L);
@@ -235,8 +234,7 @@ struct KeyLess {
 
 template <int D>
 __global__ void __launch_bounds__(SORT_THREADS)
-k_tile_sort(int n, int L, const Vec<D> *__restrict__ Y, const TreeInfo *__restrict__ info,
-            unsigned long long *__restrict__ keys, int *__restrict__ idx)
+k_tile_sort(int n, int L, const Vec<D> *Y, const TreeInfo *info, unsigned long long *keys, int *idx)
 {
     after_previous();
     using Sort = cub::BlockMergeSort<unsigned long long, SORT_THREADS, SORT_ITEMS, int>;
@@ -259,9 +257,8 @@ k_tile_sort(int n, int L, const Vec<D> *__restrict__ Y, const TreeInfo *__restri
         }
 }
 
-__global__ void __launch_bounds__(256) k_tile_rank(int n, const unsigned long long *__restrict__ tk,
-                                                   const int *__restrict__ ti, unsigned long long *__restrict__ keys,
-                                                   int *__restrict__ perm)
+__global__ void __launch_bounds__(256) k_tile_rank(int n, const unsigned long long *tk, const int *ti,
+                                                   unsigned long long *keys, int *perm)
 {
     after_previous();
     const int i = blockIdx.x * 256 + threadIdx.x;
@@ -356,8 +353,8 @@ __device__ __forceinline__ void tree_bits(int fm, int l, bool &bn, bool &bb)
 constexpr int TREE_HALO = 256;     // longest leaf_size whose keys are staged
 
 template <int D>
-__global__ void __launch_bounds__(TREE_BLOCK) k_tree_marks(TreeView tv, const int *__restrict__ perm,
-                                                           const Vec<D> *__restrict__ Y, Vec<D> *__restrict__ xt)
+__global__ void __launch_bounds__(TREE_BLOCK) k_tree_marks(TreeView tv, const int *perm, const Vec<D> *Y,
+                                                           Vec<D> *xt)
 {
     after_previous();
     __shared__ int wc[2][32][TREE_BLOCK / 32];
@@ -574,7 +571,7 @@ struct NodeRec {
 };
 __device__ __forceinline__ NodeRec node_rec(const TreeView &tv, int t)
 {
-    const int4 a = __ldg(tv.rec + 2 * (size_t)t), b = __ldg(tv.rec + 2 * (size_t)t + 1);
+    const int4 a = tv.rec[2 * (size_t)t], b = tv.rec[2 * (size_t)t + 1];
     NodeRec r;
     r.fchild = a.x;
     r.nchild = a.y & 0xff;
@@ -1239,7 +1236,7 @@ __device__ __forceinline__ void gs_rows(float *A, const float *q, int m, int tid
 // otherwise the nodes of `level` (or every leaf). Children's ranks, skeletons and coefficients
 // are read through L2.
 template <int D, bool LEAVES>
-__global__ void __launch_bounds__(IDG_THREADS) k_id(int level, IdArgs g, int n_item, const int *__restrict__ items,
+__global__ void __launch_bounds__(IDG_THREADS) k_id(int level, IdArgs g, int n_item, const int *items,
                                                     DepArgs dp)
 {
     after_previous();
@@ -1530,7 +1527,7 @@ static_assert(ID2_TINY == TINY_LEAF && ID2_SMALL == SMALL_LEAF, "the leaf lists 
 
 template <bool LEAVES, int THREADS, int NS>
 __global__ void __launch_bounds__(THREADS, id2_min_blocks<LEAVES, THREADS, NS>())
-k_id2d(int n_item, const int *__restrict__ items, LeafItems leaves, IdArgs g, DepArgs dp)
+k_id2d(int n_item, const int *items, LeafItems leaves, IdArgs g, DepArgs dp)
 {
     after_previous();
     constexpr int P = Dim<2>::NPROXY, MAXR = Dim<2>::MAXR, NW = THREADS / 32;
@@ -2096,7 +2093,7 @@ constexpr int id3_min_blocks() { return THREADS >= 512 ? 1 : (THREADS >= 256 ? 2
 // is the thread count by which S is chosen.
 template <bool LEAVES, int THREADS, int ROWS>
 __global__ void __launch_bounds__(THREADS, id3_min_blocks<THREADS>())
-k_id3(int n_item, const int *__restrict__ items, int mlo, int chains, IdArgs g, DepArgs dp)
+k_id3(int n_item, const int *items, int mlo, int chains, IdArgs g, DepArgs dp)
 {
     after_previous();
     using K = Id3<THREADS, ROWS>;
@@ -2838,7 +2835,7 @@ __global__ void __launch_bounds__(NEAR2_THREADS) k_near2d(ProdArgs g)
 // the side stream; a block per node, every thread of which walked the far list to find the finer
 // entries, took 44 / 87 / 234 us before the downward pass.
 template <int D>
-__global__ void __launch_bounds__(32 * FAR_WARPS) k_fine(const int *__restrict__ items, ProdArgs g)
+__global__ void __launch_bounds__(32 * FAR_WARPS) k_fine(const int *items, ProdArgs g)
 {
     after_previous();
     __shared__ SrcBuf<D> bufs[FAR_WARPS];
@@ -2934,7 +2931,7 @@ __device__ __forceinline__ void down_node(const ProdArgs &g, int t, int lane, fl
 // downward pass of every internal node at level >= 2 in one dependency-ordered launch
 // (persistent warps, items in increasing node id): a node waits for its parent's push
 template <int D>
-__global__ void __launch_bounds__(256) k_down_internal(int n_item, const int *__restrict__ items, ProdArgs g,
+__global__ void __launch_bounds__(256) k_down_internal(int n_item, const int *items, ProdArgs g,
                                                         DepArgs dp)
 {
     after_previous();
