@@ -31,7 +31,14 @@ def _cuda_available():
         return False
 
 
+# passes only while a job of 600 iterations at 4,000 points takes longer than the 50 ms it sleeps
+# (test_gpu_serving_overlap.py asserts the same without that premise)
+TIMING_PREMISE = ("test_job_submitted_while_running_starts_early",)
+
+
 def pytest_collection_modifyitems(config, items):
+    # run last, so that a run stopping at its first failure has run everything else
+    items.sort(key=lambda item: item.name in TIMING_PREMISE)
     if _cuda_available():
         return
     skip = pytest.mark.skip(reason="no CUDA device in this environment")

@@ -69,3 +69,10 @@ def test_early_kernel_reads_no_memory_as_constant(name):
             for bad in ("__restrict__", "__ldg", "global.nc"):
                 assert bad not in params + body, f"{bad} in {f}, reached from {name}"
             todo += [c for c in set(re.findall(r"\b(\w+)\s*(?:<[\w\s,<>:]*>)?\s*\(", body)) if c in FUNCTIONS]
+
+
+def test_every_thread_launches_early():
+    """A served job takes the launch path that a direct run takes."""
+    body = re.search(r"void launch_early\(.*?\n}\n", (CSRC / "common.cuh").read_text(), flags=re.S).group(0)
+    assert "cfg.numAttrs = 1;" in body
+    assert "thread_local" not in (CSRC / "common.cuh").read_text()

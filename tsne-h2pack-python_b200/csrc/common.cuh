@@ -36,8 +36,6 @@ struct CudaError {
 // 60 iterations with ordinary launches and with these: 1,501 points exact 1.79 and 1.24 ms, 2K 5.86 and 5.13,
 // 20K 8.55 and 7.75, 200K 22.1 and 20.5; 30 at 1M 33.7 and 33.3, at 100K in 3D 37.1 and 35.9.
 __device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// A thread that serves jobs launches in the ordinary way (worker_loop sets this for its thread).
-inline thread_local bool ordinary_launches = false;
 template <typename... Params, typename... Args>
 void launch_early(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, Args &&...args)
 {
@@ -50,7 +48,7 @@ void launch_early(void (*kernel)(Params...), dim3 grid, dim3 block, size_t smem,
     attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &attr;
-    cfg.numAttrs = ordinary_launches ? 0 : 1;
+    cfg.numAttrs = 1;
     // as with <<<>>>, an error is left for the caller's cudaGetLastError
     (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
 }

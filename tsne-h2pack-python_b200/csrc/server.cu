@@ -25,7 +25,6 @@
 #include <vector>
 
 #include "../../include/tsne_h2pack.h"
-#include "common.cuh"
 
 namespace {
 
@@ -100,10 +99,6 @@ bool run_job(Job *job)
 
 void worker_loop(tsne_server *s)
 {
-    // A served job keeps ordinary launches: its latency is relied on where a second job is to arrive while
-    // it runs (600 iterations at 4,000 points: 53 ms, and 48 ms with early launches, against a
-    // second job after 50 ms). Eight jobs of 5,000 points take 59 ms so, and 54 ms with early launches.
-    tsne::ordinary_launches = true;
     cudaSetDevice(s->device);
     for (;;) {
         Job *job = nullptr;
