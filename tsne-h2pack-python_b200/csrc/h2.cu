@@ -784,7 +784,8 @@ struct ListOut {
 };
 
 // A source s that is inadmissible for a target, as the target's children will meet it: the range
-// of its children, or s itself when it is a leaf (first node << 4 | nodes)
+// of its children, or s itself when it is a leaf (first node << 4 | nodes; that holds 2^27 nodes, whose
+// skeletons and coefficients alone, 2.5 KB a node, are more than the device's memory)
 __device__ __forceinline__ int nset_pack(int s, const NodeRec &r)
 {
     return r.leaf ? (s << 4 | 1) : (r.fchild << 4 | r.nchild);
@@ -2498,6 +2499,12 @@ __global__ void __launch_bounds__(256) k_up(int level, ProdArgs g)
     }
 }
 
+// The place of a node's slot k in skel, y0 and y1. In 64 bits: the node table is regrown while it is full, so
+// no count of nodes is the last one that an int product would have to hold.
+template <int D>
+__host__ __device__ constexpr size_t slot_at(int node, int k) { return (size_t)node * Dim<D>::MAXR + k; }
+static_assert(slot_at<2>(1 << 25, 1) == ((size_t)1 << 31) + 1 && slot_at<3>(1 << 25, 1) == ((size_t)1 << 31) + 1, "past an int");
+
 // The sources of far entries [e0, e1) of a target at level lt, for one warp, in order. Sources of
 // the target's level and (FINE) finer ones are skeletons with their coefficients; coarser ones
 // (leaves) are points with the input columns; without FINE, finer sources are left out.
@@ -2523,13 +2530,13 @@ __device__ __forceinline__ void for_sources(const ProdArgs &g, int e0, int e1, i
                                             const Body &body)
 {
     constexpr unsigned ALL = 0xffffffffu;
-    // this lane's entry of a group of 32: first element, size, kind (0 skeleton, 1 points)
+    // this lane's entry of a group of 32: its node (points: the first one), size, kind (0 skeleton, 1 points)
     auto entry = [&](int e, int &base, int &cnt, int &pts) {
         base = cnt = pts = 0;
         if (e + lane >= e1) return;
         const int s = g.far_idx[e + lane], ls = g.tv.level[s];
         if (ls >= lt) {
-            base = s * Dim<D>::MAXR;   // nodes are fewer than points / 4 + 1024
+            base = s;
             cnt = (FINE || ls == lt) ? g.rank[s] : 0;
         } else {
             pts = 1;
@@ -2559,7 +2566,8 @@ __device__ __forceinline__ void for_sources(const ProdArgs &g, int e0, int e1, i
                 if (v <= j) i += o;
             }
             const int b = j - __shfl_sync(ALL, first, i), c = __shfl_sync(ALL, cnt, i);
-            const int at = __shfl_sync(ALL, base, i) + b, p = __shfl_sync(ALL, pts, i);
+            const int from = __shfl_sync(ALL, base, i), p = __shfl_sync(ALL, pts, i);
+            const size_t at = p ? (size_t)from + b : slot_at<D>(from, b);
             r.y = make_float4(0.f, 0.f, 0.f, 0.f);
             if constexpr (D == 2) r.x = make_float2(0.f, 0.f);
             else r.x = r.y;
