@@ -3028,7 +3028,7 @@ public:
                                                         perm_.p, n, 0, D * Dim<D>::L, st_));
         sort_bytes_ = b1;
         cub_tmp_.exact(b1 + 256);
-        cap_node_ = std::max(1024, 4 * (n / 16) + 1024);
+        cap_node_ = first_cap_node(n);
         nset_cap_ = Dim<D>::NSET;
         alloc_nodes();
         TSNE_CUDA_CHECK(cudaFuncSetAttribute(k_id<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -3049,6 +3049,14 @@ public:
             id3_attr<true, 128, ID3_TINY>();
         }
     }
+
+    static int id_mcap()
+    {
+        // shared-memory rows of the ID: every internal node of the 2D tree (4 * MAXR rows)
+        // and leaves up to that size; the 3D bound keeps the CTA under 227 KB
+        return D == 2 ? (1 << D) * Dim<D>::MAXR : 240;
+    }
+    static int first_cap_node(int n) { return std::max(1024, 4 * (n / 16) + 1024); }   // regrown while it is full
 
     int build(const void *Y, int leaf_size, double tol, const std::function<void()> *overlap) override
     {
@@ -3545,13 +3553,6 @@ private:
         launches_++;
     }
 
-    static int id_mcap()
-    {
-        // shared-memory rows of the ID: every internal node of the 2D tree (4 * MAXR rows)
-        // and leaves up to that size; the 3D bound keeps the CTA under 227 KB
-        return D == 2 ? (1 << D) * Dim<D>::MAXR : 240;
-    }
-
     void alloc_nodes()
     {
         const size_t c = cap_node_;
@@ -3757,7 +3758,35 @@ private:
     DevBuf<Vec<D>> gcand_;
 };
 
+// The terms are the buffers of H2Impl. The nodes that a tree will have are taken from embeddings of uniform,
+// normal and clustered points and of runs (30K and 200K points, leaf sizes 2 to 300): at most 4.3 n / leaf_size nodes in
+// 2D and 6.5 in 3D, of them 1.13 and 0.91 internal. Tight clumps of more points than a leaf holds, each a chain
+// of nodes down to the clump's size, can have more.
+template <int D>
+size_t h2_bytes(int n, int leaf_size)
+{
+    using Impl = H2Impl<D>;
+    constexpr size_t V = sizeof(Vec<D>), MAXR = Dim<D>::MAXR, P = Dim<D>::NPROXY;
+    const double nodes = (D == 2 ? 4.5 : 6.6) * n / leaf_size, internal = (D == 2 ? 1.2 : 0.95) * n / leaf_size;
+    double cap = Impl::first_cap_node(n);
+    while (cap < nodes) cap *= 2;
+    const size_t point = 2 * (sizeof(unsigned long long) + sizeof(int)) + V + sizeof(float4) + sizeof(int) +
+                         sizeof(unsigned long long) + sizeof(int);   // (the radix sort's scratch)
+    const size_t entry = sizeof(int) * (24 + 2 * (Dim<D>::L + 1) + Dim<D>::NSET + far_slots(D) + NEAR_SLOTS) +
+                         2 * sizeof(int4) + sizeof(long long);       // of the node table and the list pass
+    const size_t node = MAXR * (V + 2 * sizeof(float4)) + sizeof(int) * 160;   // bases and list entries
+    size_t row = sizeof(float) * MAXR;                                         // of the interpolation matrices
+    if (leaf_size > (D == 2 ? Impl::id_mcap() : ID3_ROWS)) row += sizeof(float) * (P + 2) + sizeof(int) + V;
+    const double rows = n + internal * (1 << D) * MAXR;
+    return (size_t)((double)point * n + entry * cap + 1.25 * (node * nodes + row * rows));   // 1.25: DevBuf::ensure
+}
+
 }  // namespace
+
+size_t h2_device_bytes(int d, int n, int leaf_size)
+{
+    return d == 2 ? h2_bytes<2>(n, leaf_size) : h2_bytes<3>(n, leaf_size);
+}
 
 std::unique_ptr<H2Matrix> make_h2_matrix(int d, int n, cudaStream_t st)
 {

@@ -59,6 +59,10 @@ public:
     virtual void flush_timers() = 0;
 };
 
+// device bytes that the H2 matrix of n points holds at its peak (an upper estimate for embeddings as runs
+// make them: the tree is not known yet)
+size_t h2_device_bytes(int d, int n, int leaf_size);
+
 std::unique_ptr<H2Matrix> make_h2_matrix(int d, int n, cudaStream_t st);
 
 }  // namespace tsne

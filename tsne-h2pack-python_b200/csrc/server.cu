@@ -3,8 +3,8 @@
 // A server owns a pool of worker threads. Jobs (P, dimensions, parameters) are submitted at
 // any time and queue in arrival order; a worker starts the job at the head of the queue when
 // fewer than `max_concurrent` jobs run and the device memory the job needs (an upper estimate
-// from N and nnz(P)) fits under the HBM budget next to the running jobs' - or when nothing
-// runs, so that a job larger than the budget still runs, alone. Every job is a workspace of
+// from N, nnz(P), the dimensions and the leaf size) fits under the HBM budget next to the
+// running jobs' - or when nothing runs, so that a job larger than the budget still runs, alone. Every job is a workspace of
 // its own with its own CUDA stream, so the kernels of the running jobs overlap on the device,
 // and a job that arrives while others run starts as soon as a slot and memory free up
 // (continuous batching). A job's computation does not depend on what else runs: its result is
@@ -25,6 +25,7 @@
 #include <vector>
 
 #include "../../include/tsne_h2pack.h"
+#include "h2.h"
 
 namespace {
 
@@ -69,11 +70,16 @@ struct tsne_server {
 
 namespace {
 
-// device bytes a job may hold at its peak: P (padded copy, the renumbering copy and the
-// upload's temporaries), the per-point vectors, the H2 tree, lists and bases
-size_t job_bytes(int n, long long nnz)
+// device bytes a job may hold at its peak: P (padded copy, the renumbering copy and the upload's
+// temporaries), the per-point vectors, small scratch, and the H2 tree, lists and bases (below 2,000 points
+// the sums are exact). 2 KB per point for all but P, whatever the dimension and the leaf size, was less than
+// 3D jobs (2.0-2.8 KB at 100 points a leaf) and small leaves (10-14 KB at 8 points) hold.
+size_t job_bytes(int n, int d, int leaf_size, long long nnz)
 {
-    return (size_t)(32 * nnz) + (size_t)n * 2048 + (size_t(64) << 20);
+    const size_t vec = d == 2 ? sizeof(float2) : sizeof(float4);
+    const size_t point = 9 * vec + sizeof(float4) + sizeof(double) * d + 6 * sizeof(int) + 48;   // 48: P's padding
+    return (size_t)(32 * nnz) + point * n + (size_t(64) << 20) +
+           (n < 2000 ? 0 : tsne::h2_device_bytes(d, n, leaf_size > 0 ? leaf_size : 100));
 }
 
 bool run_job(Job *job)
@@ -164,7 +170,7 @@ int tsne_server_submit(tsne_server_t *s, int n_point, int low_dim, const tsne_pa
     if (params->enable_profiling && params->profiling_output_file) job->prof_file = params->profiling_output_file;
     job->params.profiling_output_file = nullptr;
     job->P = P;
-    job->bytes = job_bytes(n_point, P->row_ptr[n_point]);
+    job->bytes = job_bytes(n_point, low_dim, params->h2_leaf_size, P->row_ptr[n_point]);
     job->t_submit = now_sec();
     int id;
     {
