@@ -1261,15 +1261,20 @@ int attr_contig()
 // SM); 2 k_attr_pair (two rows per half-warp, five CTAs per SM); 3 the next step's columns
 // loaded ahead (40 registers, six CTAs per SM); 4 k_attr_stream (the column loads ahead across
 // the rows of a half-warp, five CTAs per SM). Measured at 1M points, 2D, per launch: 0.619,
-// 0.608, 0.616, 0.592 and 0.634 ms, so 2D takes form 3 by default. In 3D the fused kernel holds 48
+// 0.608, 0.616, 0.592 and 0.634 ms, so 2D takes form 3 where the window form (below) is off. In 3D the fused kernel holds 48
 // registers in every form and form 3 spills there; form 1 measured no faster than form 0 at
 // 500K points (0.352 against 0.348 ms per launch), so 3D keeps form 0. The attractive sums of a
 // rebuild iteration follow the form; their update is k_update_rows for forms 1-3.
+const char *attr_pipe_asked()   // null: unset or empty, the default
+{
+    const char *e = getenv("TSNE_ATTR_PIPE");
+    return e == nullptr || *e == '\0' ? nullptr : e;
+}
 template <int D>
 int attr_pipe()
 {
-    const char *e = getenv("TSNE_ATTR_PIPE");
-    if (e == nullptr || *e == '\0') return D == 2 ? 3 : 0;
+    const char *e = attr_pipe_asked();
+    if (e == nullptr) return D == 2 ? 3 : 0;
     const int x = atoi(e);
     return (x >= 1 && x <= 4) ? x : 0;
 }
@@ -1284,7 +1289,7 @@ template <int D>
 bool attr_window(int n, const AttrRows &rows)
 {
     const char *e = getenv("TSNE_ATTR_WINDOW");
-    const bool off = (e != nullptr && atoi(e) == 0) || getenv("TSNE_ATTR_PIPE") != nullptr || !attr_contig();
+    const bool off = (e != nullptr && atoi(e) == 0) || attr_pipe_asked() != nullptr || !attr_contig();
     return !off && rows.ranges != nullptr && (D == 2 || rows.tree_order || n <= win_pts<D>());
 }
 template <int D>
