@@ -1,4 +1,4 @@
-"""Which kernels a piece of work launches, by torch's profiler in a child process."""
+"""Which kernels a piece of work launches and how long they take, by torch's profiler in a child process."""
 import json
 import os
 import subprocess
@@ -20,13 +20,13 @@ with profile(activities=[ProfilerActivity.CUDA]) as prof:
 """
 EPILOGUE = """
     torch.cuda.synchronize()
-print("KERNELS" + json.dumps([e.key for e in prof.key_averages()]))
+print("KERNELS" + json.dumps({e.key: e.device_time_total / e.count for e in prof.key_averages()}))
 """
 
 
 def kernels_of(code, **env):
-    """Names (with template arguments) of the kernels that `code` launches; env: environment
-    variables, None to leave one unset."""
+    """The kernels that `code` launches: name (with template arguments) -> mean microseconds of a
+    launch; env: environment variables, None to leave one unset."""
     e = dict(os.environ)
     for k, v in env.items():
         e.pop(k, None)
@@ -35,4 +35,4 @@ def kernels_of(code, **env):
     src = PROLOGUE + "".join(f"    {line}\n" for line in code.strip().splitlines()) + EPILOGUE
     r = subprocess.run([sys.executable, "-c", src], env=e, capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
-    return [k for k in json.loads(r.stdout[r.stdout.rindex("KERNELS") + 7:]) if "k_" in k]
+    return {k: t for k, t in json.loads(r.stdout[r.stdout.rindex("KERNELS") + 7:]).items() if "k_" in k}

@@ -3628,8 +3628,27 @@ private:
     void launch_near(const ProdArgs &g, cudaStream_t st)
     {
         if (D == 2 && g.xin == nullptr) launch_early(k_near2d<PART>, n_node_, NEAR2_THREADS, 0, st, g);
-        else launch_early(k_near<D, 4, PART>, n_node_, NEAR_THREADS, 0, st, g);
+        else {
+            const size_t smem = PART == NEAR_BLOCKS ? near_spread() : 0;
+            if (smem > 0)
+                TSNE_CUDA_CHECK(cudaFuncSetAttribute(k_near<D, 4, PART>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     (int)smem));
+            launch_early(k_near<D, 4, PART>, n_node_, NEAR_THREADS, smem, st, g);
+        }
         launches_++;
+    }
+    // The internal 3D bases' CTAs take a whole SM each, and where there are more of them than SMs the
+    // near blocks beside them start on the first few SMs that come free. Few and large leaves
+    // would all go there, up to sixteen CTAs to an SM, and the others idle: 200K points on a line, 357 leaves of
+    // up to 700, took 7.8 ms that way and take 1.7 spread over the chip. So a CTA asks for as much shared
+    // memory (unused) as leaves room for no more than an SM's share of the leaves; nothing from 16 to an SM on.
+    size_t near_spread() const
+    {
+        constexpr size_t SM = 228 * 1024, RESERVED = 1024;   // an SM's shared memory, and the part per CTA
+        constexpr size_t OWN = NEAR_THREADS * (sizeof(Vec<D>) + sizeof(float4));
+        const int share = std::max(1, ceil_div(n_node_ - hint_, 148));
+        if (D == 2 || share >= 2048 / NEAR_THREADS) return 0;
+        return std::min<size_t>(SM / share, 227 * 1024) / 1024 * 1024 - RESERVED - OWN;
     }
     // The near blocks of the force product ([1 | Y] columns) need only the tree, the points and
     // the near lists, so a build runs them on a side stream beside the internal bases, whose
