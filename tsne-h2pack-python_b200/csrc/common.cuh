@@ -30,7 +30,7 @@ struct CudaError {
 // previous kernel's completion (and with it, link by link, for all work before it). The previous kernel may
 // still be writing when such a kernel's life begins, so it reads nothing as constant for its life: no
 // __restrict__ parameters, __ldg or ld.global.nc, which would let a read be moved above the wait (60 iterations with
-// such reads and without: 20K points 7.96 and 7.99 ms, 200K 21.27 and 21.34, 1M 74.2 and 74.4). No kernel lets its
+// such reads and without: 2K points 5.30 and 5.30 ms, 20K 7.57 and 7.57, 200K 16.56 and 16.58). No kernel lets its
 // successor in sooner (griddepcontrol.launch_dependents): blocks that wait would hold the SMs' slots,
 // which the side stream's near blocks use (30 iterations at 1M points: 33.6 ms, and 34.2 that way).
 // 60 iterations with ordinary launches and with these: 1,501 points exact 1.79 and 1.24 ms, 2K 5.86 and 5.13,

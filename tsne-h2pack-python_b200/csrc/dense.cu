@@ -709,9 +709,10 @@ k_attr_pair(int n, const int *__restrict__ rp, const int *__restrict__ col, cons
 // pointers and Y when a row starts, its first entries in the row's last step), and a CTA's row
 // range comes from a table. Rows are dealt to half-warps and summed over lanes as in
 // k_attr_update (same bits per row).
-// Per launch, form 3 -> this one: 1M points 0.679 -> 0.511 ms, 200K 0.134 -> 0.106, 300K in the
-// exaggeration phase 0.196 -> 0.156, 20K 26.7 -> 20.8 us, 2K 14.3 -> 10.3 us, 100K 3D 96.8 ->
-// 87.6 us. The window's size at 1M (before the P loads passed by L1): 64 KB 0.548 ms, 96 KB
+// Per launch, form 3 -> this one, on drawn embeddings: 1M points 0.679 -> 0.511 ms, 200K 0.134 ->
+// 0.106, 300K in the exaggeration phase 0.196 -> 0.156, 20K 26.7 -> 20.8 us, 2K 14.3 -> 10.3 us, 100K
+// 3D 96.8 -> 87.6 us. Averaged over a 1,000-iteration run at 1M points it gains less: 0.597 -> 0.579
+// ms. The window's size at 1M, drawn (before the P loads passed by L1): 64 KB 0.548 ms, 96 KB
 // 0.528, 128 KB 0.555, 160 KB 0.611, 224 KB 1.259: what the window takes is missing in L1 for
 // the lines in flight of the gathers outside it.
 constexpr int WIN_THREADS = 1024;
