@@ -3044,6 +3044,8 @@ public:
             id2_attr<false, 128, 2>();
         }
         if (D == 3) {
+            TSNE_CUDA_CHECK(cudaFuncSetAttribute(k_near<D, 4, NEAR_BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                 (int)NEAR_MOST));
             id3_attr<false, 512, ID3_ROWS>();
             id3_attr<true, 512, ID3_ROWS>();
             id3_attr<true, 512, ID3_MID>();
@@ -3630,13 +3632,7 @@ private:
     void launch_near(const ProdArgs &g, cudaStream_t st)
     {
         if (D == 2 && g.xin == nullptr) launch_early(k_near2d<PART>, n_node_, NEAR2_THREADS, 0, st, g);
-        else {
-            const size_t smem = PART == NEAR_BLOCKS ? near_spread() : 0;
-            if (smem > 0)
-                TSNE_CUDA_CHECK(cudaFuncSetAttribute(k_near<D, 4, PART>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     (int)smem));
-            launch_early(k_near<D, 4, PART>, n_node_, NEAR_THREADS, smem, st, g);
-        }
+        else launch_early(k_near<D, 4, PART>, n_node_, NEAR_THREADS, PART == NEAR_BLOCKS ? near_spread() : 0, st, g);
         launches_++;
     }
     // The internal 3D bases' CTAs take a whole SM each, and where there are more of them than SMs the
@@ -3647,11 +3643,14 @@ private:
     size_t near_spread() const
     {
         constexpr size_t SM = 228 * 1024, RESERVED = 1024;   // an SM's shared memory, and the part per CTA
-        constexpr size_t OWN = NEAR_THREADS * (sizeof(Vec<D>) + sizeof(float4));
         const int share = std::max(1, ceil_div(n_node_ - hint_, 148));
         if (D == 2 || share >= 2048 / NEAR_THREADS) return 0;
-        return std::min<size_t>(SM / share, 227 * 1024) / 1024 * 1024 - RESERVED - OWN;
+        return std::min<size_t>(SM / share / 1024 * 1024 - RESERVED - NEAR_OWN, NEAR_MOST);
     }
+    // k_near's own shared memory, and the most that a launch may ask for beside it (the kernel's limit is this
+    // constant for every workspace: it is the process's, and threads build at the same time)
+    static constexpr size_t NEAR_OWN = NEAR_THREADS * (sizeof(Vec<D>) + sizeof(float4));
+    static constexpr size_t NEAR_MOST = 227 * 1024 - NEAR_OWN;
     // The near blocks of the force product ([1 | Y] columns) need only the tree, the points and
     // the near lists, so a build runs them on a side stream beside the internal bases, whose
     // dependency chain leaves SMs idle. The fork point follows the leaf bases (which fill the
